@@ -26,6 +26,7 @@
 #include "krylov.cuh"
 #include "ilu.cuh"
 #include "bulk.cuh"
+#include "resident.cuh"
 
 namespace pfg {
 
@@ -1603,6 +1604,7 @@ Krylov::~Krylov()
 {
     if (graph_) cudaGraphExecDestroy(graph_);
     if (host_state_) cudaFreeHost(host_state_);
+    if (host_res_) cudaFreeHost(host_res_);
 }
 
 const Ilu0 &Krylov::ilu_factor(const DevMatrix &A, bool sorted, cudaStream_t st)
@@ -1987,6 +1989,13 @@ static int bicg_chunk_sym(const SellView<float> &U, float rowsum, int chunk, int
     return 7 * chunk;
 }
 
+// Largest systems (block rows) that run resident: FP64 CG, FP64 BiCGSTAB, mixed.
+// Where the two forms meet (us per iteration, kernel by kernel / resident): FP64
+// CG 389,017 rows 217.8 / 215.3; FP64 BiCGSTAB 148,877 rows 179.8 / 180.9; mixed
+// 91,125 rows 30.9 / 24.6 (CG) and 66.9 / 52.6 (BiCGSTAB), 148,877 rows 32.7 / 45.8
+// and 75.3 / 94.4 (the full FP32 copy no longer fits L2).
+constexpr int64_t kResidentRowsCG64 = 400000, kResidentRowsBiCG64 = 140000, kResidentRowsMixed = 110000;
+
 SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfig &cfg_in, cudaStream_t st)
 {
     KConfig cfg = cfg_in;
@@ -2009,14 +2018,35 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
     // mixed CG from the symmetric copy 257.6-259.1 vs 255.3-257.0 ms (the
     // gathers of z and p_old cost about what the direction pass saves).
     // Preconditioned BiCGSTAB exists only in the separate form.
-    if (cfg.fuse != 0 && cfg.fuse != 1) cfg.fuse = 0;
+    const bool free_mode = cfg.fuse != 0 && cfg.fuse != 1;
+    if (free_mode) cfg.fuse = 0;
     if (cfg.algorithm == PFG_ALG_BICGSTAB && cfg.precond != PFG_PC_NONE) cfg.fuse = 0;
     prepare(A, cfg, st);
     launches_ = 0;
+    // A solve that fits the SMs runs resident (run_resident); update_mode 1 and
+    // 2 name one of the kernel-by-kernel forms, debug prints their progress.
+    const bool may_reside = free_mode && cfg.debug == 0 && !is_ilu(cfg.precond);
+    auto plan_for = [&](const KConfig &c) {
+        ResPlan pl;
+        const bool mixed = c.precision == PFG_PREC_MIXED;
+        const int64_t most = mixed                          ? kResidentRowsMixed
+                             : c.algorithm == PFG_ALG_CG ? kResidentRowsCG64
+                                                         : kResidentRowsBiCG64;
+        if (may_reside && A.nb <= most) {
+            build_sell(A, true, false, st);  // the pattern
+            share_slices(A, st);
+            pl = plan_resident(A, c.algorithm, mixed, c.precond != PFG_PC_NONE);
+        }
+        return pl;
+    };
+    const ResPlan plan = plan_for(cfg);
     // the Krylov kernels read the sliced copy: FP64 always (residuals), FP32
     // for the mixed inner iterations
     // the symmetric-storage inner iterations read only the upper-half FP32 copy
-    build_sell(A, true, cfg.precision == PFG_PREC_MIXED && cfg.storage != PFG_STORAGE_SYMMETRIC, st);
+    // (a resident solve, whose full FP32 copy stays in L2, reads that one)
+    build_sell(A, true,
+               cfg.precision == PFG_PREC_MIXED && (cfg.storage != PFG_STORAGE_SYMMETRIC || plan.ctas > 0), st);
+    if (plan.ctas > 0 && cfg.storage == PFG_STORAGE_SYMMETRIC) check_symmetric(A, st);
     cudaEvent_t e0, e1;
     PFG_CUDA(cudaEventCreate(&e0));
     PFG_CUDA(cudaEventCreate(&e1));
@@ -2024,7 +2054,7 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
     SolveResult res;
     try {
         if (cfg.precision == PFG_PREC_MIXED) {
-            res = run_mixed(A, b, x, cfg, st);
+            res = plan.ctas > 0 ? run_resident(A, b, x, cfg, plan, st) : run_mixed(A, b, x, cfg, st);
             if (res.fallback) {
                 // The FP32 copy of the operator failed (repeated breakdowns or
                 // overflow, or FP64 residuals that stopped falling: a system
@@ -2035,14 +2065,18 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
                 c64.stop_rule = PFG_STOP_TRUE_RELATIVE;
                 c64.itrmax = std::max(1, cfg.itrmax - res.iterations);
                 prepare(A, c64, st);
-                SolveResult r2 = cfg.algorithm == PFG_ALG_CG ? run_cg64(A, b, x, c64, st)
-                                                             : run_bicgstab64(A, b, x, c64, st);
+                const ResPlan p64 = plan_for(c64);
+                SolveResult r2 = p64.ctas > 0                     ? run_resident(A, b, x, c64, p64, st)
+                                 : cfg.algorithm == PFG_ALG_CG    ? run_cg64(A, b, x, c64, st)
+                                                                  : run_bicgstab64(A, b, x, c64, st);
                 r2.iterations += res.iterations;
                 r2.replacements = res.replacements;
                 r2.fallback = 1;
                 res = r2;
             }
-        } else if (cfg.algorithm == PFG_ALG_CG)
+        } else if (plan.ctas > 0)
+            res = run_resident(A, b, x, cfg, plan, st);
+        else if (cfg.algorithm == PFG_ALG_CG)
             res = run_cg64(A, b, x, cfg, st);
         else
             res = run_bicgstab64(A, b, x, cfg, st);
@@ -2059,6 +2093,79 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
     res.launches = launches_;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    return res;
+}
+
+// Most iterations of one resident launch.
+constexpr int kResidentBudget = 4096;
+
+SolveResult Krylov::run_resident(DevMatrix &A, const double *b, double *x, const KConfig &cfg, const ResPlan &plan,
+                                 cudaStream_t st)
+{
+    const bool mixed = cfg.precision == PFG_PREC_MIXED, pc = cfg.precond != PFG_PC_NONE;
+    build_precond(A, cfg.precond, mixed, st);
+    if (!host_res_) {
+        PFG_CUDA(cudaMallocHost((void **)&host_res_, sizeof(ResState)));
+        memset(host_res_, 0, sizeof(ResState));
+        res_state_.alloc(sizeof(ResState));
+        res_slots_.alloc(kResSlots);
+    }
+    // the inboxes start empty; the rounds run on from solve to solve of one grid
+    // size, whose buffers each leaves in the order the next expects
+    unsigned round = host_res_->round;
+    if (res_ctas_ != plan.ctas || host_res_->err) {
+        PFG_CUDA(cudaMemsetAsync(res_slots_.p, 0xff, res_slots_.bytes(), st));
+        round = 0;
+    }
+    res_ctas_ = 0;  // until this solve has ended well
+    ResArgs a;
+    memset(&a, 0, sizeof a);
+    a.A64 = A.sell<double>();
+    a.A32 = A.sell<float>();
+    a.bounds = A.share.p;
+    a.b = b;
+    a.x = x;
+    a.xb = xb_.p;
+    const size_t np = (size_t)A.nb * (A.bs == 3 ? 4 : 1);
+    res_home_.ensure(plan.home_bytes);
+    a.home = res_home_.p;
+    if (mixed) {
+        res_pub32_.ensure(3 * np);
+        for (int k = 0; k < 3; ++k) a.pub32[k] = res_pub32_.p + (size_t)k * np;
+    } else {
+        res_pub64_.ensure(2 * np);
+        for (int k = 0; k < 2; ++k) a.pub64[k] = res_pub64_.p + (size_t)k * np;
+    }
+    a.dinv64 = dinv_.p;
+    a.dinv32 = dinv32_.p;
+    a.st = reinterpret_cast<ResState *>(res_state_.p);
+    a.slots = res_slots_.p;
+    a.pc = cfg.precond;
+    a.stop_rule = cfg.stop_rule;
+    a.itrmax = cfg.itrmax;
+    a.budget = kResidentBudget;
+    a.er0 = cfg.er0;
+    a.tol = cfg.relative_er;
+    a.delta = cfg.reliable_delta;
+    memset(host_res_, 0, sizeof(ResState));
+    host_res_->first = 1;
+    host_res_->round = round;
+    launches_ += run_resident_kernel(plan, a, A.bs, cfg.algorithm, mixed, host_res_, st);
+    res_ctas_ = plan.ctas;
+    const ResState &h = *host_res_;
+    SolveResult res;
+    res.status = h.status;
+    res.iterations = h.iter;
+    res.replacements = h.replacements;
+    res.rel_residual = h.rel;
+    res.fallback = h.fallback;
+    if (cfg.stop_rule == PFG_STOP_REFERENCE && cfg.algorithm == PFG_ALG_BICGSTAB && !mixed)
+        res.iter_residual = h.iter > 0 ? sqrt(h.rr / (h.rr1 > 0 ? h.rr1 : 1.0)) : 0.0;
+    else if (mixed || h.iter > 0)
+        res.iter_residual = sqrt(h.rr / (h.bb > 0 ? h.bb : 1.0));
+    if (!res.fallback && res.status == PFG_OK && cfg.stop_rule == PFG_STOP_TRUE_RELATIVE &&
+        res.rel_residual > cfg.relative_er)
+        res.status = PFG_W_NOT_CONVERGED;
     return res;
 }
 

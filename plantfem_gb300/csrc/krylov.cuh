@@ -81,19 +81,25 @@ struct DevMatrix {
     DevBuf<int> scol_u;
     DevBuf<float> s32_u;
     bool sell_u_pattern = false, s32_u_valid = false;
-    float sym_rowsum = 0.f;  // max over scalar rows of sum |a_ij| (FP32), set with s32_u
+    bool sym_checked = false;  // the values were found symmetric (check_symmetric)
+    float sym_rowsum = 0.f;  // max over scalar rows of sum |a_ij| (FP32), set with sym_checked
+
+    // resident solves: the CTAs' runs of slices (resident.cu share_slices)
+    DevBuf<int> share;
+    int share_ctas = 0, share_max = 0;
 
     // bumped whenever rp/col change: keys factors derived from the pattern
     uint64_t pattern_gen = 0;
 
     int64_t ndof() const { return nb * bs; }
     // v64 changed: every derived copy is stale
-    void values_changed() { v32_valid = s64_valid = s32_valid = s32_u_valid = false; }
+    void values_changed() { v32_valid = s64_valid = s32_valid = s32_u_valid = sym_checked = false; }
     // rp/col changed too
     void pattern_changed()
     {
         values_changed();
         sell_pattern = sell_u_pattern = false;
+        share_ctas = 0;
         pattern_gen = next_pattern_gen();
     }
     // process-wide counter: no two patterns (of any matrix) share a value
@@ -120,9 +126,12 @@ inline SellView<float> DevMatrix::sell<float>() const { return SellView<float>{n
 // values when stale.  Implemented in sell.cu.
 void build_sell(DevMatrix &A, bool want64, bool want32, cudaStream_t st);
 
-// Build (or refresh) the FP32 upper-half sliced copy of a 3x3-block matrix;
-// checks once per value change that the matrix is symmetric (blockwise, to
-// 1e-9 relative) and throws PFG_E_ARG if it is not.  Implemented in sell.cu.
+// Checks once per value change that a 3x3-block matrix is symmetric (blockwise,
+// to 1e-9 relative) and throws PFG_E_ARG if it is not.  Implemented in sell.cu.
+void check_symmetric(DevMatrix &A, cudaStream_t st);
+
+// Build (or refresh) the FP32 upper-half sliced copy of a 3x3-block matrix
+// (checked symmetric).  Implemented in sell.cu.
 void build_sell_upper(DevMatrix &A, cudaStream_t st);
 inline SellView<float> sell_upper(const DevMatrix &A)
 {
@@ -135,6 +144,8 @@ inline SellView<float> sell_upper(const DevMatrix &A)
 void block_jacobi(const DevMatrix &A, int precond, double *d64, float *d32, cudaStream_t st);
 
 class Ilu0;
+struct ResPlan;
+struct ResState;
 
 inline bool is_ilu(int precond) { return precond == PFG_PC_ILU0 || precond == PFG_PC_ILU0_SORTED; }
 
@@ -171,6 +182,9 @@ class Krylov {
     SolveResult run_cg64(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st);
     SolveResult run_bicgstab64(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st);
     SolveResult run_mixed(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st);
+    // The whole solve in one cooperative launch (resident.cuh).
+    SolveResult run_resident(DevMatrix &A, const double *b, double *x, const KConfig &cfg, const ResPlan &plan,
+                             cudaStream_t st);
     void read_state(KState &h, cudaStream_t st);
     // Hash of everything a captured chunk graph bakes in: every device pointer
     // its kernels receive and the configuration scalars.
@@ -191,6 +205,14 @@ class Krylov {
     DevBuf<unsigned int> ticket_;
     DevBuf<KState> state_;
     KState *host_state_ = nullptr;  // pinned mirror
+    // resident solves: state, its pinned mirror, exchange slots, published
+    // vectors, own vectors
+    DevBuf<unsigned char> res_state_;
+    DevBuf<double> res_slots_, res_pub64_;
+    DevBuf<float> res_pub32_;
+    DevBuf<unsigned char> res_home_;
+    ResState *host_res_ = nullptr;
+    int res_ctas_ = 0;       // CTAs that share the slots now
     // cached CUDA graphs of one chunk of iterations
     cudaGraphExec_t graph_ = nullptr;
     uint64_t graph_key_ = 0;

@@ -1,0 +1,69 @@
+// resident.cuh -- a whole CG / BiCGSTAB solve (FP64 or mixed) in one cooperative
+// launch, for systems whose product and ring fit the SMs' shared memory.
+// Implemented in resident.cu.
+#pragma once
+
+#include "krylov.cuh"
+
+namespace pfg {
+
+// Scalars of a resident solve between two launches (a launch stops after
+// `budget` iterations so that no kernel runs for seconds).
+struct ResState {
+    int phase;    // 0: start from the residual of x, 1: inside the iteration, 2: finished
+    int status;   // PFG_OK, PFG_E_BREAKDOWN, PFG_E_NONFINITE, PFG_W_NOT_CONVERGED
+    int fallback; // mixed: the caller finishes in FP64
+    int iter, restart, replacements, breakdowns, poisoned, failures, stall, first, parity;
+    double rho, beta, c2, c3, rr, rr1, bb, true_rr;
+    double rel, prev_rel, best_rel;
+    float rmax32, rmin32;
+    int err;         // raised when a wait runs out
+    unsigned round;  // exchanges made so far by the CTAs that share the slots
+};
+
+// What every resident kernel reads: matrices, the published (gathered) vectors
+// and the vectors that outlive a launch, all in global memory.
+struct ResArgs {
+    SellView<double> A64;
+    SellView<float> A32;
+    const int *bounds;  // first slice of each CTA's share (ctas + 1)
+    const double *b;
+    double *x, *xb;
+    // published vectors, 4 entries per block row of a 3x3-block system: FP64 p (CG)
+    // or M^-1 p and M^-1 e; FP32 z and the two p in turn (CG) or M^-1 p and M^-1 e
+    double *pub64[2];
+    float *pub32[3];
+    void *home;  // own vectors of every CTA, those not in shared memory
+    const double *dinv64;
+    const float *dinv32;
+    ResState *st;
+    double *slots;
+    int pc, stop_rule, itrmax, budget, stages, near;
+    double er0, tol, delta;
+};
+
+// The shared memory of a resident solve: `stages` ring stages per warp and the
+// first `near` of its own vectors.  ctas == 0: it does not fit.
+struct ResPlan {
+    int ctas = 0, stages = 0, near = 0, vectors = 0;
+    size_t smem = 0, home_bytes = 0;
+};
+
+constexpr int kResRounds = 8;    // exchange buffers in rotation
+constexpr int kResValues = 2;    // most values of one exchange
+constexpr int kResMaxCtas = 160;
+constexpr size_t kResSlots = (size_t)kResRounds * kResValues * kResMaxCtas * kResMaxCtas;
+
+// Cuts the sliced matrix into one run of slices per CTA with about equal work
+// (once per pattern: A.share, A.ctas, A.share_max).
+void share_slices(DevMatrix &A, cudaStream_t st);
+
+ResPlan plan_resident(const DevMatrix &A, int algorithm, bool mixed, bool precond);
+
+// Runs the solve from the state *host (page-locked; copied to a.st) until it is
+// finished, several launches if need be; *host then holds the final state.
+// Returns the launches made.
+int run_resident_kernel(const ResPlan &pl, ResArgs a, int bs, int algorithm, bool mixed, ResState *host,
+                        cudaStream_t st);
+
+}  // namespace pfg

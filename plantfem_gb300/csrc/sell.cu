@@ -276,11 +276,11 @@ __global__ void k_rowsum_max(int64_t nb, const int64_t *__restrict__ rp, const d
     if (lane == 0) atomicMax(out, __float_as_uint(best));
 }
 
-void build_sell_upper(DevMatrix &A, cudaStream_t st)
+void check_symmetric(DevMatrix &A, cudaStream_t st)
 {
     PFG_CHECK(A.nb > 0, PFG_E_STATE, "empty matrix");
     PFG_CHECK(A.bs == 3, PFG_E_UNSUPPORTED, "symmetric storage is built for 3x3-block matrices");
-    if (A.sell_u_pattern && A.s32_u_valid) return;
+    if (A.sym_checked) return;
     const int g = grid_for(A.nb, 256, sm_count_device() * 16);
     // the values (pattern included) changed: check the symmetry once
     {
@@ -299,6 +299,13 @@ void build_sell_upper(DevMatrix &A, cudaStream_t st)
                   "symmetric storage needs a symmetric matrix: " + std::to_string(nbad) +
                       " blocks differ from their transposes");
     }
+    A.sym_checked = true;
+}
+
+void build_sell_upper(DevMatrix &A, cudaStream_t st)
+{
+    check_symmetric(A, st);
+    if (A.sell_u_pattern && A.s32_u_valid) return;
     if (!A.sell_u_pattern) {
         A.ns_u = (A.nb + 31) / 32;
         DevBuf<int64_t> width((size_t)A.ns_u + 1);
