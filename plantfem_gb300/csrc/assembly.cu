@@ -269,11 +269,32 @@ __device__ __forceinline__ double gp_geometry(const double (*xe)[3], int gp, dou
     return gp_geometry_dn(xe, dN, G);
 }
 
-// gp_geometry with dN/dxi given (the element kernel keeps the eight Gauss
-// points' tables in shared memory: they are the same for every element).
+// det of J (row-major 3x3) by cofactors along the first column and, unless it is
+// zero, its inverse.
+__device__ __forceinline__ double det_inverse(const double (&J)[9], double (&Ji)[9])
+{
+    const double m0 = J[4] * J[8] - J[7] * J[5];
+    const double m1 = J[1] * J[8] - J[7] * J[2];
+    const double m2 = J[1] * J[5] - J[4] * J[2];
+    const double det = J[0] * m0 - J[3] * m1 + J[6] * m2;
+    if (det == 0.0) return 0.0;
+    const double d = 1.0 / det;
+    Ji[0] = d * (J[4] * J[8] - J[5] * J[7]);
+    Ji[1] = d * (J[2] * J[7] - J[1] * J[8]);
+    Ji[2] = d * (J[1] * J[5] - J[2] * J[4]);
+    Ji[3] = d * (J[5] * J[6] - J[3] * J[8]);
+    Ji[4] = d * (J[0] * J[8] - J[2] * J[6]);
+    Ji[5] = d * (J[2] * J[3] - J[0] * J[5]);
+    Ji[6] = d * (J[3] * J[7] - J[4] * J[6]);
+    Ji[7] = d * (J[1] * J[6] - J[0] * J[7]);
+    Ji[8] = d * (J[0] * J[4] - J[1] * J[3]);
+    return det;
+}
+
+// gp_geometry with dN/dxi given.
 __device__ __forceinline__ double gp_geometry_dn(const double (*xe)[3], const double (*dN)[8], double (*G)[3])
 {
-    double J[3][3];
+    double J[9], Ji[9];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -281,28 +302,14 @@ __device__ __forceinline__ double gp_geometry_dn(const double (*xe)[3], const do
             double s = 0.0;
 #pragma unroll
             for (int a = 0; a < 8; ++a) s = fma(dN[i][a], xe[a][j], s);
-            J[i][j] = s;
+            J[3 * i + j] = s;
         }
-    const double m0 = J[1][1] * J[2][2] - J[2][1] * J[1][2];
-    const double m1 = J[0][1] * J[2][2] - J[2][1] * J[0][2];
-    const double m2 = J[0][1] * J[1][2] - J[1][1] * J[0][2];
-    const double det = J[0][0] * m0 - J[1][0] * m1 + J[2][0] * m2;
+    const double det = det_inverse(J, Ji);
     if (det == 0.0) return 0.0;
-    const double d = 1.0 / det;
-    double Ji[3][3];
-    Ji[0][0] = d * (J[1][1] * J[2][2] - J[1][2] * J[2][1]);
-    Ji[0][1] = d * (J[0][2] * J[2][1] - J[0][1] * J[2][2]);
-    Ji[0][2] = d * (J[0][1] * J[1][2] - J[0][2] * J[1][1]);
-    Ji[1][0] = d * (J[1][2] * J[2][0] - J[1][0] * J[2][2]);
-    Ji[1][1] = d * (J[0][0] * J[2][2] - J[0][2] * J[2][0]);
-    Ji[1][2] = d * (J[0][2] * J[1][0] - J[0][0] * J[1][2]);
-    Ji[2][0] = d * (J[1][0] * J[2][1] - J[1][1] * J[2][0]);
-    Ji[2][1] = d * (J[0][1] * J[2][0] - J[0][0] * J[2][1]);
-    Ji[2][2] = d * (J[0][0] * J[1][1] - J[0][1] * J[1][0]);
 #pragma unroll
     for (int a = 0; a < 8; ++a)
 #pragma unroll
-        for (int p = 0; p < 3; ++p) G[a][p] = dN[0][a] * Ji[0][p] + dN[1][a] * Ji[1][p] + dN[2][a] * Ji[2][p];
+        for (int p = 0; p < 3; ++p) G[a][p] = dN[0][a] * Ji[p] + dN[1][a] * Ji[3 + p] + dN[2][a] * Ji[6 + p];
     return det;
 }
 
@@ -323,25 +330,31 @@ __device__ __forceinline__ int64_t find_slot(const int64_t *__restrict__ rp, con
     return -1;
 }
 
-// Element matrices, four threads per element.  Stiffness: B^T D B detJ summed
-// over the Gauss points (FEMDomainClass.f90:11504-11511).  With the Lame
-// constants of the element and P_ab = sum_gp detJ g_a g_b^T (g_a the
-// gradient of N_a through the reference's J^-T form), the 3x3 block is
-// K_ab = lambda P_ab + mu P_ab^T + mu tr(P_ab) I, the product with B of
-// :12283-12305 and D of :11626-11637 written out.  Mass: rho sum_gp N_a N_b
-// detJ I3 (FEMDomainClass.f90:10934-10936); row-lumped (:10940-10948): the
-// row sums on the diagonal blocks.  Only the 36 blocks b >= a are computed
-// (K and M are symmetric); each is added at (a, b) and, transposed, at (b, a).
-// Thread s of an element takes block rows s and 7 - s (nine blocks each).
-// Node coordinates, gradients and detJ of the eight Gauss points live in
-// shared memory (the four threads compute two Gauss points each); the slot
-// of every block in its CRS row comes from the element's slot map (built
-// once per pattern), so the scatter does no search.  FP64-bound: about 4.5k
-// DFMA per stiffness element.
-constexpr int kEPC = 16;  // elements per CTA
+// Element matrices, a thread per 3x3 block of the upper half (36 per element,
+// eight elements per CTA).  Stiffness: B^T D B detJ summed over the Gauss points
+// (FEMDomainClass.f90:11504-11511).  With the Lame constants of the element and
+// P_ab = sum_gp detJ g_a g_b^T (g_a the gradient of N_a through the reference's
+// J^-T form), the 3x3 block is K_ab = lambda P_ab + mu P_ab^T + mu tr(P_ab) I, the
+// product with B of :12283-12305 and D of :11626-11637 written out.  Mass: rho
+// sum_gp N_a N_b detJ I3 (FEMDomainClass.f90:10934-10936); row-lumped
+// (:10940-10948): the row sums on the diagonal blocks.  Only the 36 blocks b >= a
+// are computed (K and M are symmetric); each is added at (a, b) and, transposed, at
+// (b, a).  The slot of every block in its CRS row comes from the element's slot map
+// (built once per pattern), so the scatter does no search.
+// What bounds it: the FP64 pipe (about 5.2k multiply-adds per stiffness element,
+// 17 cycles of the chip's 304 per clock) on large meshes, the chain of one
+// thread's multiply-adds (65 cycles each) on small ones.  So the work of an element
+// is cut as fine as its data flow allows: the Jacobians' entries (9 per Gauss
+// point), their inverses, the gradients (a thread per node and Gauss point) and the
+// blocks, each spread over the whole CTA.  Per colour launch (an eighth of the mesh):
+// four threads per element with nine blocks each took 181 us at 20^3 and 17x15x13
+// (whatever the size) and 806 us at 64^3; this takes 26 us and 444 us (the pipe's
+// share at 64^3: 290 us).
+constexpr int kEPC = 8;  // elements per CTA
+constexpr int kElemThreads = 36 * kEPC;
 
-template <int GPU, int MINB>
-__global__ void __launch_bounds__(4 * kEPC, MINB)
+template <int MINB>
+__global__ void __launch_bounds__(kElemThreads, MINB)
     k_element_matrix(int64_t n_el, const int *__restrict__ elems, const double *__restrict__ xyz, int64_t nn,
                      const int *__restrict__ conn, int64_t ne, int kind, const double *__restrict__ p0,
                      const double *__restrict__ p1, int bcast, const int64_t *__restrict__ rp,
@@ -349,160 +362,179 @@ __global__ void __launch_bounds__(4 * kEPC, MINB)
                      int *err)
 {
     __shared__ double sX[kEPC][8][3];
-    __shared__ double sH[kEPC][8][8][3];  // [element][gp][node][dim]: sqrt|detJ| g (G itself where detJ <= 0)
-    __shared__ double sW[kEPC][8];
+    __shared__ double sH[kEPC][8][8][3];  // [element][gp][node][dim]: sqrt(detJ) g (g itself where a detJ <= 0)
+    __shared__ double sJ[kEPC][8][9];     // dN/dxi x, then its inverse
+    __shared__ double sW[kEPC][8], sR[kEPC][8];
     __shared__ double sDN[8][3][8];       // dN/dxi per Gauss point
+    __shared__ double sN[8][8];           // N per Gauss point and node
     __shared__ int sNode[kEPC][8];
     __shared__ int sPos[kEPC];            // every detJ of the element > 0
-    const int q = threadIdx.x >> 2, sub = threadIdx.x & 3;
-    for (int gp = threadIdx.x; gp < 8; gp += blockDim.x) gp_dshape(gp, sDN[gp]);
-    __syncthreads();
+    const int tid = threadIdx.x;
+    if (tid < 8) gp_dshape(tid, sDN[tid]);
+    if (tid >= 64 && tid < 128) sN[(tid - 64) >> 3][tid & 7] = shape_N(tid & 7, (tid - 64) >> 3);
+    // this thread's block (a, b), b >= a, of element q
+    const int q4 = tid / 36;
+    int a4 = 0, b4 = tid - 36 * q4;
+    while (b4 >= 8 - a4) {
+        b4 -= 8 - a4;
+        ++a4;
+    }
+    b4 += a4;
     for (int64_t base = (int64_t)blockIdx.x * kEPC; base < n_el; base += (int64_t)gridDim.x * kEPC) {
-        const int64_t li = base + q;
-        const bool valid = li < n_el;
-        const int e = valid ? (elems ? elems[li] : (int)li) : 0;
-        if (valid)
+        const int here = (int)min((int64_t)kEPC, n_el - base);
+        if (tid < 8 * here) {
+            const int q = tid >> 3, v = tid & 7;
+            const int64_t li = base + q;
+            const int e = elems ? elems[li] : (int)li;
+            const int node = conn[(int64_t)v * ne + e];
+            sNode[q][v] = node;
+            sX[q][v][0] = xyz[node];
+            sX[q][v][1] = xyz[nn + node];
+            sX[q][v][2] = xyz[2 * nn + node];
+        }
+        __syncthreads();
+        for (int t = tid; t < 72 * here; t += kElemThreads) {
+            const int q = t / 72, r = t - 72 * q, gp = r / 9, ij = r - 9 * gp, i = ij / 3, j = ij - 3 * i;
+            double s = 0.0;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int v = sub + 4 * h;
-                const int node = conn[(int64_t)v * ne + e];
-                sNode[q][v] = node;
-                sX[q][v][0] = xyz[node];
-                sX[q][v][1] = xyz[nn + node];
-                sX[q][v][2] = xyz[2 * nn + node];
-            }
-        __syncwarp();
-        bool pos = true;
-        if (valid)
+            for (int v = 0; v < 8; ++v) s = fma(sDN[gp][i][v], sX[q][v][j], s);
+            sJ[q][gp][ij] = s;
+        }
+        __syncthreads();
+        if (tid < 8 * kEPC) {
+            const int q = tid >> 3, gp = tid & 7;
+            double det = 1.0;
+            if (q < here) {
+                double J[9], Ji[9];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int gp = sub + 4 * h;
-                const double det = gp_geometry_dn(sX[q], sDN[gp], sH[q][gp]);
-                sW[q][gp] = det;
+                for (int k = 0; k < 9; ++k) J[k] = sJ[q][gp][k];
+                det = det_inverse(J, Ji);
                 if (det == 0.0) *err = 1;
-                pos = pos && det > 0.0;
+                sW[q][gp] = det;
+#pragma unroll
+                for (int k = 0; k < 9; ++k) sJ[q][gp][k] = Ji[k];
             }
-        {  // the element's four lanes (a quad of the warp) agree on whether every detJ > 0
-            int pv = pos ? 1 : 0;
+            // the element's eight lanes agree on whether every detJ > 0: then
+            // P_ab = sum_gp h_a h_b^T with h = sqrt(detJ) g; otherwise g stays and
+            // each term takes its detJ
+            int pv = det > 0.0 ? 1 : 0;
             pv &= __shfl_xor_sync(0xffffffffu, pv, 1);
             pv &= __shfl_xor_sync(0xffffffffu, pv, 2);
-            pos = pv != 0;
-        }
-        __syncwarp();
-        if (valid && kind == 0) {
-            // P_ab = sum_gp detJ g_a g_b^T = sum_gp h_a h_b^T with h = sqrt(detJ) g when
-            // every detJ > 0; otherwise G stays and each term takes its detJ
-            if (sub == 0) sPos[q] = pos ? 1 : 0;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int gp = sub + 4 * h;
-                if (pos) {
-                    const double r = sqrt(sW[q][gp]);
-#pragma unroll
-                    for (int v = 0; v < 8; ++v)
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) sH[q][gp][v][d] *= r;
-                }
+            pv &= __shfl_xor_sync(0xffffffffu, pv, 4);
+            if (q < here) {
+                sPos[q] = pv;
+                sR[q][gp] = pv && kind == 0 ? sqrt(det) : 1.0;
             }
         }
-        __syncwarp();
-        if (valid) {
-            double lam = 0.0, mu = 0.0, rho = 0.0;
-            if (kind == 0)
+        __syncthreads();
+        if (kind == 0) {
+            for (int t = tid; t < 64 * here; t += kElemThreads) {
+                const int q = t >> 6, gp = (t >> 3) & 7, v = t & 7;
+                const double r = sR[q][gp];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    const double g = sDN[gp][0][v] * sJ[q][gp][p] + sDN[gp][1][v] * sJ[q][gp][3 + p] +
+                                     sDN[gp][2][v] * sJ[q][gp][6 + p];
+                    sH[q][gp][v][p] = g * r;
+                }
+            }
+            __syncthreads();
+        }
+        const int q = q4, a = a4, b = b4;
+        if (q < here && !(kind == 2 && a != b && mode == 0)) {  // lumped: diagonal blocks only
+            const int64_t li = base + q;
+            const int e = elems ? elems[li] : (int)li;
+            double *va = nullptr, *vb = nullptr;
+            int na = 0, nb = 0;
+            if (mode == 0) {
+                const uint16_t *sl = slots + (int64_t)e * 64;
+                const int ra = sNode[q][a], rb = sNode[q][b];
+                const int64_t r0 = rp[ra], r1 = rp[rb];
+                na = (int)(rp[ra + 1] - r0);
+                nb = (int)(rp[rb + 1] - r1);
+                va = val + r0 * 9 + sl[a * 8 + b];
+                vb = val + r1 * 9 + sl[b * 8 + a];
+            }
+            double K[3][3];
+            if (kind == 0) {
+                double P[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+                if (sPos[q]) {
+#pragma unroll 4
+                    for (int gp = 0; gp < 8; ++gp) {
+                        const double ha[3] = {sH[q][gp][a][0], sH[q][gp][a][1], sH[q][gp][a][2]};
+                        const double hb[3] = {sH[q][gp][b][0], sH[q][gp][b][1], sH[q][gp][b][2]};
+#pragma unroll
+                        for (int i = 0; i < 3; ++i)
+#pragma unroll
+                            for (int j = 0; j < 3; ++j) P[i][j] = fma(ha[i], hb[j], P[i][j]);
+                    }
+                } else {
+                    for (int gp = 0; gp < 8; ++gp) {
+                        const double w = sW[q][gp];
+                        const double wa[3] = {w * sH[q][gp][a][0], w * sH[q][gp][a][1], w * sH[q][gp][a][2]};
+                        const double gb[3] = {sH[q][gp][b][0], sH[q][gp][b][1], sH[q][gp][b][2]};
+#pragma unroll
+                        for (int i = 0; i < 3; ++i)
+#pragma unroll
+                            for (int j = 0; j < 3; ++j) P[i][j] = fma(wa[i], gb[j], P[i][j]);
+                    }
+                }
+                double lam, mu;
                 lame(bcast ? p0[0] : p0[e], bcast ? p1[0] : p1[e], lam, mu);
-            else
-                rho = bcast ? p0[0] : p0[e];
-            const uint16_t *sl = slots ? slots + (int64_t)e * 64 : nullptr;
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                const int a = h == 0 ? sub : 7 - sub;
-#pragma unroll 1
-                for (int b = a; b < 8; ++b) {
-                    double K[3][3];
-                    if (kind == 0) {
-                        double P[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-                        if (sPos[q]) {
-#pragma unroll GPU
-                            for (int gp = 0; gp < 8; ++gp) {
-                                const double ha[3] = {sH[q][gp][a][0], sH[q][gp][a][1], sH[q][gp][a][2]};
-                                const double hb[3] = {sH[q][gp][b][0], sH[q][gp][b][1], sH[q][gp][b][2]};
+                const double mt = mu * (P[0][0] + P[1][1] + P[2][2]);
 #pragma unroll
-                                for (int i = 0; i < 3; ++i)
+                for (int i = 0; i < 3; ++i)
 #pragma unroll
-                                    for (int j = 0; j < 3; ++j) P[i][j] = fma(ha[i], hb[j], P[i][j]);
-                            }
-                        } else {
-                            for (int gp = 0; gp < 8; ++gp) {
-                                const double w = sW[q][gp];
-                                const double wa[3] = {w * sH[q][gp][a][0], w * sH[q][gp][a][1], w * sH[q][gp][a][2]};
-                                const double gb[3] = {sH[q][gp][b][0], sH[q][gp][b][1], sH[q][gp][b][2]};
+                    for (int j = 0; j < 3; ++j) K[i][j] = fma(lam, P[i][j], mu * P[j][i]) + (i == j ? mt : 0.0);
+            } else {
+                const double rho = bcast ? p0[0] : p0[e];
+                double m = 0.0;
+                if (kind == 1) {
 #pragma unroll
-                                for (int i = 0; i < 3; ++i)
+                    for (int gp = 0; gp < 8; ++gp) m += sN[gp][a] * sN[gp][b] * sW[q][gp];
+                    m *= rho;
+                } else if (a == b) {
+                    for (int bb = 0; bb < 8; ++bb) {
+                        double mb = 0.0;
 #pragma unroll
-                                    for (int j = 0; j < 3; ++j) P[i][j] = fma(wa[i], gb[j], P[i][j]);
-                            }
-                        }
-                        const double mt = mu * (P[0][0] + P[1][1] + P[2][2]);
-#pragma unroll
-                        for (int i = 0; i < 3; ++i)
-#pragma unroll
-                            for (int j = 0; j < 3; ++j)
-                                K[i][j] = fma(lam, P[i][j], mu * P[j][i]) + (i == j ? mt : 0.0);
-                    } else {
-                        double m = 0.0;
-                        if (kind == 1) {
-#pragma unroll
-                            for (int gp = 0; gp < 8; ++gp) m += shape_N(a, gp) * shape_N(b, gp) * sW[q][gp];
-                            m *= rho;
-                        } else if (a == b) {
-                            for (int bb = 0; bb < 8; ++bb) {
-                                double mb = 0.0;
-#pragma unroll
-                                for (int gp = 0; gp < 8; ++gp) mb += shape_N(a, gp) * shape_N(bb, gp) * sW[q][gp];
-                                m += rho * mb;
-                            }
-                        }
-#pragma unroll
-                        for (int i = 0; i < 3; ++i)
-#pragma unroll
-                            for (int j = 0; j < 3; ++j) K[i][j] = (i == j) ? m : 0.0;
-                        if (kind == 2 && a != b && mode == 0) continue;  // lumped: diagonal blocks only
+                        for (int gp = 0; gp < 8; ++gp) mb += sN[gp][a] * sN[gp][bb] * sW[q][gp];
+                        m += rho * mb;
                     }
-                    if (mode == 1) {
-                        double *o = out + (int64_t)e * 576;
+                }
 #pragma unroll
-                        for (int i = 0; i < 3; ++i)
+                for (int i = 0; i < 3; ++i)
 #pragma unroll
-                            for (int j = 0; j < 3; ++j) {
-                                o[(3 * b + j) * 24 + 3 * a + i] = K[i][j];
-                                if (a != b) o[(3 * a + i) * 24 + 3 * b + j] = K[i][j];
-                            }
-                        continue;
+                    for (int j = 0; j < 3; ++j) K[i][j] = (i == j) ? m : 0.0;
+            }
+            if (mode == 1) {
+                double *o = out + (int64_t)e * 576;
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        o[(3 * b + j) * 24 + 3 * a + i] = K[i][j];
+                        if (a != b) o[(3 * a + i) * 24 + 3 * b + j] = K[i][j];
                     }
-                    {
-                        const int ra = sNode[q][a];
-                        const int64_t r0 = rp[ra];
-                        const int nblk = (int)(rp[ra + 1] - r0);
-                        double *v = val + r0 * 9 + sl[a * 8 + b];
+            } else {
+                // a colour's elements share no node: every entry has one writer
+                double old[9];
 #pragma unroll
-                        for (int i = 0; i < 3; ++i)
+                for (int k = 0; k < 9; ++k) old[k] = va[(int64_t)k * na];
 #pragma unroll
-                            for (int j = 0; j < 3; ++j) v[(int64_t)(3 * i + j) * nblk] += K[i][j];
-                    }
-                    if (a != b) {
-                        const int rb = sNode[q][b];
-                        const int64_t r0 = rp[rb];
-                        const int nblk = (int)(rp[rb + 1] - r0);
-                        double *v = val + r0 * 9 + sl[b * 8 + a];
+                for (int i = 0; i < 3; ++i)
 #pragma unroll
-                        for (int i = 0; i < 3; ++i)
+                    for (int j = 0; j < 3; ++j) va[(int64_t)(3 * i + j) * na] = old[3 * i + j] + K[i][j];
+                if (a != b) {
 #pragma unroll
-                            for (int j = 0; j < 3; ++j) v[(int64_t)(3 * j + i) * nblk] += K[i][j];
-                    }
+                    for (int k = 0; k < 9; ++k) old[k] = vb[(int64_t)k * nb];
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) vb[(int64_t)(3 * j + i) * nb] = old[3 * j + i] + K[i][j];
                 }
             }
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -560,24 +592,21 @@ template <typename Kern>
 static int element_grid(Kern kern, int64_t n)
 {
     int per_sm = 0;
-    PFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 4 * kEPC, 0));
+    PFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kElemThreads, 0));
     if (per_sm <= 0) per_sm = 1;
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + kEPC - 1) / kEPC, (int64_t)per_sm * sm_count_device()));
 }
 
-// The element kernel's configuration: Gauss-point loop unrolled 4x, at least
-// 6 CTAs per SM (168 registers).  Measured at 100^3 (1M elements, 8 colour
-// launches): 22.1 ms against 23.2 ms fully unrolled (252 registers) and
-// 27.1 ms at 128 registers (spills).
+// The element kernel's configuration: at least 2 CTAs per SM (96 registers).
 using ElementKernel = void (*)(int64_t, const int *, const double *, int64_t, const int *, int64_t, int,
                                const double *, const double *, int, const int64_t *, const uint16_t *, double *, int,
                                double *, int *);
-static const ElementKernel kElementKernel = k_element_matrix<4, 6>;
+static const ElementKernel kElementKernel = k_element_matrix<2>;
 
 template <typename... Args>
 static void launch_element_matrix(int64_t n, cudaStream_t st, Args... args)
 {
-    kElementKernel<<<element_grid(kElementKernel, n), 4 * kEPC, 0, st>>>(n, args...);
+    kElementKernel<<<element_grid(kElementKernel, n), kElemThreads, 0, st>>>(n, args...);
 }
 
 void assemble_elements(const DevMesh &m, DevMatrix &K, int kind, const double *p0, const double *p1, bool broadcast,
