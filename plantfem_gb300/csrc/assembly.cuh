@@ -60,8 +60,9 @@ void adjoint_grad_E(const DevMesh &m, const double *u, const double *lam, const 
 
 // Dirichlet elimination of FEMSolver_%solve (FEMSolverClass.f90:1707-1756)
 // on the device, in place: rhs_i -= K_ij u_j for fixed j (every row), then
-// rhs(fixed) = value, zero fixed rows and columns, unit diagonal.
-void apply_dirichlet(DevMatrix &K, double *rhs, const uint8_t *fixed, const double *fixval, cudaStream_t st);
+// rhs(fixed) = value, zero fixed rows and columns, unit diagonal.  Returns whether
+// a stored value changed (false: the matrix was eliminated already).
+bool apply_dirichlet(DevMatrix &K, double *rhs, const uint8_t *fixed, const double *fixval, cudaStream_t st);
 // x(fixed) = value (FEMSolverClass.f90:1814-1823).
 void restore_fixed(int64_t n, double *x, const uint8_t *fixed, const double *fixval, cudaStream_t st);
 

@@ -1751,11 +1751,22 @@ void block_jacobi(const DevMatrix &A, int precond, double *d64, float *d32, cuda
 void Krylov::build_precond(const DevMatrix &A, int precond, bool fp32, cudaStream_t st)
 {
     if (precond == PFG_PC_NONE || is_ilu(precond)) return;
+    // kept while the matrix's values stay (time steps, further right-hand sides)
+    if (dinv_gen_ == A.value_gen && dinv_pc_ == precond &&
+        (!fp32 || (dinv32_gen_ == A.value_gen && dinv32_pc_ == precond)))
+        return;
     const size_t m = (size_t)std::max<int64_t>(A.nb * A.bs * A.bs, 1);
+    dinv_gen_ = dinv32_gen_ = 0;
     dinv_.ensure(m);
     if (fp32) dinv32_.ensure(m);
     block_jacobi(A, precond, dinv_.p, fp32 ? dinv32_.p : nullptr, st);
     ++launches_;
+    dinv_gen_ = A.value_gen;
+    dinv_pc_ = precond;
+    if (fp32) {
+        dinv32_gen_ = A.value_gen;
+        dinv32_pc_ = precond;
+    }
 }
 
 void Krylov::read_state(KState &h, cudaStream_t st)
@@ -2347,6 +2358,7 @@ SolveResult Krylov::run_mixed(DevMatrix &A, const double *b, double *x, const KC
         // upper half (checked symmetric) and its zeroed accumulator: 4 floats
         // per row (CG) or three fixed-point planes (BiCGSTAB)
         build_sell_upper(A, st);
+        if (!cg) bound_rows(A, st);
         if (cg) {
             y4_.ensure((size_t)A.nb * 4);
             PFG_CUDA(cudaMemsetAsync(y4_.p, 0, (size_t)A.nb * 4 * sizeof(float), st));
@@ -2614,6 +2626,7 @@ void Krylov::profile(DevMatrix &A, int kernel, int reps, cudaStream_t st, double
     if (kernel <= 2 || kernel == 5 || kernel == 6) build_sell(A, f64, !f64, st);
     if (kernel >= 7) {
         build_sell_upper(A, st);
+        bound_rows(A, st);
         y4_.ensure((size_t)A.nb * 4);
         PFG_CUDA(cudaMemsetAsync(y4_.p, 0, (size_t)A.nb * 4 * sizeof(float), st));
     }

@@ -82,18 +82,23 @@ struct DevMatrix {
     DevBuf<float> s32_u;
     bool sell_u_pattern = false, s32_u_valid = false;
     bool sym_checked = false;  // the values were found symmetric (check_symmetric)
-    float sym_rowsum = 0.f;  // max over scalar rows of sum |a_ij| (FP32), set with sym_checked
+    bool sym_rowsum_valid = false;
+    float sym_rowsum = 0.f;  // max over scalar rows of sum |a_ij| (FP32; bound_rows)
 
     // resident solves: the CTAs' runs of slices (resident.cu share_slices)
     DevBuf<int> share;
     int share_ctas = 0, share_max = 0;
 
-    // bumped whenever rp/col change: keys factors derived from the pattern
-    uint64_t pattern_gen = 0;
+    // bumped whenever rp/col (the values) change: key what is derived from them
+    uint64_t pattern_gen = 0, value_gen = 0;
 
     int64_t ndof() const { return nb * bs; }
     // v64 changed: every derived copy is stale
-    void values_changed() { v32_valid = s64_valid = s32_valid = s32_u_valid = sym_checked = false; }
+    void values_changed()
+    {
+        v32_valid = s64_valid = s32_valid = s32_u_valid = sym_checked = sym_rowsum_valid = false;
+        value_gen = next_pattern_gen();
+    }
     // rp/col changed too
     void pattern_changed()
     {
@@ -102,7 +107,7 @@ struct DevMatrix {
         share_ctas = 0;
         pattern_gen = next_pattern_gen();
     }
-    // process-wide counter: no two patterns (of any matrix) share a value
+    // process-wide counter: no two patterns or values (of any matrix) share one
     static uint64_t next_pattern_gen()
     {
         static std::atomic<uint64_t> counter{0};
@@ -129,6 +134,9 @@ void build_sell(DevMatrix &A, bool want64, bool want32, cudaStream_t st);
 // Checks once per value change that a 3x3-block matrix is symmetric (blockwise,
 // to 1e-9 relative) and throws PFG_E_ARG if it is not.  Implemented in sell.cu.
 void check_symmetric(DevMatrix &A, cudaStream_t st);
+
+// A.sym_rowsum, once per value change (the fixed-point product's bound).
+void bound_rows(DevMatrix &A, cudaStream_t st);
 
 // Build (or refresh) the FP32 upper-half sliced copy of a 3x3-block matrix
 // (checked symmetric).  Implemented in sell.cu.
@@ -193,6 +201,9 @@ class Krylov {
 
     int64_t n_ = 0;
     int bs_ = 3;
+    // what dinv_ / dinv32_ were built from
+    uint64_t dinv_gen_ = 0, dinv32_gen_ = 0;
+    int dinv_pc_ = 0, dinv32_pc_ = 0;
     // FP64 work vectors
     DevBuf<double> r_, r0_, z_, pA_, pB_, q_, yA_, yB_, e_, v_, dinv_, ph_, eh_;
     DevBuf<double> xb_;  // mixed: x before the fold of an FP32 correction

@@ -32,46 +32,70 @@ __global__ void k_sell_pattern(int64_t nb, int64_t ns, const int64_t *__restrict
     }
 }
 
-// Slice values, one warp per slice (lane = row of the slice), one entry plane
-// (r, c) and up to kTileK slots at a time through shared memory: each row's
-// plane is read as one contiguous run of its blocks (block row layout,
-// bsr.cuh) and written back slot by slot as 32 consecutive lanes.
-constexpr int kTileK = 64;
-constexpr int kTileWarps = 2;
+// Slice values: a warp per (slice, entry plane), so a 3x3-block slice is a CTA of
+// nine warps; kTileK slots at a time through a shared-memory tile of the warp.  Each
+// row's plane is read as one contiguous run of its blocks (block row layout,
+// bsr.cuh), eight rows' loads in flight, and written back slot by slot as 32
+// consecutive lanes; FP64 and FP32 copies come from one read.  Bound by HBM on
+// large meshes, by the latency of the 32 row reads on small ones: a warp per slice
+// that took the nine planes in turn ran 831 us at 274,625 rows (FP64 copy) and 157 us
+// at 4,032; this runs 230 us and 12 us (1.1 GB moved: 4.9 TB/s).
+constexpr int kTileK = 32;
 
-template <int BS, typename T>
-__global__ void __launch_bounds__(32 * kTileWarps)
+template <int BS>
+constexpr int kSellSlices = BS == 3 ? 1 : 8;  // slices per CTA
+template <int BS>
+constexpr int kSellThreads = 32 * BS * BS * kSellSlices<BS>;
+template <int BS>
+constexpr size_t kSellTile = (size_t)BS * BS * kSellSlices<BS> * 32 * (kTileK + 1) * sizeof(double);
+
+template <int BS>
+__global__ void __launch_bounds__(kSellThreads<BS>)
     k_sell_values(int64_t nb, int64_t ns, const int64_t *__restrict__ rp, const double *__restrict__ v64,
-                  const int64_t *__restrict__ sptr, T *__restrict__ sval)
+                  const int64_t *__restrict__ sptr, double *__restrict__ s64, float *__restrict__ s32)
 {
     constexpr int BB = BS * BS;
-    __shared__ T tile[kTileWarps][32][kTileK + 1];
+    extern __shared__ double dyn_tile[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int64_t s = (int64_t)blockIdx.x * kTileWarps + w; s < ns; s += (int64_t)gridDim.x * kTileWarps) {
+    double *tile = dyn_tile + (size_t)w * 32 * (kTileK + 1);
+    const int e = w % BB;
+    for (int64_t s = (int64_t)blockIdx.x * kSellSlices<BS> + w / BB; s < ns; s += (int64_t)gridDim.x * kSellSlices<BS>) {
         const int64_t b0 = sptr[s];
         const int wdt = (int)(sptr[s + 1] - b0);
         const int64_t row = s * 32 + lane;
         const int64_t r0 = row < nb ? rp[row] : 0;
         const int nblk = row < nb ? (int)(rp[row + 1] - r0) : 0;
-        for (int e = 0; e < BB; ++e)
-            for (int kc = 0; kc < wdt; kc += kTileK) {
-                for (int l = 0; l < 32; ++l) {
-                    const int64_t r0l = __shfl_sync(0xffffffffu, r0, l);
-                    const int nl = __shfl_sync(0xffffffffu, nblk, l);
-                    for (int kk = lane; kk < kTileK; kk += 32) {
-                        const int k = kc + kk;
-                        tile[w][l][kk] = k < nl ? (T)v64[r0l * BB + (int64_t)e * nl + k] : T(0);
-                    }
-                }
-                __syncwarp();
-                const int kend = min(kTileK, wdt - kc);
-                for (int kk = 0; kk < kend; ++kk) sval[((b0 + kc + kk) * BB + e) * 32 + lane] = tile[w][lane][kk];
-                __syncwarp();
+        for (int kc = 0; kc < wdt; kc += kTileK) {
+#pragma unroll 8
+            for (int l = 0; l < 32; ++l) {
+                const int64_t r0l = __shfl_sync(0xffffffffu, r0, l);
+                const int nl = __shfl_sync(0xffffffffu, nblk, l);
+                const int k = kc + lane;
+                tile[l * (kTileK + 1) + lane] = k < nl ? ld_stream(v64 + r0l * BB + (int64_t)e * nl + k) : 0.0;
             }
+            __syncwarp();
+            const int kend = min(kTileK, wdt - kc);
+#pragma unroll 4
+            for (int kk = 0; kk < kend; ++kk) {
+                const double v = tile[lane * (kTileK + 1) + kk];
+                const int64_t o = ((b0 + kc + kk) * BB + e) * 32 + lane;
+                if (s64) s64[o] = v;
+                if (s32) s32[o] = (float)v;
+            }
+            __syncwarp();
+        }
     }
 }
 
-static int tile_grid(int64_t ns) { return (int)std::min<int64_t>((ns + kTileWarps - 1) / kTileWarps, sm_count_device() * 32); }
+template <int BS>
+static void launch_sell_values(DevMatrix &A, double *s64, float *s32, cudaStream_t st)
+{
+    PFG_CUDA(cudaFuncSetAttribute(k_sell_values<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSellTile<BS>));
+    const int64_t ctas = (A.ns + kSellSlices<BS> - 1) / kSellSlices<BS>;
+    k_sell_values<BS><<<(int)std::min<int64_t>(ctas, sm_count_device() * 16), kSellThreads<BS>, kSellTile<BS>, st>>>(
+        A.nb, A.ns, A.rp.p, A.v64.p, A.sptr.p, s64, s32);
+    PFG_CUDA(cudaGetLastError());
+}
 
 void build_sell(DevMatrix &A, bool want64, bool want32, cudaStream_t st)
 {
@@ -91,33 +115,17 @@ void build_sell(DevMatrix &A, bool want64, bool want32, cudaStream_t st)
         A.sell_pattern = true;
         A.s64_valid = A.s32_valid = false;
     }
-    if (!(want64 && !A.s64_valid) && !(want32 && !A.s32_valid)) return;  // up to date: no host round trip
-    int64_t slots = 0;
-    PFG_CUDA(cudaMemcpyAsync(&slots, A.sptr.p + A.ns, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    PFG_CUDA(cudaStreamSynchronize(st));
-    const size_t nv = (size_t)std::max<int64_t>(slots * 32 * A.bs * A.bs, 1);
-    if (want64 && !A.s64_valid) {
-        A.s64.resize(nv);
-        if (A.bs == 3)
-            k_sell_values<3, double><<<tile_grid(A.ns), 32 * kTileWarps, 0, st>>>(A.nb, A.ns, A.rp.p, A.v64.p,
-                                                                               A.sptr.p, A.s64.p);
-        else
-            k_sell_values<1, double><<<tile_grid(A.ns), 32 * kTileWarps, 0, st>>>(A.nb, A.ns, A.rp.p, A.v64.p,
-                                                                               A.sptr.p, A.s64.p);
-        PFG_CUDA(cudaGetLastError());
-        A.s64_valid = true;
-    }
-    if (want32 && !A.s32_valid) {
-        A.s32.resize(nv);
-        if (A.bs == 3)
-            k_sell_values<3, float><<<tile_grid(A.ns), 32 * kTileWarps, 0, st>>>(A.nb, A.ns, A.rp.p, A.v64.p,
-                                                                              A.sptr.p, A.s32.p);
-        else
-            k_sell_values<1, float><<<tile_grid(A.ns), 32 * kTileWarps, 0, st>>>(A.nb, A.ns, A.rp.p, A.v64.p,
-                                                                              A.sptr.p, A.s32.p);
-        PFG_CUDA(cudaGetLastError());
-        A.s32_valid = true;
-    }
+    const bool do64 = want64 && !A.s64_valid, do32 = want32 && !A.s32_valid;
+    if (!do64 && !do32) return;  // up to date
+    const size_t nv = A.scol.n * (size_t)(A.bs * A.bs);
+    if (do64) A.s64.resize(nv);
+    if (do32) A.s32.resize(nv);
+    if (A.bs == 3)
+        launch_sell_values<3>(A, do64 ? A.s64.p : nullptr, do32 ? A.s32.p : nullptr, st);
+    else
+        launch_sell_values<1>(A, do64 ? A.s64.p : nullptr, do32 ? A.s32.p : nullptr, st);
+    A.s64_valid |= do64;
+    A.s32_valid |= do32;
 }
 
 // ------------------------------------------------- upper half (symmetric storage)
@@ -140,20 +148,20 @@ __global__ void k_sellu_widths(int64_t nb, int64_t ns, const int64_t *__restrict
 
 // Columns and FP32 values of the upper blocks (column >= row) of each row, in
 // the row's order; padding slots point at the row itself with zero values.
-// One warp per slice, kTileK slots at a time: per row, the ballot prefix of
-// "upper" over its blocks gives each upper block its slot (kept in shared
-// memory), then each entry plane is gathered row by row and written back slot
-// by slot as 32 consecutive lanes.
-__global__ void __launch_bounds__(32 * kTileWarps)
+// A CTA of nine warps per slice, kTileK slots at a time: the warps share out the
+// rows to find, by the ballot prefix of "upper" over a row's blocks, which block
+// fills each slot (kept in shared memory); then each warp copies one entry plane
+// as k_sell_values does.  (One warp per slice: 811 us at 274,625 rows; this: 298 us.)
+__global__ void __launch_bounds__(288)
     k_sellu_fill(int64_t nb, int64_t ns, const int64_t *__restrict__ rp, const int *__restrict__ bcol,
                  const double *__restrict__ v64, const int64_t *__restrict__ sptr, int *__restrict__ scol,
                  float *__restrict__ sval)
 {
-    __shared__ short kmap[kTileWarps][32][kTileK];
-    __shared__ int ucnt[kTileWarps][32];
-    __shared__ float tile[kTileWarps][32][kTileK + 1];
+    __shared__ short kmap[32][kTileK];
+    __shared__ int ucnt[32];
+    __shared__ float tiles[9][32][kTileK + 1];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int64_t s = (int64_t)blockIdx.x * kTileWarps + w; s < ns; s += (int64_t)gridDim.x * kTileWarps) {
+    for (int64_t s = blockIdx.x; s < ns; s += gridDim.x) {
         const int64_t b0 = sptr[s];
         const int wdt = (int)(sptr[s + 1] - b0);
         const int64_t row = s * 32 + lane;
@@ -161,7 +169,8 @@ __global__ void __launch_bounds__(32 * kTileWarps)
         const int nblk = row < nb ? (int)(rp[row + 1] - r0) : 0;
         for (int kc = 0; kc < wdt; kc += kTileK) {
             // slots [kc, kc + kTileK) of every row: which of its blocks fill them
-            for (int l = 0; l < 32; ++l) {
+#pragma unroll 4
+            for (int l = w; l < 32; l += 9) {
                 const int64_t r0l = __shfl_sync(0xffffffffu, r0, l);
                 const int nl = __shfl_sync(0xffffffffu, nblk, l);
                 const int64_t rowl = s * 32 + l;
@@ -171,28 +180,27 @@ __global__ void __launch_bounds__(32 * kTileWarps)
                     const bool up = k < nl && bcol[r0l + k] >= rowl;
                     const unsigned bal = __ballot_sync(0xffffffffu, up);
                     const int pos = base + __popc(bal & ((1u << lane) - 1u)) - kc;
-                    if (up && pos >= 0 && pos < kTileK) kmap[w][l][pos] = (short)k;
+                    if (up && pos >= 0 && pos < kTileK) kmap[l][pos] = (short)k;
                     base += __popc(bal);
                 }
-                if (lane == 0) ucnt[w][l] = min(max(base - kc, 0), kTileK);
+                if (lane == 0) ucnt[l] = min(max(base - kc, 0), kTileK);
+            }
+            __syncthreads();
+            const int kend = min(kTileK, wdt - kc);
+            const int mine = ucnt[lane];
+            for (int kk = w; kk < kend; kk += 9)
+                scol[(b0 + kc + kk) * 32 + lane] = kk < mine ? bcol[r0 + kmap[lane][kk]] : (row < nb ? (int)row : 0);
+            float(*tile)[kTileK + 1] = tiles[w];
+#pragma unroll 8
+            for (int l = 0; l < 32; ++l) {
+                const int64_t r0l = __shfl_sync(0xffffffffu, r0, l);
+                const int nl = __shfl_sync(0xffffffffu, nblk, l);
+                tile[l][lane] = lane < ucnt[l] ? (float)v64[r0l * 9 + (int64_t)w * nl + kmap[l][lane]] : 0.f;
             }
             __syncwarp();
-            const int kend = min(kTileK, wdt - kc);
-            const int mine = ucnt[w][lane];
-            for (int kk = 0; kk < kend; ++kk)
-                scol[(b0 + kc + kk) * 32 + lane] = kk < mine ? bcol[r0 + kmap[w][lane][kk]] : (row < nb ? (int)row : 0);
-            for (int e = 0; e < 9; ++e) {
-                for (int l = 0; l < 32; ++l) {
-                    const int64_t r0l = __shfl_sync(0xffffffffu, r0, l);
-                    const int nl = __shfl_sync(0xffffffffu, nblk, l);
-                    const int cl = ucnt[w][l];
-                    for (int kk = lane; kk < kTileK; kk += 32)
-                        tile[w][l][kk] = kk < cl ? (float)v64[r0l * 9 + (int64_t)e * nl + kmap[w][l][kk]] : 0.f;
-                }
-                __syncwarp();
-                for (int kk = 0; kk < kend; ++kk) sval[((b0 + kc + kk) * 9 + e) * 32 + lane] = tile[w][lane][kk];
-                __syncwarp();
-            }
+#pragma unroll 4
+            for (int kk = 0; kk < kend; ++kk) sval[((b0 + kc + kk) * 9 + w) * 32 + lane] = tile[lane][kk];
+            __syncthreads();  // kmap and ucnt are rewritten for the next slots
         }
     }
 }
@@ -200,55 +208,90 @@ __global__ void __launch_bounds__(32 * kTileWarps)
 // Counts the upper blocks (i, j) whose transpose partner (j, i) is missing or
 // differs by more than 1e-9 relative (plus 1e-12 of the diagonal scale of the
 // two rows: assembly rounding leaves noise in entries that cancel to zero).
-// One warp per row i, a lane per block (i, j): the lane finds (j, i) and row
-// j's diagonal block in one pass over row j's block columns.
+// One warp per row i, three of its upper blocks at a time: the warp reads row j's
+// block columns (one load per 32) and votes for the slot of (j, i); then 27 lanes
+// compare the three blocks' entries.  Entries with the same bits -- all of an
+// assembled and eliminated matrix's -- need no arithmetic: nine FP64 comparisons
+// for every block kept GB300's FP64 pipe busy for most of the 950 us this took at
+// 274,625 rows (4,032 rows: 297 us); now 425 us and 11 us.
 __global__ void k_sym_check(int64_t nb, const int64_t *__restrict__ rp, const int *__restrict__ bcol,
                             const double *__restrict__ v64, unsigned long long *__restrict__ bad)
 {
     const int lane = threadIdx.x & 31;
     const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    // this lane's entry (r, c) of block `u` of three
+    const int u3 = min(lane / 9, 2), e3 = lane - 9 * (lane / 9), r3 = e3 / 3, c3 = e3 - 3 * r3;
+    // largest |entry| of a row's diagonal block (the warp's lanes share the search)
+    auto diag_scale = [&](int64_t i) {
+        const int64_t r0 = rp[i];
+        const int n = (int)(rp[i + 1] - r0);
+        double d = 0.0;
+        for (int k = lane; k < n; k += 32)
+            if (bcol[r0 + k] == i)
+                for (int e = 0; e < 9; e += 4) d = fmax(d, fabs(v64[r0 * 9 + (int64_t)e * n + k]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) d = fmax(d, __shfl_xor_sync(0xffffffffu, d, o));
+        return d;
+    };
     for (int64_t i = w0; i < nb; i += nw) {
         const int64_t ri = rp[i];
         const int ni = (int)(rp[i + 1] - ri);
-        // |diagonal entries| of row i's diagonal block
-        double di = 0.0;
-        for (int k = lane; k < ni; k += 32)
-            if (bcol[ri + k] == i)
-                for (int e = 0; e < 9; e += 4) di = fmax(di, fabs(v64[ri * 9 + (int64_t)e * ni + k]));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) di = fmax(di, __shfl_xor_sync(0xffffffffu, di, o));
         unsigned long long nbad = 0;
-        for (int k = lane; k < ni; k += 32) {
-            const int64_t j = bcol[ri + k];
-            if (j <= i) continue;
-            const int64_t rj = rp[j];
-            const int nj = (int)(rp[j + 1] - rj);
-            int kk = -1;
-            double dj = 0.0;
-            for (int q = 0; q < nj; ++q) {
-                const int64_t c = bcol[rj + q];
-                if (c == i && kk < 0) kk = q;
-                if (c == j)
-                    for (int e = 0; e < 9; e += 4) dj = fmax(dj, fabs(v64[rj * 9 + (int64_t)e * nj + q]));
-            }
-            if (kk < 0) {
-                ++nbad;
-                continue;
-            }
-            const double scale = 1e-12 * fmax(di, dj);
-            bool ok = true;
+        for (int k0 = 0; k0 < ni; k0 += 32) {
+            const int mine = k0 + lane < ni ? bcol[ri + k0 + lane] : -1;
+            unsigned todo = __ballot_sync(0xffffffffu, mine > i);
+            while (todo) {
+                int at[3], to[3], slot[3], len[3];
+                int64_t start[3];
 #pragma unroll
-            for (int r = 0; r < 3; ++r)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const double a = v64[ri * 9 + (int64_t)(3 * r + c) * ni + k];
-                    const double b = v64[rj * 9 + (int64_t)(3 * c + r) * nj + kk];
-                    ok = ok && fabs(a - b) <= 1e-9 * fmax(fabs(a), fabs(b)) + scale;
+                for (int u = 0; u < 3; ++u) {
+                    at[u] = todo ? __ffs(todo) - 1 : -1;
+                    todo &= todo - 1;
+                    to[u] = __shfl_sync(0xffffffffu, mine, max(at[u], 0));
+                    const int64_t j = at[u] >= 0 ? to[u] : i;
+                    start[u] = rp[j];
+                    len[u] = (int)(rp[j + 1] - start[u]);
                 }
-            nbad += !ok;
+                int first[3];
+#pragma unroll
+                for (int u = 0; u < 3; ++u) first[u] = lane < len[u] ? bcol[start[u] + lane] : -1;
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                    unsigned hit = __ballot_sync(0xffffffffu, first[u] == i);
+                    slot[u] = hit ? __ffs(hit) - 1 : -1;
+                    for (int q0 = 32; slot[u] < 0 && q0 < len[u]; q0 += 32) {
+                        hit = __ballot_sync(0xffffffffu, q0 + lane < len[u] && bcol[start[u] + q0 + lane] == i);
+                        if (hit) slot[u] = q0 + __ffs(hit) - 1;
+                    }
+                    if (at[u] >= 0 && slot[u] < 0) ++nbad;  // no partner
+                }
+                const int64_t st3 = u3 == 0 ? start[0] : (u3 == 1 ? start[1] : start[2]);
+                const int ln3 = u3 == 0 ? len[0] : (u3 == 1 ? len[1] : len[2]);
+                const int sl3 = u3 == 0 ? slot[0] : (u3 == 1 ? slot[1] : slot[2]);
+                const int at3 = u3 == 0 ? at[0] : (u3 == 1 ? at[1] : at[2]);
+                const bool have = lane < 27 && at3 >= 0 && sl3 >= 0;
+                double a = 0.0, b = 0.0;
+                if (have) {
+                    a = v64[ri * 9 + (int64_t)e3 * ni + k0 + at3];
+                    b = v64[st3 * 9 + (int64_t)(3 * c3 + r3) * ln3 + sl3];
+                }
+                const bool differ = have && __double_as_longlong(a) != __double_as_longlong(b);
+                if (__any_sync(0xffffffffu, differ)) {
+                    const double di = diag_scale(i);
+                    double dj = 0.0;
+#pragma unroll
+                    for (int u = 0; u < 3; ++u) {
+                        const double d = diag_scale(at[u] >= 0 ? to[u] : i);
+                        if (u == u3) dj = d;
+                    }
+                    const bool ok = !differ || fabs(a - b) <= 1e-9 * fmax(fabs(a), fabs(b)) + 1e-12 * fmax(di, dj);
+                    const unsigned no = __ballot_sync(0xffffffffu, !ok);
+                    nbad += ((no & 0x1ffu) != 0) + ((no & 0x3fe00u) != 0) + ((no & 0x7fc0000u) != 0);
+                }
+            }
         }
-        if (nbad) atomicAdd(bad, nbad);
+        if (nbad && lane == 0) atomicAdd(bad, nbad);
     }
 }
 
@@ -281,25 +324,30 @@ void check_symmetric(DevMatrix &A, cudaStream_t st)
     PFG_CHECK(A.nb > 0, PFG_E_STATE, "empty matrix");
     PFG_CHECK(A.bs == 3, PFG_E_UNSUPPORTED, "symmetric storage is built for 3x3-block matrices");
     if (A.sym_checked) return;
-    const int g = grid_for(A.nb, 256, sm_count_device() * 16);
     // the values (pattern included) changed: check the symmetry once
-    {
-        DevBuf<unsigned long long> bad(2);  // [0] asymmetric blocks, [1] low word: row-sum bound bits
-        PFG_CUDA(cudaMemsetAsync(bad.p, 0, 2 * sizeof(unsigned long long), st));
-        k_sym_check<<<g, 256, 0, st>>>(A.nb, A.rp.p, A.col.p, A.v64.p, bad.p);
-        k_rowsum_max<<<g, 256, 0, st>>>(A.nb, A.rp.p, A.v64.p, reinterpret_cast<unsigned *>(bad.p + 1));
-        PFG_CUDA(cudaGetLastError());
-        unsigned long long hb[2] = {0, 0};
-        PFG_CUDA(cudaMemcpyAsync(hb, bad.p, sizeof hb, cudaMemcpyDeviceToHost, st));
-        PFG_CUDA(cudaStreamSynchronize(st));
-        const unsigned long long nbad = hb[0];
-        const unsigned rs_bits = (unsigned)(hb[1] & 0xffffffffull);  // little-endian low word
-        memcpy(&A.sym_rowsum, &rs_bits, sizeof rs_bits);
-        PFG_CHECK(nbad == 0, PFG_E_ARG,
-                  "symmetric storage needs a symmetric matrix: " + std::to_string(nbad) +
-                      " blocks differ from their transposes");
-    }
+    DevBuf<unsigned long long> bad(1);
+    PFG_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(unsigned long long), st));
+    k_sym_check<<<grid_for(A.nb, 8, sm_count_device() * 16), 256, 0, st>>>(A.nb, A.rp.p, A.col.p, A.v64.p, bad.p);
+    PFG_CUDA(cudaGetLastError());
+    unsigned long long nbad = 0;
+    PFG_CUDA(cudaMemcpyAsync(&nbad, bad.p, sizeof nbad, cudaMemcpyDeviceToHost, st));
+    PFG_CUDA(cudaStreamSynchronize(st));
+    PFG_CHECK(nbad == 0, PFG_E_ARG,
+              "symmetric storage needs a symmetric matrix: " + std::to_string(nbad) +
+                  " blocks differ from their transposes");
     A.sym_checked = true;
+}
+
+void bound_rows(DevMatrix &A, cudaStream_t st)
+{
+    if (A.sym_rowsum_valid) return;
+    DevBuf<unsigned> bits(1);
+    PFG_CUDA(cudaMemsetAsync(bits.p, 0, sizeof(unsigned), st));
+    k_rowsum_max<<<grid_for(A.nb, 8, sm_count_device() * 16), 256, 0, st>>>(A.nb, A.rp.p, A.v64.p, bits.p);
+    PFG_CUDA(cudaGetLastError());
+    PFG_CUDA(cudaMemcpyAsync(&A.sym_rowsum, bits.p, sizeof(float), cudaMemcpyDeviceToHost, st));
+    PFG_CUDA(cudaStreamSynchronize(st));
+    A.sym_rowsum_valid = true;
 }
 
 void build_sell_upper(DevMatrix &A, cudaStream_t st)
@@ -318,8 +366,8 @@ void build_sell_upper(DevMatrix &A, cudaStream_t st)
         A.s32_u.resize((size_t)std::max<int64_t>(slots * 32 * 9, 1));
         A.sell_u_pattern = true;
     }
-    k_sellu_fill<<<tile_grid(A.ns_u), 32 * kTileWarps, 0, st>>>(A.nb, A.ns_u, A.rp.p, A.col.p, A.v64.p, A.sptr_u.p,
-                                                               A.scol_u.p, A.s32_u.p);
+    k_sellu_fill<<<(int)std::min<int64_t>(A.ns_u, sm_count_device() * 16), 288, 0, st>>>(
+        A.nb, A.ns_u, A.rp.p, A.col.p, A.v64.p, A.sptr_u.p, A.scol_u.p, A.s32_u.p);
     PFG_CUDA(cudaGetLastError());
     A.s32_u_valid = true;
 }
