@@ -216,6 +216,15 @@ __global__ void __launch_bounds__(kThreads) k_residual64(SellView<double> A, con
     }
 }
 
+// The solver's inverse diagonal blocks are kept in planes, as the sliced matrix is:
+// entry e of row's block at pc_at(row) + 32 e, so the 32 lanes of a warp read each
+// entry as one line (block by block, a warp's nine loads touch 81 lines).
+template <int BS>
+__device__ __forceinline__ int64_t pc_at(int64_t row)
+{
+    return (row >> 5) * (32 * BS * BS) + (row & 31);
+}
+
 template <int BS, typename T>
 __device__ __forceinline__ void pc_apply(int pc, const T *__restrict__ dinv, int64_t row, const T (&r)[BS],
                                          T (&z)[BS])
@@ -225,12 +234,12 @@ __device__ __forceinline__ void pc_apply(int pc, const T *__restrict__ dinv, int
         for (int i = 0; i < BS; ++i) z[i] = r[i];
         return;
     }
-    const T *D = dinv + row * (BS * BS);
+    const T *D = dinv + pc_at<BS>(row);
 #pragma unroll
     for (int i = 0; i < BS; ++i) {
         T s = T(0);
 #pragma unroll
-        for (int j = 0; j < BS; ++j) s = fma(__ldg(D + i * BS + j), r[j], s);
+        for (int j = 0; j < BS; ++j) s = fma(__ldg(D + (i * BS + j) * 32), r[j], s);
         z[i] = s;
     }
 }
@@ -239,7 +248,7 @@ __device__ __forceinline__ void pc_apply(int pc, const T *__restrict__ dinv, int
 // diagonal entries only (point Jacobi).  A zero pivot keeps the identity, as
 // JacobiPreconditionerCRS skips rows with A_kk == 0 (FEMSolverClass.f90:2519).
 template <int BS>
-__global__ void k_precond(BsrView<double> A, int pc, double *__restrict__ d64, float *__restrict__ d32)
+__global__ void k_precond(BsrView<double> A, int pc, double *__restrict__ d64, float *__restrict__ d32, bool planes)
 {
     for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < A.nb;
          row += (int64_t)gridDim.x * blockDim.x) {
@@ -284,8 +293,9 @@ __global__ void k_precond(BsrView<double> A, int pc, double *__restrict__ d64, f
         }
 #pragma unroll
         for (int e = 0; e < BS * BS; ++e) {
-            d64[row * BS * BS + e] = Inv[e];
-            if (d32) d32[row * BS * BS + e] = (float)Inv[e];
+            const int64_t o = planes ? pc_at<BS>(row) + 32 * e : row * BS * BS + e;
+            d64[o] = Inv[e];
+            if (d32) d32[o] = (float)Inv[e];
         }
     }
 }
@@ -373,6 +383,22 @@ __global__ void __launch_bounds__(kThreads) k_cg_dir(int64_t n, const T *__restr
     const T beta = st_beta<T>(S);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         p[i] = fma(beta, p[i], z[i]);
+}
+
+// The FP32 direction pass of the symmetric path, 16 bytes at a time.
+__global__ void __launch_bounds__(kThreads)
+    k_cg_dir_sym(int64_t n, const float *__restrict__ z, float *__restrict__ p, KState *S)
+{
+    if (S->done | S->need_update) return;
+    const float beta = S->beta32;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    const float4 *z4 = reinterpret_cast<const float4 *>(z);
+    float4 *p4 = reinterpret_cast<float4 *>(p);
+    for (int64_t i = t; i < n / 4; i += stride) {
+        const float4 a = p4[i], b = z4[i];
+        p4[i] = make_float4(fmaf(beta, a.x, b.x), fmaf(beta, a.y, b.y), fmaf(beta, a.z, b.z), fmaf(beta, a.w, b.w));
+    }
+    if (t < n % 4) p[n - 1 - t] = fmaf(beta, p[n - 1 - t], z[n - 1 - t]);
 }
 
 // q = A p; pq = p.q; fin: alpha = rho / pq.
@@ -1731,20 +1757,20 @@ void block_jacobi_inverse(const DevMatrix &A, int pc, double *d64, cudaStream_t 
 {
     const int g = grid_for(A.nb, 256, sm_count() * 8);
     if (A.bs == 3)
-        k_precond<3><<<g, 256, 0, st>>>(A.view<double>(), pc, d64, nullptr);
+        k_precond<3><<<g, 256, 0, st>>>(A.view<double>(), pc, d64, nullptr, false);
     else
-        k_precond<1><<<g, 256, 0, st>>>(A.view<double>(), pc, d64, nullptr);
+        k_precond<1><<<g, 256, 0, st>>>(A.view<double>(), pc, d64, nullptr, false);
     PFG_CUDA(cudaGetLastError());
 }
 
-void block_jacobi(const DevMatrix &A, int precond, double *d64, float *d32, cudaStream_t st)
+void block_jacobi(const DevMatrix &A, int precond, double *d64, float *d32, cudaStream_t st, bool planes)
 {
     if (precond == PFG_PC_NONE || A.nb == 0) return;
     const int g = grid_for(A.nb, 256, sm_count() * 8);
     if (A.bs == 3)
-        k_precond<3><<<g, 256, 0, st>>>(A.view<double>(), precond, d64, d32);
+        k_precond<3><<<g, 256, 0, st>>>(A.view<double>(), precond, d64, d32, planes);
     else
-        k_precond<1><<<g, 256, 0, st>>>(A.view<double>(), precond, d64, d32);
+        k_precond<1><<<g, 256, 0, st>>>(A.view<double>(), precond, d64, d32, planes);
     PFG_CUDA(cudaGetLastError());
 }
 
@@ -1755,11 +1781,11 @@ void Krylov::build_precond(const DevMatrix &A, int precond, bool fp32, cudaStrea
     if (dinv_gen_ == A.value_gen && dinv_pc_ == precond &&
         (!fp32 || (dinv32_gen_ == A.value_gen && dinv32_pc_ == precond)))
         return;
-    const size_t m = (size_t)std::max<int64_t>(A.nb * A.bs * A.bs, 1);
+    const size_t m = (size_t)((A.nb + 31) / 32 * 32 * A.bs * A.bs);
     dinv_gen_ = dinv32_gen_ = 0;
     dinv_.ensure(m);
     if (fp32) dinv32_.ensure(m);
-    block_jacobi(A, precond, dinv_.p, fp32 ? dinv32_.p : nullptr, st);
+    block_jacobi(A, precond, dinv_.p, fp32 ? dinv32_.p : nullptr, st, true);
     ++launches_;
     dinv_gen_ = A.value_gen;
     dinv_pc_ = precond;
@@ -1952,7 +1978,7 @@ static int cg_chunk_sym(const SellView<float> &U, bool fuse, int chunk, int64_t 
                         unsigned *tk, double tol, double delta, int itrmax, cudaStream_t st)
 {
     const int64_t n = nb * 3;
-    const int gd = resident_grid(k_cg_dir<float>, (n + 31) / 32);
+    const int gd = resident_grid(k_cg_dir_sym, (n + 127) / 128);
     const int gu = resident_grid(k_cg_update<3, float, 4>, (nb + 31) / 32);
     for (int it = 0; it < chunk; ++it) {
         if (fuse) {  // direction update inside the product (ping-pong pA / pB)
@@ -1960,7 +1986,7 @@ static int cg_chunk_sym(const SellView<float> &U, bool fuse, int chunk, int64_t 
             k_cg_update<3, float, 4><<<gu, kThreads, 0, st>>>(nb, x, r, z, pA, pB, q4, dinv, pc, S, pd, pf, tk, tol,
                                                               delta, itrmax);
         } else {
-            k_cg_dir<float><<<gd, kThreads, 0, st>>>(n, z, pA, S);
+            k_cg_dir_sym<<<gd, kThreads, 0, st>>>(n, z, pA, S);
             launch_cg_spmv_sym(false, U, nullptr, pA, nullptr, q4, S, pd, pf, tk, st);
             k_cg_update<3, float, 4><<<gu, kThreads, 0, st>>>(nb, x, r, z, pA, pA, q4, dinv, pc, S, pd, pf, tk, tol,
                                                               delta, itrmax);

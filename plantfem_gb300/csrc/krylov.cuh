@@ -148,8 +148,8 @@ inline SellView<float> sell_upper(const DevMatrix &A)
 
 // Inverse of every diagonal block (PFG_PC_BLOCK_JACOBI) or diagonal entry
 // (PFG_PC_JACOBI) of A into d64 (and d32 unless null), BS*BS values per block
-// row.  Implemented in krylov.cu.
-void block_jacobi(const DevMatrix &A, int precond, double *d64, float *d32, cudaStream_t st);
+// row (`planes`: entry planes of 32 rows instead).  Implemented in krylov.cu.
+void block_jacobi(const DevMatrix &A, int precond, double *d64, float *d32, cudaStream_t st, bool planes = false);
 
 class Ilu0;
 struct ResPlan;

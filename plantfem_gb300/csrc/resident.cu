@@ -1004,14 +1004,17 @@ struct Own {
                 }
         }
     }
-    // planes k .. k + BS - 1 (BS * BS per slice) = the rows' inverse diagonal blocks
+    // the rows' inverse diagonal blocks (planes: BS * BS of 32 per slice), in shared
+    // memory as vectors k .. k + BS - 1 if those are
     __device__ const T *planes(const Grid &g, int k, const T *dinv, int64_t nb) const
     {
-        T *o = k + BS <= count ? reinterpret_cast<T *>(near) + k * n : home + k * all + (size_t)g.s0 * (BS - 1) * BS * 32;
+        const T *far = dinv + (size_t)g.s0 * (BS * BS * 32);
+        if (k + BS > count) return far;
+        T *o = reinterpret_cast<T *>(near) + k * n;
         RES_ROWS(g, nb)
 #pragma unroll
         for (int e = 0; e < BS * BS; ++e)
-            o[(sl * BS * BS + e) * 32 + g.lane] = __ldg(dinv + row * (BS * BS) + e);
+            o[(sl * BS * BS + e) * 32 + g.lane] = __ldg(far + (sl * BS * BS + e) * 32 + g.lane);
         return o;
     }
 };
@@ -1550,7 +1553,7 @@ ResPlan plan_resident(const DevMatrix &A, int algorithm, bool mixed, bool precon
     pl.stages = stages;
     pl.near = near;
     pl.smem = fixed + (size_t)near * vec + (size_t)stages * stage;
-    pl.home_bytes = (size_t)pl.vectors * (size_t)A.ns * plane * word;
+    pl.home_bytes = (size_t)(pl.vectors - (precond ? A.bs : 0)) * (size_t)A.ns * plane * word;
     return pl;
 }
 
