@@ -181,6 +181,54 @@ __global__ void __launch_bounds__(kThreads) k_spmv_sell(SellView<T> A, const T *
     }
 }
 
+// y = A x with a CTA of kWarps warps per slice: each takes an eighth of the slots,
+// the sums are added in warp order.  Both ends gain from the fine split: a warp per
+// slice puts a 1,430-row matrix on 6 SMs, each bound by its FP64 pipe (a slice of 27
+// slots is 3,900 of its cycles), and leaves whole slices as the last wave's grain.
+// The caller's call, us, warp per slice -> this: 343 rows 34.7 -> 21.5, 9,261 rows
+// 34.8 -> 23.3, 19,683 rows 35.2 -> 30.2, 35,937 rows 48.8 -> 38.3, 117,649 rows
+// 82.9 -> 74.2, 531,441 rows 265 -> 253, 1.03M rows 471 -> 470 (about 18 us of each
+// are the call's own; the FP64 pipe's share at 1.03M rows is 420 us).
+template <int BS, typename T>
+__global__ void __launch_bounds__(kThreads) k_spmv_split(SellView<T> A, const T *__restrict__ x, T *__restrict__ y)
+{
+    __shared__ T part[kWarps][BS][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int64_t s = blockIdx.x; s < A.ns; s += gridDim.x) {
+        const int64_t b0 = A.sptr[s];
+        const int wdt = (int)(A.sptr[s + 1] - b0);
+        const int k0 = wdt * w / kWarps, k1 = wdt * (w + 1) / kWarps;
+        T acc[BS];
+#pragma unroll
+        for (int i = 0; i < BS; ++i) acc[i] = T(0);
+#pragma unroll 4
+        for (int k = k0; k < k1; ++k) {
+            T a[BS * BS], xv[BS];
+            const int c = ld_stream(A.col + (b0 + k) * 32 + lane);
+#pragma unroll
+            for (int e = 0; e < BS * BS; ++e) a[e] = ld_stream(A.val + ((b0 + k) * (BS * BS) + e) * 32 + lane);
+#pragma unroll
+            for (int i = 0; i < BS; ++i) xv[i] = __ldg(x + (int64_t)BS * c + i);
+#pragma unroll
+            for (int i = 0; i < BS; ++i)
+#pragma unroll
+                for (int j = 0; j < BS; ++j) acc[i] = fma(a[i * BS + j], xv[j], acc[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < BS; ++i) part[w][i][lane] = acc[i];
+        __syncthreads();
+        for (int t = threadIdx.x; t < BS * 32; t += kThreads) {
+            const int i = t >> 5, l = t & 31;
+            T v = part[0][i][l];
+#pragma unroll
+            for (int q = 1; q < kWarps; ++q) v += part[q][i][l];
+            const int64_t row = s * 32 + l;
+            if (row < A.nb) y[BS * row + i] = v;
+        }
+        __syncthreads();
+    }
+}
+
 // r = b - A x in FP64; totals: true_rr = r.r and bb = b.b into KState.
 template <int BS>
 __global__ void __launch_bounds__(kThreads) k_residual64(SellView<double> A, const double *__restrict__ b,
@@ -1667,12 +1715,11 @@ void Krylov::spmv64_sliced(DevMatrix &A, const double *x, double *y, cudaStream_
 {
     if (A.nb == 0) return;
     build_sell(A, true, false, st);
+    const int g = (int)std::min<int64_t>(A.ns, 1 << 20);
     if (A.bs == 3)
-        k_spmv_sell<3, double><<<resident_grid(k_spmv_sell<3, double>, A.ns), kThreads, 0, st>>>(A.sell<double>(), x,
-                                                                                                 y);
+        k_spmv_split<3, double><<<g, kThreads, 0, st>>>(A.sell<double>(), x, y);
     else
-        k_spmv_sell<1, double><<<resident_grid(k_spmv_sell<1, double>, A.ns), kThreads, 0, st>>>(A.sell<double>(), x,
-                                                                                                 y);
+        k_spmv_split<1, double><<<g, kThreads, 0, st>>>(A.sell<double>(), x, y);
     PFG_CUDA(cudaGetLastError());
 }
 
@@ -2139,7 +2186,7 @@ constexpr int kResidentBudget = 4096;
 SolveResult Krylov::run_resident(DevMatrix &A, const double *b, double *x, const KConfig &cfg, const ResPlan &plan,
                                  cudaStream_t st)
 {
-    const bool mixed = cfg.precision == PFG_PREC_MIXED, pc = cfg.precond != PFG_PC_NONE;
+    const bool mixed = cfg.precision == PFG_PREC_MIXED;
     build_precond(A, cfg.precond, mixed, st);
     if (!host_res_) {
         PFG_CUDA(cudaMallocHost((void **)&host_res_, sizeof(ResState)));
