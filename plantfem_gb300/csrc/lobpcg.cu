@@ -617,6 +617,14 @@ __device__ __forceinline__ float2 df_add(float2 a, float2 b)
     return make_float2(t, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z2)), __fsub_rn(e, z2)));
 }
 
+// The blocks of the iteration's three linear combinations (the vectors, their K and
+// their M images): one launch, blockIdx.y picks.
+template <typename T>
+struct CombSet {
+    const T *X[3], *W[3], *P[3];
+    T *Xn[3], *Pn[3];
+};
+
 // Y = A X for every panel (one warp per (slice, panel), one lane per block
 // row); rows of fixed DOFs are zeroed (the reduce_crs_matrix restriction).
 template <int BS, typename T>
@@ -735,12 +743,179 @@ __global__ void __launch_bounds__(kT) k_spmm_df(SellView<double> A, const float2
     }
 }
 
+// The products with kParts<T> warps per (slice, panel), each with a run of the
+// slice's slots, the parts added in order: for systems whose slices and panels alone
+// do not fill the GPU with warps.  A warp's slots are a chain of dependent loads (column,
+// then three panel rows), 27 of them in a hex mesh: 49 us per launch at 31,775 rows
+// and two panels, whatever the bytes.  PAIR (FP32, K and M of one pattern): both
+// products in one pass, so the columns and the panel rows, most of the traffic, are
+// read once.  Measured there: K X and M X 94 -> 30 us (FP32; two parts 35, eight 42), one
+// double-float product 96 -> 55 us (four parts 73, eight 83).
+template <typename T>
+constexpr int kParts = std::is_same<T, float2>::value ? 2 : 4;
+
+template <typename T>
+struct MulAcc;
+template <>
+struct MulAcc<float> {
+    using Value = float;
+    float v;
+    __device__ void zero() { v = 0.f; }
+    __device__ void add(float a, float x) { v = fmaf(a, x, v); }
+    __device__ float get() const { return v; }
+    __device__ static float sum(float a, float b) { return a + b; }
+    __device__ static float none() { return 0.f; }
+};
+template <>
+struct MulAcc<float2> {
+    using Value = float2;
+    DFAcc v;
+    __device__ void zero() { v.zero(); }
+    __device__ void add(float2 a, float2 x) { v.add(a, x); }
+    __device__ float2 get() const { return v.get2(); }
+    __device__ static float2 sum(float2 a, float2 b) { return df_add(a, b); }
+    __device__ static float2 none() { return make_float2(0.f, 0.f); }
+};
+
+// the first NC columns of a panel row, 16 bytes a load
+template <int NC>
+__device__ __forceinline__ void ld_cols(const float *p, float (&v)[PW])
+{
+#pragma unroll
+    for (int u = 0; u < NC / 4; ++u) {
+        const float4 w = __ldg(reinterpret_cast<const float4 *>(p) + u);
+        v[4 * u] = w.x;
+        v[4 * u + 1] = w.y;
+        v[4 * u + 2] = w.z;
+        v[4 * u + 3] = w.w;
+    }
+}
+template <int NC>
+__device__ __forceinline__ void ld_cols(const float2 *p, float2 (&v)[PW])
+{
+#pragma unroll
+    for (int u = 0; u < NC / 2; ++u) {
+        const float4 w = __ldg(reinterpret_cast<const float4 *>(p) + u);
+        v[2 * u] = make_float2(w.x, w.y);
+        v[2 * u + 1] = make_float2(w.z, w.w);
+    }
+}
+
+// Slots [k0, k1) of a lane's row times the first NC columns of panel q.
+template <int BS, int NC, typename T, int NM>
+__device__ __forceinline__ void spmm_slots(int64_t b0, int k0, int k1, int lane, const int *__restrict__ scol,
+                                           const T *__restrict__ v0, const T *__restrict__ v1, int64_t n, int q,
+                                           const T *__restrict__ X, MulAcc<T> (&acc)[NM][BS][PW])
+{
+    for (int k = k0; k < k1; ++k) {
+        const int col = ld_stream(scol + (b0 + k) * 32 + lane);
+        T a[NM][BS * BS];
+#pragma unroll
+        for (int e = 0; e < BS * BS; ++e) {
+            const int64_t o = ((b0 + k) * (BS * BS) + e) * 32 + lane;
+            a[0][e] = __ldg(v0 + o);
+            if (NM == 2) a[NM - 1][e] = __ldg(v1 + o);
+        }
+#pragma unroll
+        for (int cc = 0; cc < BS; ++cc) {
+            T xv[PW];
+            ld_cols<NC>(panel_row(X, n, q, (int64_t)BS * col + cc), xv);
+#pragma unroll
+            for (int m = 0; m < NM; ++m)
+#pragma unroll
+                for (int r = 0; r < BS; ++r)
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) acc[m][r][c].add(a[m][r * BS + cc], xv[c]);
+        }
+    }
+}
+
+// A's pattern with two sets of values (v1 unused without PAIR); a last panel of at
+// most four columns is computed as four (its padding stays zero)
+template <int BS, typename T, bool PAIR>
+__global__ void __launch_bounds__(kT)
+    k_spmm_parts(int64_t nb, int64_t ns, const int64_t *__restrict__ sptr, const int *__restrict__ scol,
+                 const T *__restrict__ v0, const T *__restrict__ v1, int np, int cols,
+                 const T *__restrict__ X, T *__restrict__ Y0, T *__restrict__ Y1, const uint8_t *__restrict__ fixed)
+{
+    using A = MulAcc<T>;
+    constexpr int NM = PAIR ? 2 : 1, kGroups = kT / 32 / kParts<T>;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    T *sm = reinterpret_cast<T *>(smraw);  // [group][part - 1][matrix][r][c][lane]
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, grp = w / kParts<T>, part = w % kParts<T>;
+    const int64_t n = nb * BS;
+    for (int64_t u0 = (int64_t)blockIdx.x * kGroups; u0 < ns * np; u0 += (int64_t)gridDim.x * kGroups) {
+        const int64_t u = u0 + grp;
+        const bool on = u < ns * np;
+        const int64_t s = on ? u / np : 0;
+        const int q = on ? (int)(u - s * np) : 0;
+        A acc[NM][BS][PW];
+#pragma unroll
+        for (int m = 0; m < NM; ++m)
+#pragma unroll
+            for (int r = 0; r < BS; ++r)
+#pragma unroll
+                for (int c = 0; c < PW; ++c) acc[m][r][c].zero();
+        if (on) {
+            const int64_t b0 = sptr[s];
+            const int wdt = (int)(sptr[s + 1] - b0);
+            const int k0 = wdt * part / kParts<T>, k1 = wdt * (part + 1) / kParts<T>;
+            if (cols - q * PW > PW / 2)
+                spmm_slots<BS, PW, T, NM>(b0, k0, k1, lane, scol, v0, v1, n, q, X, acc);
+            else
+                spmm_slots<BS, PW / 2, T, NM>(b0, k0, k1, lane, scol, v0, v1, n, q, X, acc);
+        }
+        T *mine = sm + (size_t)(grp * (kParts<T> - 1) + part - 1) * (NM * BS * PW * 32) + lane;
+        if (part > 0)
+#pragma unroll
+            for (int m = 0; m < NM; ++m)
+#pragma unroll
+                for (int r = 0; r < BS; ++r)
+#pragma unroll
+                    for (int c = 0; c < PW; ++c) mine[((m * BS + r) * PW + c) * 32] = acc[m][r][c].get();
+        __syncthreads();
+        const int64_t row = s * 32 + lane;
+        if (part == 0 && on && row < nb) {
+            const T *first = sm + (size_t)grp * (kParts<T> - 1) * (NM * BS * PW * 32) + lane;
+#pragma unroll
+            for (int m = 0; m < NM; ++m)
+#pragma unroll
+                for (int r = 0; r < BS; ++r) {
+                    const int64_t i = (int64_t)BS * row + r;
+                    const bool f = fixed && fixed[i];
+                    T yv[PW];
+#pragma unroll
+                    for (int c = 0; c < PW; ++c) {
+                        T v = acc[m][r][c].get();
+#pragma unroll
+                        for (int g = 0; g < kParts<T> - 1; ++g)
+                            v = A::sum(v, first[(size_t)g * (NM * BS * PW * 32) + ((m * BS + r) * PW + c) * 32]);
+                        yv[c] = f ? A::none() : v;
+                    }
+                    st_row((m == 0 ? Y0 : Y1) + ((int64_t)q * n + i) * PW, yv);
+                }
+        }
+        __syncthreads();
+    }
+}
+
+// *same = 0 where two arrays differ
+template <typename I>
+__global__ void k_compare(int64_t n, const I *__restrict__ a, const I *__restrict__ b, int *same)
+{
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        if (a[i] != b[i]) *same = 0;
+}
+
 // k_lincomb with the blocks, the coefficients and the results in double-float.
 __global__ void __launch_bounds__(kT)
-    k_lincomb_df(int64_t n, int k, int nblk, const float2 *__restrict__ X, const float2 *__restrict__ W,
-                 const float2 *__restrict__ P, const double *__restrict__ C, float2 *__restrict__ Xn,
-                 float2 *__restrict__ Pn)
+    k_lincomb_df(int64_t n, int k, int nblk, const CombSet<float2> set, const double *__restrict__ C)
 {
+    const float2 *__restrict__ X = set.X[blockIdx.y];
+    const float2 *__restrict__ W = set.W[blockIdx.y];
+    const float2 *__restrict__ P = set.P[blockIdx.y];
+    float2 *__restrict__ Xn = set.Xn[blockIdx.y];
+    float2 *__restrict__ Pn = set.Pn[blockIdx.y];
     extern __shared__ __align__(16) unsigned char smraw[];
     float2 *sC = (float2 *)smraw;
     const int m = nblk * k;
@@ -892,10 +1067,10 @@ __device__ __forceinline__ void gram_lds4(const float2 *p, float2 (&v)[kGramSub]
 // p = (i, j), i <= j, numbered row by row over the upper triangle of the
 // m = nblk k real columns.
 //
-// Register-tiled outer products: the padded m_p x m_p matrix is cut into 8 x 8
-// tiles; the upper-triangle tiles (I <= J) are split into four 4 x 4 sub-tiles,
-// one per thread (4 * T (T + 1) / 2 threads for T = m_p / 8 tile columns, at
-// most 312).  A step stages kGramRows rows of every panel of S, K S and M S
+// Register-tiled outer products: each block's k columns are cut into groups of
+// four, and a thread takes the 4 x 4 tile of a pair of groups I <= J (G (G + 1) / 2
+// threads for G = nblk ceil(k / 4) groups, at most 300; no tile below the diagonal
+// and none of the padding alone: 45 threads at k = 12 where 8 x 8 tiles took 84).  A step stages kGramRows rows of every panel of S, K S and M S
 // into shared memory, one panel tile after another: the rows of a panel are
 // contiguous in global memory, so each warp copies whole tiles with 16-byte
 // loads.  Per staged row a thread reads its 4 values of S and 4 of each image
@@ -903,8 +1078,7 @@ __device__ __forceinline__ void gram_lds4(const float2 *p, float2 (&v)[kGramSub]
 // (per CTA row range; the ranges are summed in FP64), FP64 for FP64 panels,
 // or double-float (DF: double-float panels of the mixed mode's second phase)
 // on the FP32 pipe.  Padding columns are staged as they are
-// stored and their sums are not written; the sub-tile below the diagonal of
-// a diagonal tile is computed and not written.
+// stored and their sums are not written.
 template <typename T, bool DF>
 __global__ void __launch_bounds__(320)
     k_gram(int64_t n, int k, int nblk, const T *S0, const T *S1, const T *S2, const T *K0, const T *K1, const T *K2,
@@ -917,7 +1091,8 @@ __global__ void __launch_bounds__(320)
     const int m = nblk * k;
     const int npairs = m * (m + 1) / 2;
     const int tiles = mp / PW;
-    const int ntasks = kGramSub * tiles * (tiles + 1) / 2;
+    const int per_block = (k + kGramSub - 1) / kGramSub, groups = nblk * per_block;
+    const int ntasks = groups * (groups + 1) / 2;
     using Ar = GramArith<T, DF>;
     using St = typename Ar::Stage;
     constexpr int TE = gram_tile_elems<St>();
@@ -925,16 +1100,17 @@ __global__ void __launch_bounds__(320)
     const bool active = (int)threadIdx.x < ntasks;
     int ti = 0, tj = 0, oi = 0, oj = 0;
     if (active) {
-        const int tp = threadIdx.x >> 2, sub = threadIdx.x & 3;
-        int I = 0, rem = tp;
-        while (rem >= tiles - I) {
-            rem -= tiles - I;
+        int I = 0, rem = threadIdx.x;
+        while (rem >= groups - I) {
+            rem -= groups - I;
             ++I;
         }
-        ti = I;
-        tj = I + rem;
-        oi = kGramSub * (sub >> 1);
-        oj = kGramSub * (sub & 1);
+        const int J = I + rem;
+        const int ci = I % per_block * kGramSub, cj = J % per_block * kGramSub;  // within the blocks
+        ti = I / per_block * np + ci / PW;
+        tj = J / per_block * np + cj / PW;
+        oi = ci % PW;
+        oj = cj % PW;
     }
     typename Ar::Acc aA[kGramSub][kGramSub], aB[kGramSub][kGramSub];
 #pragma unroll
@@ -995,14 +1171,46 @@ __global__ void __launch_bounds__(320)
         }
 }
 
-// Sum the per-CTA partials in CTA order (deterministic).
-__global__ void k_reduce_parts(const double *__restrict__ part, int nparts, int len, double *__restrict__ out)
+// Sum the per-CTA partials (deterministic): a CTA takes 32 values, its 32 warps a
+// share of the partials each, added in warp order.  (A thread per value that ran
+// through the partials alone: 55 us for 304 partials of 1,332 values; this 15.)
+__global__ void __launch_bounds__(1024)
+    k_reduce_parts(const double *__restrict__ part, int nparts, int len, double *__restrict__ out)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int b = 0; b < nparts; ++b) s += part[(int64_t)b * len + i];
-        out[i] = s;
+    __shared__ double sums[32][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    double s = 0.0;
+    if (i < len)
+#pragma unroll 8
+        for (int b = w; b < nparts; b += 32) s += part[(int64_t)b * len + i];
+    sums[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && i < len) {
+        double t = 0.0;
+        for (int k = 0; k < 32; ++k) t += sums[k][lane];
+        out[i] = t;
     }
+}
+
+// The residuals' partials (per column |R|^2, |MX|^2, max|R|) of nparts CTAs: a warp
+// per entry.
+__global__ void k_reduce_residual(const double *__restrict__ part, int nparts, int len, double *__restrict__ out)
+{
+    const int lane = threadIdx.x & 31, e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (e >= len) return;
+    const bool top = e % 3 == 2;
+    double v = 0.0;
+    for (int b = lane; b < nparts; b += 32) {
+        const double x = part[(int64_t)b * len + e];
+        v = top ? fmax(v, x) : v + x;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double x = __shfl_xor_sync(0xffffffffu, v, o);
+        v = top ? fmax(v, x) : v + x;
+    }
+    if (lane == 0) out[e] = v;
 }
 
 // Pn = W C_w + P C_p ; Xn = X C_x + Pn   (C: m x k column-major, FP64).
@@ -1013,9 +1221,13 @@ __global__ void k_reduce_parts(const double *__restrict__ part, int nparts, int 
 // move with 16-byte accesses.
 template <typename T>
 __global__ void __launch_bounds__(kT)
-    k_lincomb(int64_t n, int k, int nblk, const T *__restrict__ X, const T *__restrict__ W, const T *__restrict__ P,
-              const double *__restrict__ C, T *__restrict__ Xn, T *__restrict__ Pn)
+    k_lincomb(int64_t n, int k, int nblk, const CombSet<T> set, const double *__restrict__ C)
 {
+    const T *__restrict__ X = set.X[blockIdx.y];
+    const T *__restrict__ W = set.W[blockIdx.y];
+    const T *__restrict__ P = set.P[blockIdx.y];
+    T *__restrict__ Xn = set.Xn[blockIdx.y];
+    T *__restrict__ Pn = set.Pn[blockIdx.y];
     extern __shared__ __align__(16) unsigned char smraw[];
     T *sC = (T *)smraw;
     const int m = nblk * k;
@@ -1061,20 +1273,52 @@ __global__ void __launch_bounds__(kT)
 
 // R = KX - MX diag(lam); per column: |R_j|^2, |MX_j|^2, max|R_j|  -> part[cta][3k]
 // (entry 3 j + {0, 1, 2} of CTA x's row).  CTA (x, q) takes the rows of panel
-// q, so a thread's sums are 3 x 8 registers and its rows move as vectors.
+// q, so a thread's sums are 3 x 8 registers and its rows move as vectors.  The
+// sums are FP64 (no FP32 underflow of squares for badly scaled systems); what bounds
+// a small system is adding them across the CTA on the FP64 pipe, so the 16 sums
+// are halved from lane to lane (16 additions per warp instead of 80) and FP32
+// maxima stay FP32: 56 -> 22 us at 95k rows, k = 12.
+// double-float panels: the difference on the FP32 pipe (lam split once per
+// column), the sums of the leading floats (seven digits are all a norm needs).
+__device__ __forceinline__ float res_lam(float, double l) { return (float)l; }
+__device__ __forceinline__ double res_lam(double, double l) { return l; }
+__device__ __forceinline__ float2 res_lam(float2, double l) { return df_split(-l); }
+__device__ __forceinline__ float res_diff(float k, float m, float l) { return k - m * l; }
+__device__ __forceinline__ double res_diff(double k, double m, double l) { return k - m * l; }
+__device__ __forceinline__ float2 res_diff(float2 k, float2 m, float2 l)
+{
+    DFAcc a;  // k + m (-lam)
+    a.hi = k.x;
+    a.lo = k.y;
+    a.add(m, l);
+    return a.get2();
+}
+__device__ __forceinline__ float res_head(float v) { return v; }
+__device__ __forceinline__ double res_head(double v) { return v; }
+__device__ __forceinline__ float res_head(float2 v) { return v.x; }
+__device__ __forceinline__ void res_zero(float &v) { v = 0.f; }
+__device__ __forceinline__ void res_zero(double &v) { v = 0.0; }
+__device__ __forceinline__ void res_zero(float2 &v) { v = make_float2(0.f, 0.f); }
+__device__ __forceinline__ float res_max(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double res_max(double a, double b) { return fmax(a, b); }
+
 template <typename T>
 __global__ void __launch_bounds__(kT)
     k_residual(int64_t n, int k, const T *__restrict__ KX, const T *__restrict__ MX, const double *__restrict__ lam,
                T *__restrict__ R, double *part)
 {
-    __shared__ double sred[3 * PW][kT / 32];
+    using H = decltype(res_head(T()));  // float or double
+    __shared__ double sred[2 * PW][kT / 32];
+    __shared__ H smax[PW][kT / 32];
     const int q = blockIdx.y;
-    double rr[PW], mm[PW], mx[PW];
+    double v[2 * PW];  // |R|^2 of the panel's columns, then |MX|^2
+    H mx[PW];
     T lq[PW];
 #pragma unroll
     for (int c = 0; c < PW; ++c) {
-        rr[c] = mm[c] = mx[c] = 0.0;
-        lq[c] = q * PW + c < k ? (T)lam[q * PW + c] : T(0);
+        v[c] = v[PW + c] = 0.0;
+        mx[c] = H(0);
+        lq[c] = res_lam(T(), q * PW + c < k ? lam[q * PW + c] : 0.0);
     }
     for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < n; row += (int64_t)gridDim.x * blockDim.x) {
         const int64_t off = ((int64_t)q * n + row) * PW;
@@ -1084,102 +1328,47 @@ __global__ void __launch_bounds__(kT)
 #pragma unroll
         for (int c = 0; c < PW; ++c) {
             if (q * PW + c >= k) {
-                kv[c] = T(0);
+                res_zero(kv[c]);
                 continue;
             }
-            const T r = kv[c] - mv[c] * lq[c];
-            kv[c] = r;
-            const double rd = (double)r, md = (double)mv[c];
-            rr[c] = fma(rd, rd, rr[c]);
-            mm[c] = fma(md, md, mm[c]);
-            mx[c] = fmax(mx[c], fabs(rd));
+            kv[c] = res_diff(kv[c], mv[c], lq[c]);
+            const H r = res_head(kv[c]);
+            const double rd = (double)r, md = (double)res_head(mv[c]);
+            v[c] = fma(rd, rd, v[c]);
+            v[PW + c] = fma(md, md, v[PW + c]);
+            mx[c] = res_max(mx[c], r < H(0) ? -r : r);
         }
         st_row(R + off, kv);
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // lane l ends up with value l >> 1 over the warp
+#pragma unroll
+    for (int h = PW, o = 16; h > 0; h >>= 1, o >>= 1) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double send = upper ? v[i] : v[i + h];
+            const double stay = upper ? v[i + h] : v[i];
+            v[i] = stay + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    if ((lane & 1) == 0) sred[lane >> 1][wid] = v[0];
 #pragma unroll
     for (int c = 0; c < PW; ++c) {
-        double a = warp_sum(rr[c]), b = warp_sum(mm[c]), m = mx[c];
+        H m = mx[c];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) {
-            sred[3 * c][wid] = a;
-            sred[3 * c + 1][wid] = b;
-            sred[3 * c + 2][wid] = m;
-        }
+        for (int o = 16; o > 0; o >>= 1) m = res_max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) smax[c][wid] = m;
     }
     __syncthreads();
     if (threadIdx.x < 3 * PW) {
         const int c = threadIdx.x / 3, t = threadIdx.x % 3;
         if (q * PW + c < k) {
-            double v = 0.0;
-            for (int w = 0; w < (int)(blockDim.x / 32); ++w) v = t == 2 ? fmax(v, sred[3 * c + t][w]) : v + sred[3 * c + t][w];
-            part[(int64_t)blockIdx.x * 3 * k + 3 * (q * PW + c) + t] = v;
-        }
-    }
-}
-
-// k_residual for double-float panels: R = KX - MX diag(lam) in double-float
-// arithmetic on the FP32 pipe (lam split once per column); the sums of
-// |r|^2 and |m|^2 and max|r| take the leading floats (seven digits are all a
-// residual norm needs) into FP64 accumulators (no FP32 underflow of squares
-// for badly scaled systems), reduced across threads as in k_residual.
-__global__ void __launch_bounds__(kT)
-    k_residual_df(int64_t n, int k, const float2 *__restrict__ KX, const float2 *__restrict__ MX,
-                  const double *__restrict__ lam, float2 *__restrict__ R, double *part)
-{
-    __shared__ double sred[3 * PW][kT / 32];
-    const int q = blockIdx.y;
-    double rr[PW], mm[PW], mx[PW];
-    float2 lq[PW];
-#pragma unroll
-    for (int c = 0; c < PW; ++c) {
-        rr[c] = mm[c] = mx[c] = 0.0;
-        lq[c] = q * PW + c < k ? df_split(-lam[q * PW + c]) : make_float2(0.f, 0.f);
-    }
-    for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < n; row += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t off = ((int64_t)q * n + row) * PW;
-        float2 kv[PW], mv[PW];
-        ld_row(KX + off, kv);
-        ld_row(MX + off, mv);
-#pragma unroll
-        for (int c = 0; c < PW; ++c) {
-            if (q * PW + c >= k) {
-                kv[c] = make_float2(0.f, 0.f);
-                continue;
-            }
-            DFAcc a;  // k + m (-lam)
-            a.hi = kv[c].x;
-            a.lo = kv[c].y;
-            a.add(mv[c], lq[c]);
-            const float2 r = a.get2();
-            kv[c] = r;
-            const double rd = (double)r.x, md = (double)mv[c].x;
-            rr[c] = fma(rd, rd, rr[c]);
-            mm[c] = fma(md, md, mm[c]);
-            mx[c] = fmax(mx[c], fabs(rd));
-        }
-        st_row(R + off, kv);
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int c = 0; c < PW; ++c) {
-        double a = warp_sum(rr[c]), b = warp_sum(mm[c]), m = mx[c];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) {
-            sred[3 * c][wid] = a;
-            sred[3 * c + 1][wid] = b;
-            sred[3 * c + 2][wid] = m;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 3 * PW) {
-        const int c = threadIdx.x / 3, t = threadIdx.x % 3;
-        if (q * PW + c < k) {
-            double v = 0.0;
-            for (int w = 0; w < (int)(blockDim.x / 32); ++w) v = t == 2 ? fmax(v, sred[3 * c + t][w]) : v + sred[3 * c + t][w];
-            part[(int64_t)blockIdx.x * 3 * k + 3 * (q * PW + c) + t] = v;
+            double x = 0.0;
+            for (int w = 0; w < kT / 32; ++w)
+                x = t == 2 ? fmax(x, (double)smax[c][w]) : x + sred[t * PW + c][w];
+            part[(int64_t)blockIdx.x * 3 * k + 3 * (q * PW + c) + t] = x;
         }
     }
 }
@@ -1342,10 +1531,22 @@ struct Ctx {
     DevBuf<float2> df_K, df_M;  // the sliced FP64 matrix values as double-float pairs (mixed second phase)
     const DevMatrix *dfK = nullptr, *dfM = nullptr;
     int launches = 0;
-    DevBuf<double> part, gram, C, lam_d, dinv;
-    std::vector<double> hg, hC, hlam;
+    DevBuf<double> part, gram, C, lam_d, dinv, rsum;
+    std::vector<double> hC, hlam;
+    double *pin = nullptr;     // page-locked: the small matrices and sums on their way
+    cudaEvent_t sums = nullptr;  // the residuals' sums have arrived
+    bool one_pattern = false;  // K and M share their sliced pattern
     int ngrid;
+    ~Ctx()
+    {
+        if (pin) cudaFreeHost(pin);
+        if (sums) cudaEventDestroy(sums);
+    }
 };
+
+// doubles of Ctx::pin: both Gram triangles and the coefficients of three blocks of
+// at most 32 columns
+constexpr size_t kPinDoubles = 96 * 97 + 96 * 32 + 3 * 32;
 
 template <typename T>
 SellView<T> sell_of(const DevMatrix &A)
@@ -1371,9 +1572,41 @@ static void to_df(Ctx &c, const double *a, float2 *b, int64_t len)
     ++c.launches;
 }
 
+// Systems of few (slice, panel) units per SM share a unit among kParts<T> warps.  A
+// matrix alone: whole units win from about 50 per SM on (double-float, whole against
+// shared: 351 and 349 us at 54 per SM, 552 and 593 at 93, 1,078 and 1,383 at 190); the
+// fused pair pays for longer (two products against the pair: 195 and 142 us at 54, 301
+// and 241 at 93, 595 and 782 at 190).
+static bool few_units(const Ctx &c, const DevMatrix &A, int64_t per_sm) { return A.ns * c.np < sms() * per_sm; }
+constexpr int64_t kUnitsAlone = 48, kUnitsPair = 96;
+
+// Y0 = A X (Y1 = B X too when PAIR: values v1 on A's pattern), kParts warps per unit.
+template <typename T, bool PAIR>
+static void spmm_parts(Ctx &c, const DevMatrix &A, const T *v0, const T *v1, const T *X, T *Y0, T *Y1)
+{
+    constexpr int kGroups = kT / 32 / kParts<T>;
+    const size_t smem = (size_t)kGroups * (kParts<T> - 1) * (PAIR ? 2 : 1) * A.bs * PW * 32 * sizeof(T);
+    const int64_t ctas = (A.ns * c.np + kGroups - 1) / kGroups;
+    const int g = (int)std::min<int64_t>(ctas, (int64_t)sms() * 64);
+    if (A.bs == 3) {
+        PFG_CUDA(cudaFuncSetAttribute(k_spmm_parts<3, T, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_spmm_parts<3, T, PAIR><<<g, kT, smem, c.st>>>(A.nb, A.ns, A.sptr.p, A.scol.p, v0, v1, c.np, c.k, X, Y0,
+                                                        Y1, c.fixed);
+    } else {
+        k_spmm_parts<1, T, PAIR><<<g, kT, smem, c.st>>>(A.nb, A.ns, A.sptr.p, A.scol.p, v0, v1, c.np, c.k, X, Y0,
+                                                        Y1, c.fixed);
+    }
+    PFG_CUDA(cudaGetLastError());
+    ++c.launches;
+}
+
 // Y = A X, panels in double-float, A's values as double-float pairs.
 static void spmm_df(Ctx &c, const DevMatrix &A, const float2 *X, float2 *Y)
 {
+    if (few_units(c, A, kUnitsAlone)) {
+        spmm_parts<float2, false>(c, A, df_values(c, A), nullptr, X, Y, nullptr);
+        return;
+    }
     const SellView<double> v = A.sell<double>();
     int per = 0;
     if (A.bs == 3)
@@ -1396,6 +1629,12 @@ void spmm(Ctx &c, const DevMatrix &A, const T *X, T *Y)
     if constexpr (std::is_same<T, float2>::value) {
         spmm_df(c, A, X, Y);
     } else {
+        if constexpr (std::is_same<T, float>::value) {
+            if (few_units(c, A, kUnitsAlone)) {
+                spmm_parts<float, false>(c, A, A.s32.p, nullptr, X, Y, nullptr);
+                return;
+            }
+        }
         const SellView<T> v = sell_of<T>(A);
         int per = 0;
         if (A.bs == 3)
@@ -1418,6 +1657,12 @@ void spmm(Ctx &c, const DevMatrix &A, const T *X, T *Y)
 template <typename T>
 void spmm_pair(Ctx &c, const DevMatrix &K, const DevMatrix &M, const T *X, T *KX, T *MX)
 {
+    if constexpr (std::is_same<T, float>::value) {
+        if (c.one_pattern && few_units(c, K, kUnitsPair)) {
+            spmm_parts<float, true>(c, K, K.s32.p, M.s32.p, X, KX, MX);
+            return;
+        }
+    }
     spmm<T>(c, K, X, KX);
     spmm<T>(c, M, X, MX);
 }
@@ -1429,45 +1674,51 @@ void gram(Ctx &c, int nblk, const Blocks<T> &B, std::vector<double> &GA, std::ve
     const int npairs = m * (m + 1) / 2;
     const int mp = nblk * c.kp;
     const int tiles = mp / PW;
-    const int threads = (kGramSub * tiles * (tiles + 1) / 2 + 31) / 32 * 32;
+    const int groups = nblk * ((c.k + kGramSub - 1) / kGramSub);
+    const int threads = (groups * (groups + 1) / 2 + 31) / 32 * 32;
     // staged tiles: 3 matrices x tiles; a double-float value is 8 bytes like a double
     const size_t smem = (size_t)3 * tiles * (kGramRows * PW + 64 / sizeof(T)) * sizeof(T);
-    const int g = c.ngrid;
-    c.part.ensure((size_t)g * 2 * npairs);
-    c.gram.ensure((size_t)2 * npairs);
     // float2: double-float panels (mixed second phase); float: FP32; double: IEEE FP64
     constexpr bool kDF = std::is_same<T, float2>::value;
     auto kern = k_gram<T, kDF>;
     PFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // about 20 warps per SM: two CTAs of ten at k = 24, seven of three at k = 12 (two of
+    // three left the pipes to latency: 58 us at 95k rows, now 29), a staged step each
+    int occ = 0;
+    PFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
+    const int per_sm = std::max(1, std::min(std::max(2, 20 * 32 / threads), occ));
+    const int g = (int)std::max<int64_t>(1, std::min<int64_t>((c.n + kGramRows - 1) / kGramRows, (int64_t)sms() * per_sm));
+    c.part.ensure((size_t)g * 2 * npairs);
+    c.gram.ensure((size_t)2 * npairs);
     kern<<<g, threads, smem, c.st>>>(c.n, c.k, nblk, B.X.p, B.W.p, B.P.p, B.KX.p, B.KW.p, B.KP.p, B.MX.p, B.MW.p,
                                      B.MP.p, c.part.p);
-    k_reduce_parts<<<grid_for(2 * npairs, 256, 64), 256, 0, c.st>>>(c.part.p, g, 2 * npairs, c.gram.p);
+    k_reduce_parts<<<(2 * npairs + 31) / 32, 1024, 0, c.st>>>(c.part.p, g, 2 * npairs, c.gram.p);
     PFG_CUDA(cudaGetLastError());
     c.launches += 2;
-    c.hg.resize((size_t)2 * npairs);
-    PFG_CUDA(cudaMemcpyAsync(c.hg.data(), c.gram.p, 2 * npairs * sizeof(double), cudaMemcpyDeviceToHost, c.st));
+    PFG_CUDA(cudaMemcpyAsync(c.pin, c.gram.p, 2 * npairs * sizeof(double), cudaMemcpyDeviceToHost, c.st));
     PFG_CUDA(cudaStreamSynchronize(c.st));
     GA.assign((size_t)m * m, 0.0);
     GB.assign((size_t)m * m, 0.0);
     int p = 0;
     for (int i = 0; i < m; ++i)
         for (int j = i; j < m; ++j, ++p) {
-            GA[(size_t)j * m + i] = GA[(size_t)i * m + j] = c.hg[p];
-            GB[(size_t)j * m + i] = GB[(size_t)i * m + j] = c.hg[npairs + p];
+            GA[(size_t)j * m + i] = GA[(size_t)i * m + j] = c.pin[p];
+            GB[(size_t)j * m + i] = GB[(size_t)i * m + j] = c.pin[npairs + p];
         }
 }
 
 template <typename T>
-void lincomb(Ctx &c, int nblk, const T *X, const T *W, const T *P, T *Xn, T *Pn)
+void lincomb(Ctx &c, int nblk, const CombSet<T> &set)
 {
     const int m = nblk * c.k;
     const size_t smem = (size_t)m * c.kp * sizeof(T);  // (a double-float coefficient is 8 bytes too)
+    const dim3 g((unsigned)grid_for(c.n, kT, sms() * 8), 3);
     if constexpr (std::is_same<T, float2>::value) {
         PFG_CUDA(cudaFuncSetAttribute(k_lincomb_df, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_lincomb_df<<<grid_for(c.n, kT, sms() * 8), kT, smem, c.st>>>(c.n, c.k, nblk, X, W, P, c.C.p, Xn, Pn);
+        k_lincomb_df<<<g, kT, smem, c.st>>>(c.n, c.k, nblk, set, c.C.p);
     } else {
         PFG_CUDA(cudaFuncSetAttribute(k_lincomb<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_lincomb<T><<<grid_for(c.n, kT, sms() * 8), kT, smem, c.st>>>(c.n, c.k, nblk, X, W, P, c.C.p, Xn, Pn);
+        k_lincomb<T><<<g, kT, smem, c.st>>>(c.n, c.k, nblk, set, c.C.p);
     }
     PFG_CUDA(cudaGetLastError());
     ++c.launches;
@@ -1486,17 +1737,24 @@ int rayleigh_ritz(Ctx &c, int nblk, const Blocks<T> &B, double rank_tol)
     if (got < c.k) return got;
     c.C.ensure((size_t)m * c.k);
     c.lam_d.ensure((size_t)c.k);
-    PFG_CUDA(cudaMemcpyAsync(c.C.p, c.hC.data(), (size_t)m * c.k * sizeof(double), cudaMemcpyHostToDevice, c.st));
-    PFG_CUDA(cudaMemcpyAsync(c.lam_d.p, c.hlam.data(), c.k * sizeof(double), cudaMemcpyHostToDevice, c.st));
+    // (the copies have left these buffers before the next synchronisation that precedes their reuse)
+    double *pc = c.pin + 96 * 97, *pl = pc + 96 * 32;
+    std::copy(c.hC.begin(), c.hC.end(), pc);
+    std::copy(c.hlam.begin(), c.hlam.end(), pl);
+    PFG_CUDA(cudaMemcpyAsync(c.C.p, pc, (size_t)m * c.k * sizeof(double), cudaMemcpyHostToDevice, c.st));
+    PFG_CUDA(cudaMemcpyAsync(c.lam_d.p, pl, c.k * sizeof(double), cudaMemcpyHostToDevice, c.st));
     return got;
 }
 
 template <typename T>
 void apply_rr(Ctx &c, int nblk, Blocks<T> &B)
 {
-    lincomb<T>(c, nblk, B.X.p, B.W.p, B.P.p, B.Xn.p, B.Pn.p);
-    lincomb<T>(c, nblk, B.KX.p, B.KW.p, B.KP.p, B.KXn.p, B.KPn.p);
-    lincomb<T>(c, nblk, B.MX.p, B.MW.p, B.MP.p, B.MXn.p, B.MPn.p);
+    lincomb<T>(c, nblk,
+               CombSet<T>{{B.X.p, B.KX.p, B.MX.p},
+                          {B.W.p, B.KW.p, B.MW.p},
+                          {B.P.p, B.KP.p, B.MP.p},
+                          {B.Xn.p, B.KXn.p, B.MXn.p},
+                          {B.Pn.p, B.KPn.p, B.MPn.p}});
     std::swap(B.X, B.Xn);
     std::swap(B.P, B.Pn);
     std::swap(B.KX, B.KXn);
@@ -1509,30 +1767,31 @@ struct ResInfo {
     std::vector<double> rel, maxabs;
 };
 
+// R and the residuals' sums, on their way to the host
 template <typename T>
-ResInfo residuals(Ctx &c, Blocks<T> &B)
+void residuals(Ctx &c, Blocks<T> &B)
 {
-    const int g = std::min(c.ngrid, 1024);
+    const int g = (int)std::min<int64_t>((c.n + kT - 1) / kT, c.ngrid);
     c.part.ensure((size_t)g * 3 * c.k);
-    if constexpr (std::is_same<T, float2>::value)
-        k_residual_df<<<dim3(g, c.np), kT, 0, c.st>>>(c.n, c.k, B.KX.p, B.MX.p, c.lam_d.p, B.R.p, c.part.p);
-    else
-        k_residual<T><<<dim3(g, c.np), kT, 0, c.st>>>(c.n, c.k, B.KX.p, B.MX.p, c.lam_d.p, B.R.p, c.part.p);
+    c.rsum.ensure((size_t)3 * c.k);
+    k_residual<T><<<dim3(g, c.np), kT, 0, c.st>>>(c.n, c.k, B.KX.p, B.MX.p, c.lam_d.p, B.R.p, c.part.p);
+    k_reduce_residual<<<(3 * c.k + 7) / 8, 256, 0, c.st>>>(c.part.p, g, 3 * c.k, c.rsum.p);
     PFG_CUDA(cudaGetLastError());
-    ++c.launches;
-    std::vector<double> h((size_t)g * 3 * c.k);
-    PFG_CUDA(cudaMemcpyAsync(h.data(), c.part.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c.st));
-    PFG_CUDA(cudaStreamSynchronize(c.st));
+    c.launches += 2;
+    double *h = c.pin + 96 * 97 + 96 * 32;
+    PFG_CUDA(cudaMemcpyAsync(h, c.rsum.p, (size_t)3 * c.k * sizeof(double), cudaMemcpyDeviceToHost, c.st));
+    PFG_CUDA(cudaEventRecord(c.sums, c.st));
+}
+
+static ResInfo read_residuals(Ctx &c)
+{
+    PFG_CUDA(cudaEventSynchronize(c.sums));
+    const double *h = c.pin + 96 * 97 + 96 * 32;
     ResInfo ri;
     ri.rel.assign(c.k, 0.0);
     ri.maxabs.assign(c.k, 0.0);
     for (int j = 0; j < c.k; ++j) {
-        double rr = 0, mm = 0, mx = 0;
-        for (int b = 0; b < g; ++b) {
-            rr += h[(size_t)b * 3 * c.k + 3 * j];
-            mm += h[(size_t)b * 3 * c.k + 3 * j + 1];
-            mx = std::max(mx, h[(size_t)b * 3 * c.k + 3 * j + 2]);
-        }
+        const double rr = h[3 * j], mm = h[3 * j + 1], mx = h[3 * j + 2];
         const double den = std::fabs(c.hlam[j]) * std::sqrt(mm);
         ri.rel[j] = den > 0 ? std::sqrt(rr) / den : std::sqrt(rr);
         ri.maxabs[j] = mx;
@@ -1542,6 +1801,26 @@ ResInfo residuals(Ctx &c, Blocks<T> &B)
 
 constexpr int kRefreshImages = 10;
 constexpr int kFp32Stall = 50;
+
+// W = T R
+template <typename T>
+void precondition(Ctx &c, const EigConfig &cfg, Blocks<T> &B)
+{
+    const int gp = grid_for(c.nb, kT, sms() * 8);
+    if constexpr (std::is_same<T, float2>::value) {
+        if (c.bs == 3)
+            k_eig_precond_df<3><<<gp, kT, 0, c.st>>>(c.nb, c.k, c.dinv.p, cfg.precond, B.R.p, B.W.p, c.fixed);
+        else
+            k_eig_precond_df<1><<<gp, kT, 0, c.st>>>(c.nb, c.k, c.dinv.p, cfg.precond, B.R.p, B.W.p, c.fixed);
+    } else {
+        if (c.bs == 3)
+            k_eig_precond<3, T><<<gp, kT, 0, c.st>>>(c.nb, c.k, c.dinv.p, cfg.precond, B.R.p, B.W.p, c.fixed);
+        else
+            k_eig_precond<1, T><<<gp, kT, 0, c.st>>>(c.nb, c.k, c.dinv.p, cfg.precond, B.R.p, B.W.p, c.fixed);
+    }
+    PFG_CUDA(cudaGetLastError());
+    ++c.launches;
+}
 
 // One precision phase.  start: 0 random, 1 X already holds a start block.
 template <typename T>
@@ -1558,8 +1837,7 @@ int phase(Ctx &c, DevMatrix &K, DevMatrix &M, Blocks<T> &B, const EigConfig &cfg
         }
     }
     const double rank_tol = fp32_phase ? 1e-9 : 1e-13;
-    spmm<T>(c, K, B.X.p, B.KX.p);
-    spmm<T>(c, M, B.X.p, B.MX.p);
+    spmm_pair<T>(c, K, M, B.X.p, B.KX.p, B.MX.p);
     // Rayleigh-Ritz on X alone (X of LOBPCG_CRS, SparseClass.f90:2063-2067)
     if (rayleigh_ritz<T>(c, 1, B, rank_tol) < c.k) throw Error(PFG_E_BREAKDOWN, "LOBPCG: start block is rank deficient");
     apply_rr<T>(c, 1, B);
@@ -1567,7 +1845,14 @@ int phase(Ctx &c, DevMatrix &K, DevMatrix &M, Blocks<T> &B, const EigConfig &cfg
     double best = 1e300, best_lsum = 1e300;
     int since_best = 0, since_refresh = 0;
     for (;;) {
-        ResInfo ri = residuals<T>(c, B);
+        // W = T R and its images go to the stream before the residuals are read: the host's
+        // tests cost no gap on the device (after the last iteration W is left over)
+        residuals<T>(c, B);
+        if (iters_left > 0) {
+            precondition<T>(c, cfg, B);
+            spmm_pair<T>(c, K, M, B.W.p, B.KW.p, B.MW.p);
+        }
+        const ResInfo ri = read_residuals(c);
         max_rel = 0.0;
         double maxabs = 0.0;
         for (int j = 0; j < cfg.nev; ++j) {
@@ -1606,22 +1891,6 @@ int phase(Ctx &c, DevMatrix &K, DevMatrix &M, Blocks<T> &B, const EigConfig &cfg
         if (iters_left <= 0) return -1;
         --iters_left;
         ++iters_done;
-        // W = T R, its images
-        const int gp = grid_for(c.nb, kT, sms() * 8);
-        if constexpr (std::is_same<T, float2>::value) {
-            if (c.bs == 3)
-                k_eig_precond_df<3><<<gp, kT, 0, c.st>>>(c.nb, c.k, c.dinv.p, cfg.precond, B.R.p, B.W.p, c.fixed);
-            else
-                k_eig_precond_df<1><<<gp, kT, 0, c.st>>>(c.nb, c.k, c.dinv.p, cfg.precond, B.R.p, B.W.p, c.fixed);
-        } else {
-            if (c.bs == 3)
-                k_eig_precond<3, T><<<gp, kT, 0, c.st>>>(c.nb, c.k, c.dinv.p, cfg.precond, B.R.p, B.W.p, c.fixed);
-            else
-                k_eig_precond<1, T><<<gp, kT, 0, c.st>>>(c.nb, c.k, c.dinv.p, cfg.precond, B.R.p, B.W.p, c.fixed);
-        }
-        PFG_CUDA(cudaGetLastError());
-        ++c.launches;
-        spmm_pair<T>(c, K, M, B.W.p, B.KW.p, B.MW.p);
         int nblk = haveP ? 3 : 2;
         int got = rayleigh_ritz<T>(c, nblk, B, rank_tol);
         if (got < c.k && nblk == 3) {
@@ -1667,6 +1936,8 @@ EigResult lobpcg_solve(DevMatrix &K, DevMatrix &M, const uint8_t *fixed, const E
     c.fixed = fixed;
     c.ngrid = sms() * 2;
     PFG_CHECK(c.n >= 3 * c.k, PFG_E_ARG, "eig: block size too large for the system");
+    PFG_CUDA(cudaMallocHost((void **)&c.pin, kPinDoubles * sizeof(double)));
+    PFG_CUDA(cudaEventCreateWithFlags(&c.sums, cudaEventDisableTiming));
     EigResult res;
     cudaEvent_t e0, e1;
     PFG_CUDA(cudaEventCreate(&e0));
@@ -1680,6 +1951,17 @@ EigResult lobpcg_solve(DevMatrix &K, DevMatrix &M, const uint8_t *fixed, const E
     double max_rel = 0.0, ref_r1 = -1.0;
     build_sell(K, true, cfg.precision == PFG_PREC_MIXED, st);
     build_sell(M, true, cfg.precision == PFG_PREC_MIXED, st);
+    if (cfg.precision == PFG_PREC_MIXED && K.ns == M.ns && K.scol.n == M.scol.n) {
+        DevBuf<int> same(1);
+        int one = 1;
+        PFG_CUDA(cudaMemcpyAsync(same.p, &one, sizeof(int), cudaMemcpyHostToDevice, st));
+        k_compare<<<grid_for(K.ns + 1, 256), 256, 0, st>>>(K.ns + 1, K.sptr.p, M.sptr.p, same.p);
+        k_compare<<<grid_for((int64_t)K.scol.n, 256), 256, 0, st>>>((int64_t)K.scol.n, K.scol.p, M.scol.p, same.p);
+        PFG_CUDA(cudaGetLastError());
+        PFG_CUDA(cudaMemcpyAsync(&one, same.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+        PFG_CUDA(cudaStreamSynchronize(st));
+        c.one_pattern = one != 0;
+    }
     Blocks<double> B64;
     Blocks<float2> Bdf;
     if (cfg.precision == PFG_PREC_MIXED) {

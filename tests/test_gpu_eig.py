@@ -167,3 +167,46 @@ def test_eig_dense_refuses_large_problems(cuda):
     with pytest.raises(N.NativeError) as e:
         s.eig(5)
     assert e.value.code == -9 and "use_LOBPCG" in str(e.value)
+
+
+def _ring(n, seed):
+    """Symmetric, diagonally dominant, a ragged band; the lowest pairs well apart."""
+    rng = np.random.default_rng(seed)
+    i = np.arange(n)
+    d = 4.0 + np.where(i < 40, 0.25 * i, 10.0 + 0.5 * rng.random(n))
+    far = np.where(rng.random(n - 7) < 0.5, 0.3, 0.0)
+    return sp.diags([far, np.full(n - 1, -0.4), d, np.full(n - 1, -0.4), far], [-7, -1, 0, 1, 7], format="csr")
+
+
+# Block sizes of one half panel (3), of whole and half panels (12, 28); row counts on
+# both sides of the limits between shared and whole slices (n / 32 slices times the
+# panels against 48 and 96 per SM); K and M of one pattern and of two.
+@pytest.mark.parametrize("n,block,one_pattern,precision", [
+    (97, 3, True, "mixed"), (1000, 12, False, "mixed"), (3001, 28, True, "mixed"), (60000, 28, True, "mixed"),
+    (60000, 28, False, "mixed"), (130001, 28, True, "mixed"), (1000, 12, True, "fp64")])
+def test_eig_products_of_every_form(cuda, n, block, one_pattern, precision):
+    import scipy.sparse.linalg as sl
+
+    nev = block - 2 if block < 12 else 6
+    K = _ring(n, n)
+    if one_pattern:
+        M = K.copy()
+        M.data = np.where(M.data > 1.0, 2.0, 0.05 * M.data)
+    else:
+        M = sp.diags([np.full(n - 1, 0.02), np.full(n, 2.0), np.full(n - 1, 0.02)], [-1, 0, 1], format="csr")
+    s = FEMSolver()
+    for A, name in ((K, "A"), (M, "B")):
+        s.setCRS(CRS=((A.indptr + 1).astype(np.int64), (A.indices + 1).astype(np.int32), A.data))
+        s.keepThisMatrixAs(name)
+    s.use_LOBPCG = True
+    s.LOBPCG_TOL = 1e-9
+    lam, X = s.eig(nev, block_size=block, preconditioning="Jacobi", precision=precision)
+    assert s.last_info["status"] == 0, s.last_info
+    # the solver's own residual is at most 1e-9; FP64 and double-float products of at
+    # most five terms add less than that
+    R = K @ X - (M @ X) * lam[None, :]
+    rel = np.linalg.norm(R, axis=0) / (np.abs(lam) * np.linalg.norm(M @ X, axis=0))
+    assert rel.max() <= 2e-9, rel
+    assert np.abs(X.T @ (M @ X) - np.eye(nev)).max() <= 1e-8
+    w = np.sort(sl.eigsh(K.tocsc(), nev, M.tocsc(), sigma=0.0, return_eigenvectors=False))
+    assert np.abs(lam - w).max() / w.max() <= 1e-9
