@@ -550,15 +550,6 @@ __device__ __forceinline__ void lds_row(const double *p, double (&v)[PW])
         v[2 * u + 1] = w.y;
     }
 }
-__device__ __forceinline__ void lds_row(const float2 *p, float2 (&v)[PW])
-{
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const float4 w = reinterpret_cast<const float4 *>(p)[u];
-        v[2 * u] = make_float2(w.x, w.y);
-        v[2 * u + 1] = make_float2(w.z, w.w);
-    }
-}
 
 // Double-FP32 ("double-float") arithmetic on the FP32 pipe, for the second
 // phase of the mixed LOBPCG (its Gram, SpMM and linear combinations of FP64
@@ -594,6 +585,110 @@ struct DFAcc {
         const float z = __fsub_rn(s, hi);
         return make_float2(s, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, z)), __fsub_rn(lo, z)));
     }
+};
+
+// Two FP32 values in one 64-bit register pair: add, mul and fma.rn.f32x2 work on
+// both.  The pipe does no more of them per clock than of the scalar forms (measured
+// 128 values per clock and SM either way), but in half the issue slots and fewer
+// registers: linear combinations 996 -> 852 us at 398k rows and 24 columns, 78 -> 56
+// at 95k and 12 (where the half panel counts too), the Gram matrices 104 -> 94 there
+// and 1,195 -> 1,177 at the larger size (pipe-bound at 12 operations a multiply-add).
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2_pack(float a, float b)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 f2_get(F2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Two DFAcc side by side, the same operations in the same order (a subtraction as an
+// FMA by -1, which rounds once just so): the same bits.  a is common to both.
+struct DFLeft {  // a double-float factor and its negated head, each twice
+    F2 h, nh, l;
+    __device__ explicit DFLeft(float2 a) : h(f2_pack(a.x, a.x)), nh(f2_pack(-a.x, -a.x)), l(f2_pack(a.y, a.y)) {}
+};
+struct DFAcc2 {
+    F2 hi, lo;
+    __device__ void zero() { hi = lo = 0ull; }
+    __device__ void add(const DFLeft &a, F2 bh, F2 bl)
+    {
+        const F2 m1 = 0xbf800000bf800000ull;  // (-1, -1)
+        const F2 np = f2_mul(a.nh, bh);       // -p
+        F2 e = f2_fma(a.h, bh, np);
+        e = f2_fma(a.h, bl, e);
+        e = f2_fma(a.l, bh, e);
+        const F2 t = f2_fma(np, m1, hi);
+        const F2 z = f2_fma(hi, m1, t);
+        const F2 u = f2_fma(f2_fma(z, m1, t), m1, hi);  // hi - (t - z)
+        const F2 err = f2_fma(f2_add(np, z), m1, u);    // + (p - z)
+        hi = t;
+        lo = f2_add(lo, f2_add(err, e));
+    }
+    __device__ DFAcc get(int c) const
+    {
+        const float2 h = f2_get(hi), l = f2_get(lo);
+        DFAcc r;
+        r.hi = c ? h.y : h.x;
+        r.lo = c ? l.y : l.x;
+        return r;
+    }
+};
+
+// Eight double-float values, heads and tails in pairs of columns, and the sums of
+// a x row over them.  (The sliced products keep DFAcc: their rows come one by one
+// from L2, and packed they took 571 us where DFAcc takes 465.)
+struct DFRow {
+    F2 h[PW / 2], l[PW / 2];
+    template <int NC>
+    __device__ void load_paired(const float2 *p)  // shared memory: two heads, two tails
+    {
+#pragma unroll
+        for (int u = 0; u < NC / 2; ++u) {
+            const ulonglong2 w = reinterpret_cast<const ulonglong2 *>(p)[u];
+            h[u] = w.x;
+            l[u] = w.y;
+        }
+    }
+};
+struct DFRowAcc {
+    DFAcc2 v[PW / 2];
+    __device__ void zero()
+    {
+#pragma unroll
+        for (int u = 0; u < PW / 2; ++u) v[u].zero();
+    }
+    template <int NC>
+    __device__ void add(float2 a, const DFRow &x)
+    {
+        const DFLeft f(a);
+#pragma unroll
+        for (int u = 0; u < NC / 2; ++u) v[u].add(f, x.h[u], x.l[u]);
+    }
+    __device__ float2 get(int c) const { return v[c >> 1].get(c & 1).get2(); }
 };
 
 __device__ __forceinline__ float2 df_split(double x)
@@ -909,7 +1004,8 @@ __global__ void k_compare(int64_t n, const I *__restrict__ a, const I *__restric
 
 // k_lincomb with the blocks, the coefficients and the results in double-float.
 __global__ void __launch_bounds__(kT)
-    k_lincomb_df(int64_t n, int k, int nblk, const CombSet<float2> set, const double *__restrict__ C)
+    k_lincomb_df(int64_t n, int k, int nblk,
+                 const __grid_constant__ CombSet<float2> set, const double *__restrict__ C)
 {
     const float2 *__restrict__ X = set.X[blockIdx.y];
     const float2 *__restrict__ W = set.W[blockIdx.y];
@@ -923,90 +1019,51 @@ __global__ void __launch_bounds__(kT)
     const int kp = np * PW;
     for (int e = threadIdx.x; e < m * kp; e += blockDim.x) {
         const int r = e / kp, j = e - r * kp;
-        sC[e] = j < k ? df_split(C[(int64_t)j * m + r]) : make_float2(0.f, 0.f);
+        const float2 v = j < k ? df_split(C[(int64_t)j * m + r]) : make_float2(0.f, 0.f);
+        float *at = reinterpret_cast<float *>(sC + (e & ~1)) + (e & 1);  // two heads, two tails
+        at[0] = v.x;
+        at[2] = v.y;
     }
     __syncthreads();
     for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < n; row += (int64_t)gridDim.x * blockDim.x) {
         for (int qo = 0; qo < np; ++qo) {
-            DFAcc ax[PW], ap[PW];
-#pragma unroll
-            for (int c = 0; c < PW; ++c) {
-                ax[c].zero();
-                ap[c].zero();
-            }
-            for (int b = 0; b < nblk; ++b) {
+            DFRowAcc ax, ap;
+            ax.zero();
+            ap.zero();
+            const bool half = k - qo * PW <= PW / 2;  // (the padding stays zero)
+            auto block = [&](const float2 *S, int b, DFRowAcc &acc) {
                 for (int qi = 0; qi < np; ++qi) {
                     float2 v[PW];
-                    ld_row(panel_row(b == 0 ? X : (b == 1 ? W : P), n, qi, row), v);
+                    ld_row(panel_row(S, n, qi, row), v);
 #pragma unroll
                     for (int c = 0; c < PW; ++c) {
                         const int i = qi * PW + c;
                         if (i >= k) break;
-                        float2 cr[PW];
-                        lds_row(sC + (int64_t)(b * k + i) * kp + qo * PW, cr);
-#pragma unroll
-                        for (int o = 0; o < PW; ++o) {
-                            if (b == 0)
-                                ax[o].add(v[c], cr[o]);
-                            else
-                                ap[o].add(v[c], cr[o]);
+                        const float2 *at = sC + (b * k + i) * kp + qo * PW;
+                        DFRow cr;
+                        if (half) {
+                            cr.load_paired<PW / 2>(at);
+                            acc.add<PW / 2>(v[c], cr);
+                        } else {
+                            cr.load_paired<PW>(at);
+                            acc.add<PW>(v[c], cr);
                         }
                     }
                 }
-            }
+            };
+            block(X, 0, ax);
+            for (int b = 1; b < nblk; ++b) block(b == 1 ? W : P, b, ap);
             float2 pv[PW], xv[PW];
 #pragma unroll
             for (int o = 0; o < PW; ++o) {
-                pv[o] = ap[o].get2();
-                xv[o] = df_add(ax[o].get2(), pv[o]);
+                pv[o] = ap.get(o);
+                xv[o] = df_add(ax.get(o), pv[o]);
             }
             st_row(Pn + ((int64_t)qo * n + row) * PW, pv);
             st_row(Xn + ((int64_t)qo * n + row) * PW, xv);
         }
     }
 }
-
-struct F64Acc {
-    double v;
-    __device__ void zero() { v = 0.0; }
-    __device__ void add(double a, double b) { v = fma(a, b, v); }
-    __device__ double get() const { return v; }
-};
-// FP32 panels (the mixed first phase): plain FP32 multiply-adds per thread
-// over its CTA's rows (about n / 300 terms), partial sums added in FP64.
-struct F32Acc {
-    float v;
-    __device__ void zero() { v = 0.f; }
-    __device__ void add(float a, float b) { v = fmaf(a, b, v); }
-    __device__ double get() const { return (double)v; }
-};
-
-// Staged operand type and accumulator of the Gram kernel per storage type:
-// FP32 panels (FP32 sums), FP64 panels (FP64 sums), double-float panels
-// (double-float sums; DF = true).
-template <typename T, bool DF>
-struct GramArith;
-template <>
-struct GramArith<float, false> {
-    using Stage = float;
-    using Acc = F32Acc;
-    __device__ static float stage(float x) { return x; }
-    __device__ static float none() { return 0.f; }
-};
-template <>
-struct GramArith<double, false> {
-    using Stage = double;
-    using Acc = F64Acc;
-    __device__ static double stage(double x) { return x; }
-    __device__ static double none() { return 0.0; }
-};
-template <>
-struct GramArith<float2, true> {  // panels already in double-float (mixed second phase)
-    using Stage = float2;
-    using Acc = DFAcc;
-    __device__ static float2 stage(float2 x) { return x; }
-    __device__ static float2 none() { return make_float2(0.f, 0.f); }
-};
 
 constexpr int kGramRows = 32;  // rows staged in shared memory per step
 constexpr int kGramSub = 4;    // each thread owns a 4 x 4 sub-tile of both Gram matrices
@@ -1031,35 +1088,94 @@ __device__ __forceinline__ void gram_stage16(const double *src, double *dst)
 {
     *reinterpret_cast<double2 *>(dst) = __ldg(reinterpret_cast<const double2 *>(src));
 }
-__device__ __forceinline__ void gram_stage16(const float2 *src, float2 *dst)
+__device__ __forceinline__ void gram_stage16(const float2 *src, float2 *dst)  // two heads, two tails
 {
-    *reinterpret_cast<float4 *>(dst) = __ldg(reinterpret_cast<const float4 *>(src));
+    const float4 w = __ldg(reinterpret_cast<const float4 *>(src));
+    *reinterpret_cast<float4 *>(dst) = make_float4(w.x, w.z, w.y, w.w);
 }
-// four consecutive staged values (16- or 32-byte aligned)
-__device__ __forceinline__ void gram_lds4(const float *p, float (&v)[kGramSub])
-{
-    const float4 w = *reinterpret_cast<const float4 *>(p);
-    v[0] = w.x;
-    v[1] = w.y;
-    v[2] = w.z;
-    v[3] = w.w;
-}
-__device__ __forceinline__ void gram_lds4(const double *p, double (&v)[kGramSub])
-{
-    const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
-    v[0] = a.x;
-    v[1] = a.y;
-    v[2] = b.x;
-    v[3] = b.y;
-}
-__device__ __forceinline__ void gram_lds4(const float2 *p, float2 (&v)[kGramSub])
-{
-    const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
-    v[0] = make_float2(a.x, a.y);
-    v[1] = make_float2(a.z, a.w);
-    v[2] = make_float2(b.x, b.y);
-    v[3] = make_float2(b.z, b.w);
-}
+
+// A thread's 4 x 4 sums of one Gram matrix by panel type, s y^T added per row (four
+// staged values each, 16-byte shared loads): FP32 panels in FP32 over the CTA's rows
+// (the CTAs' sums are added in FP64), FP64 panels in FP64, double-float panels (the
+// mixed mode's second phase) in double-float.
+template <typename T>
+struct GramTile {
+    struct Four {
+        T v[kGramSub];
+        __device__ explicit Four(const float *p)
+        {
+            const float4 w = *reinterpret_cast<const float4 *>(p);
+            v[0] = w.x;
+            v[1] = w.y;
+            v[2] = w.z;
+            v[3] = w.w;
+        }
+        __device__ explicit Four(const double *p)
+        {
+            const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
+            v[0] = a.x;
+            v[1] = a.y;
+            v[2] = b.x;
+            v[3] = b.y;
+        }
+    };
+    using Left = Four;
+    using Right = Four;
+    T a[kGramSub][kGramSub];
+    __device__ void zero()
+    {
+#pragma unroll
+        for (int i = 0; i < kGramSub; ++i)
+#pragma unroll
+            for (int j = 0; j < kGramSub; ++j) a[i][j] = T(0);
+    }
+    __device__ void add(int i, const Left &s, const Right &y)
+    {
+#pragma unroll
+        for (int j = 0; j < kGramSub; ++j) a[i][j] = fma(s.v[i], y.v[j], a[i][j]);
+    }
+    __device__ double get(int i, int j) const { return (double)a[i][j]; }
+};
+template <>
+struct GramTile<float2> {
+    struct Left {
+        float4 p[2];  // two heads, two tails
+        __device__ explicit Left(const float2 *q)
+        {
+            p[0] = reinterpret_cast<const float4 *>(q)[0];
+            p[1] = reinterpret_cast<const float4 *>(q)[1];
+        }
+        __device__ float2 at(int i) const
+        {
+            const float4 w = p[i >> 1];
+            return (i & 1) ? make_float2(w.y, w.w) : make_float2(w.x, w.z);
+        }
+    };
+    struct Right {
+        ulonglong2 p[2];
+        __device__ explicit Right(const float2 *q)
+        {
+            p[0] = reinterpret_cast<const ulonglong2 *>(q)[0];
+            p[1] = reinterpret_cast<const ulonglong2 *>(q)[1];
+        }
+    };
+    DFAcc2 a[kGramSub][2];
+    __device__ void zero()
+    {
+#pragma unroll
+        for (int i = 0; i < kGramSub; ++i) {
+            a[i][0].zero();
+            a[i][1].zero();
+        }
+    }
+    __device__ void add(int i, const Left &s, const Right &y)
+    {
+        const DFLeft f(s.at(i));
+        a[i][0].add(f, y.p[0].x, y.p[0].y);
+        a[i][1].add(f, y.p[1].x, y.p[1].y);
+    }
+    __device__ double get(int i, int j) const { return a[i][j >> 1].get(j & 1).get(); }
+};
 
 // Upper triangles of S^T (K S) and S^T (M S), S = [X W P] (nblk blocks of k
 // columns, each padded to kp = 8 np columns): each CTA reduces a contiguous
@@ -1079,7 +1195,7 @@ __device__ __forceinline__ void gram_lds4(const float2 *p, float2 (&v)[kGramSub]
 // or double-float (DF: double-float panels of the mixed mode's second phase)
 // on the FP32 pipe.  Padding columns are staged as they are
 // stored and their sums are not written.
-template <typename T, bool DF>
+template <typename T>
 __global__ void __launch_bounds__(320)
     k_gram(int64_t n, int k, int nblk, const T *S0, const T *S1, const T *S2, const T *K0, const T *K1, const T *K2,
            const T *M0, const T *M1, const T *M2, double *part)
@@ -1093,10 +1209,8 @@ __global__ void __launch_bounds__(320)
     const int tiles = mp / PW;
     const int per_block = (k + kGramSub - 1) / kGramSub, groups = nblk * per_block;
     const int ntasks = groups * (groups + 1) / 2;
-    using Ar = GramArith<T, DF>;
-    using St = typename Ar::Stage;
-    constexpr int TE = gram_tile_elems<St>();
-    St *sS = (St *)smraw;  // [3][tiles][TE]: S, K S, M S
+    constexpr int TE = gram_tile_elems<T>();
+    T *sS = (T *)smraw;  // [3][tiles][TE]: S, K S, M S
     const bool active = (int)threadIdx.x < ntasks;
     int ti = 0, tj = 0, oi = 0, oj = 0;
     if (active) {
@@ -1112,19 +1226,14 @@ __global__ void __launch_bounds__(320)
         oi = ci % PW;
         oj = cj % PW;
     }
-    typename Ar::Acc aA[kGramSub][kGramSub], aB[kGramSub][kGramSub];
-#pragma unroll
-    for (int a = 0; a < kGramSub; ++a)
-#pragma unroll
-        for (int b = 0; b < kGramSub; ++b) {
-            aA[a][b].zero();
-            aB[a][b].zero();
-        }
+    GramTile<T> aA, aB;
+    aA.zero();
+    aB.zero();
     const int64_t per = (n + gridDim.x - 1) / gridDim.x;
     const int64_t r0 = (int64_t)blockIdx.x * per, r1 = min(n, r0 + per);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     constexpr int kPer16 = 16 / (int)sizeof(T);  // source values per 16-byte move
-    const St *pS = sS + ti * TE + oi, *pK = sS + (tiles + tj) * TE + oj, *pM = sS + (2 * tiles + tj) * TE + oj;
+    const T *pS = sS + ti * TE + oi, *pK = sS + (tiles + tj) * TE + oj, *pM = sS + (2 * tiles + tj) * TE + oj;
     for (int64_t t0 = r0; t0 < r1; t0 += kGramRows) {
         const int rows = (int)((r1 - t0) < (int64_t)kGramRows ? (r1 - t0) : (int64_t)kGramRows);
         const int units = rows * PW / kPer16;  // 16-byte moves per tile
@@ -1135,23 +1244,19 @@ __global__ void __launch_bounds__(320)
             const T *base = mat == 0 ? (b == 0 ? S0 : (b == 1 ? S1 : S2))
                                      : (mat == 1 ? (b == 0 ? K0 : (b == 1 ? K1 : K2)) : (b == 0 ? M0 : (b == 1 ? M1 : M2)));
             const T *src = base + ((int64_t)q * n + t0) * PW;
-            St *dst = sS + ta * TE;
+            T *dst = sS + ta * TE;
             for (int u = lane; u < units; u += 32) gram_stage16(src + u * kPer16, dst + u * kPer16);
         }
         __syncthreads();
         if (active) {
             for (int r = 0; r < rows; ++r) {
-                St si[kGramSub], yk[kGramSub], ym[kGramSub];
-                gram_lds4(pS + r * PW, si);
-                gram_lds4(pK + r * PW, yk);
-                gram_lds4(pM + r * PW, ym);
+                const typename GramTile<T>::Left si(pS + r * PW);
+                const typename GramTile<T>::Right yk(pK + r * PW), ym(pM + r * PW);
 #pragma unroll
-                for (int a = 0; a < kGramSub; ++a)
-#pragma unroll
-                    for (int b = 0; b < kGramSub; ++b) {
-                        aA[a][b].add(si[a], yk[b]);
-                        aB[a][b].add(si[a], ym[b]);
-                    }
+                for (int a = 0; a < kGramSub; ++a) {
+                    aA.add(a, si, yk);
+                    aB.add(a, si, ym);
+                }
             }
         }
     }
@@ -1166,8 +1271,8 @@ __global__ void __launch_bounds__(320)
             const int i = bi * k + ci, j = bj * k + cj;
             if (i > j) continue;
             const int p = i * m - i * (i - 1) / 2 + (j - i);
-            part[(int64_t)blockIdx.x * 2 * npairs + p] = aA[a][b].get();
-            part[(int64_t)blockIdx.x * 2 * npairs + npairs + p] = aB[a][b].get();
+            part[(int64_t)blockIdx.x * 2 * npairs + p] = aA.get(a, b);
+            part[(int64_t)blockIdx.x * 2 * npairs + npairs + p] = aB.get(a, b);
         }
 }
 
@@ -1678,9 +1783,7 @@ void gram(Ctx &c, int nblk, const Blocks<T> &B, std::vector<double> &GA, std::ve
     const int threads = (groups * (groups + 1) / 2 + 31) / 32 * 32;
     // staged tiles: 3 matrices x tiles; a double-float value is 8 bytes like a double
     const size_t smem = (size_t)3 * tiles * (kGramRows * PW + 64 / sizeof(T)) * sizeof(T);
-    // float2: double-float panels (mixed second phase); float: FP32; double: IEEE FP64
-    constexpr bool kDF = std::is_same<T, float2>::value;
-    auto kern = k_gram<T, kDF>;
+    auto kern = k_gram<T>;
     PFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // about 20 warps per SM: two CTAs of ten at k = 24, seven of three at k = 12 (two of
     // three left the pipes to latency: 58 us at 95k rows, now 29), a staged step each
