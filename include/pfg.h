@@ -398,7 +398,8 @@ typedef struct pfg_batch_config {
     int32_t threads;       /* threads per CTA (256, 512 or 1024): block rows of one CTA tile */
     int32_t cluster;       /* CTAs that solve one large system together (1, 2, 4 or 8) */
     double team_fraction;  /* share of the systems, largest estimated cost first, solved by a
-                              whole cluster; the rest are solved by single CTAs */
+                              whole cluster; the rest are solved by single CTAs, or by
+                              larger teams where one would outlast the others */
 } pfg_batch_config;
 
 typedef struct pfg_batch_info {

@@ -1,11 +1,12 @@
 // batch.cu -- persistent batched CG over many independent systems (batch.cuh).
 //
-// One launch solves every bound system.  Each CTA (or each cluster of CTAs,
-// for the largest systems) takes the next job from an atomic queue and runs a
-// complete preconditioned CG on it, with team-local reductions and no grid-wide
-// synchronisation; when the queue is empty the CTA retires.  Jobs are ordered
-// by estimated cost (the iteration count of the previous solve of the same
-// system, when there was one), so the longest systems start first.
+// One launch solves every bound system.  Each CTA (or each team of CTAs, for the
+// largest systems: a whole cluster, then its halves, each from its own queue) takes the
+// next job from an atomic queue and runs a complete preconditioned CG on it, with
+// team-local reductions and no grid-wide synchronisation; when the queues are empty
+// the CTA retires.  Jobs are ordered by estimated cost (the iteration count of the
+// previous solve of the same system, when there was one), so the longest systems
+// start first, and in the largest teams.
 //
 // Team step of one CG iteration (each warp of the team owns whole 32-row
 // slices of the system's sliced-ELL matrix, dealt out over the CTAs first so that
@@ -34,7 +35,7 @@ namespace cg = cooperative_groups;
 namespace pfg {
 namespace {
 
-constexpr int kMaxCluster = 8;
+constexpr int kMaxCluster = kMaxTeam;
 constexpr int kAbortEvery = 64;   // iterations between two reads of the abort flag
 // Mixed precision hands a system over to FP64 CG (from its current x) after
 // kMaxFailures FP32 passes in a row that broke down, overflowed or diverged
@@ -49,20 +50,61 @@ struct TeamShared {
     double slot[2][kMaxCluster][4];   // CTA totals of team reductions, one row per rank (every CTA holds all)
     double wpart[2][32][4];           // per-warp partials (FP64), double-buffered
     float wpart32[2][32][4];          // per-warp compensated partials (s, c pairs), double-buffered
+    uint64_t bar[kTeamSizes];         // mbarriers of teams smaller than the cluster, one per size
+    int lost;                         // a wait on one of them ran out
     double scalar[2][4];              // what thread 0 made of a reduction's totals, for the whole CTA
     int job;
 };
 
 struct Team {
-    int rank;   // CTA rank in the team
-    int size;   // CTAs in the team (1: a single CTA, no cluster barrier)
-    int nred;   // reductions done on this job (alternates the double buffers)
+    int rank;          // CTA rank in the team
+    int size;          // CTAs in the team (1: a single CTA)
+    int base;          // the team's first CTA in the cluster
+    bool whole;        // the team is the whole cluster
+    int level;         // mbarrier of this size
+    unsigned parity;   // of the mbarrier's current phase
+    int nred;          // reductions done on this job (alternates the double buffers)
 };
 
-__device__ __forceinline__ void team_sync(const Team &tm)
+constexpr long long kBarrierClocks = 1ll << 32;  // about two seconds, then a wait gives up
+
+// Barrier of the CTAs of a team, with release and acquire over the cluster: the
+// hardware's cluster barrier for a whole cluster; for a part of one an mbarrier in every
+// CTA's shared memory on which each CTA of the team arrives once.  A wait that runs out
+// marks the CTA lost: its solves end with an internal error.
+__device__ __forceinline__ void team_barrier(Team &tm, TeamShared &sh)
+{
+    if (tm.whole) {
+        cg::this_cluster().sync();
+        return;
+    }
+    __syncthreads();
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&sh.bar[tm.level]);
+    if ((int)threadIdx.x < tm.size) {
+        uint32_t remote;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(bar), "r"(tm.base + (int)threadIdx.x));
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
+    }
+    uint32_t done = 0;
+    const long long t0 = clock64();
+    while (!done) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(tm.parity)
+            : "memory");
+        if (!done && (*(volatile int *)&sh.lost || clock64() - t0 > kBarrierClocks)) break;
+    }
+    if (!done) *(volatile int *)&sh.lost = 1;
+    tm.parity ^= 1;
+}
+
+__device__ __forceinline__ void team_sync(Team &tm, TeamShared &sh)
 {
     if (tm.size > 1)
-        cg::this_cluster().sync();
+        team_barrier(tm, sh);
     else
         __syncthreads();
 }
@@ -111,11 +153,11 @@ __device__ __forceinline__ int team_reduce(double (&v)[NV], Team &tm, TeamShared
     if (tm.size > 1) {
         cg::cluster_group cl = cg::this_cluster();
         if (wid == 0 && lane < tm.size) {
-            double *dst = cl.map_shared_rank(&sh.slot[buf][tm.rank][0], lane);
+            double *dst = cl.map_shared_rank(&sh.slot[buf][tm.rank][0], tm.base + lane);
 #pragma unroll
             for (int k = 0; k < NV; ++k) dst[k] = v[k];
         }
-        cl.sync();
+        team_barrier(tm, sh);
         if (wid == 0) {
             // lane 16 k + r: value k of rank r
             const int r = lane & 15, k = NV == 2 ? lane >> 4 : 0;
@@ -178,14 +220,14 @@ __device__ __forceinline__ void team_sum_comp(Comp32 (&v)[NV], float (&tot)[NV],
     if (tm.size > 1) {
         cg::cluster_group cl = cg::this_cluster();
         if (wid == 0 && lane < tm.size) {
-            double *dst = cl.map_shared_rank(&sh.slot[buf][tm.rank][0], lane);
+            double *dst = cl.map_shared_rank(&sh.slot[buf][tm.rank][0], tm.base + lane);
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
                 dst[2 * k] = (double)v[k].s;
                 dst[2 * k + 1] = (double)v[k].c;
             }
         }
-        cl.sync();
+        team_barrier(tm, sh);
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             v[k].s = lane < tm.size ? (float)sh.slot[buf][lane][2 * k] : 0.f;
@@ -524,20 +566,20 @@ __device__ int cg64(const BatchParams &P, const BatchMesh &D, Team &tm, TeamShar
                 }
             }
         }
-        team_sync(tm);
+        team_sync(tm, sh);
     }
     const double rt = residual64(D, sp, tm, sh);
     rel = bb > 0.0 ? sqrt(rt / bb) : 0.0;
     return status;
 }
 
-__device__ void finish_job(const BatchParams &P, int m, const BatchMesh &D, Team &tm, int status, int it,
-                           int reps, int fallback, double rel)
+__device__ void finish_job(const BatchParams &P, int m, const BatchMesh &D, Team &tm, const TeamShared &sh,
+                           int status, int it, int reps, int fallback, double rel)
 {
     restore_fixed_rows(D, team_span(tm, blockDim.x / 32), D.A64.nb);
     if (tm.rank == 0 && threadIdx.x == 0) {
         BatchOut o;
-        o.status = status;
+        o.status = sh.lost ? PFG_E_INTERNAL : status;
         o.iterations = it;
         o.replacements = reps;
         o.team_size = tm.size;
@@ -554,7 +596,7 @@ __device__ void solve_fp64(const BatchParams &P, int m, Team &tm, TeamShared &sh
     int it = 0, restarts = 0;
     double rel = 0.0;
     const int status = cg64<NT>(P, D, tm, sh, it, restarts, rel);
-    finish_job(P, m, D, tm, status, it, restarts, fallback, rel);
+    finish_job(P, m, D, tm, sh, status, it, restarts, fallback, rel);
 }
 
 // ------------------------------------------- FP32 CG with FP64 replacement
@@ -631,7 +673,7 @@ __device__ void solve_mixed(const BatchParams &P, int m, Team &tm, TeamShared &s
                     D.p32[i] = beta == 0.f ? D.z32[i] : fmaf(beta, D.p32[i], D.z32[i]);
                 }
             }
-            team_sync(tm);
+            team_sync(tm, sh);
         }
         // FP32 iterations until the residual fell by delta (or trouble)
         bool poisoned = false, broke = false, diverged = false;
@@ -711,7 +753,7 @@ __device__ void solve_mixed(const BatchParams &P, int m, Team &tm, TeamShared &s
                     D.p32[i] = fmaf(beta, D.p32[i], D.z32[i]);
                 }
             }
-            team_sync(tm);
+            team_sync(tm, sh);
         }
         // Keep the FP32 correction only if it lowers the FP64 residual: the
         // candidate b - K (x + x32) goes to q64; on acceptance it becomes r64
@@ -735,7 +777,7 @@ __device__ void solve_mixed(const BatchParams &P, int m, Team &tm, TeamShared &s
                 D.x32[i] = 0.f;
             }
         }
-        team_sync(tm);
+        team_sync(tm, sh);
         ++reps;
         if (accepted) cur_rt = rt;
         rt = cur_rt;
@@ -765,7 +807,7 @@ __device__ void solve_mixed(const BatchParams &P, int m, Team &tm, TeamShared &s
             break;
         }
     }
-    finish_job(P, m, D, tm, status, it, reps, fallback, rel);
+    finish_job(P, m, D, tm, sh, status, it, reps, fallback, rel);
 }
 
 template <bool MIXED, int NT>
@@ -778,34 +820,56 @@ __device__ __forceinline__ void solve_job(const BatchParams &P, int m, Team &tm,
 }
 
 template <bool MIXED, int NT>
-__global__ void __launch_bounds__(NT, 1) k_batch_cg(BatchParams P)
+__global__ void __launch_bounds__(NT, 1) k_batch_cg(const __grid_constant__ BatchParams P)
 {
     __shared__ TeamShared sh;
     if (P.cluster > 1) {
-        // team phase: the cluster takes jobs together
+        // team phases: the cluster takes jobs together, then its halves, ...
         cg::cluster_group cl = cg::this_cluster();
-        const int rank = (int)cl.block_rank();
-        for (;;) {
-            if (rank == 0 && threadIdx.x == 0) sh.job = (int)atomicAdd(P.queue, 1u);
-            cl.sync();
-            const int job = *cl.map_shared_rank(&sh.job, 0);
-            cl.sync();  // every CTA has read the job before rank 0 overwrites it
-            if (job >= P.n_team) break;
-            Team tm{rank, P.cluster, 0};
-            solve_job<MIXED, NT>(P, P.order[job], tm, sh);
+        const int me = (int)cl.block_rank();
+        if (threadIdx.x == 0) {
+            sh.lost = 0;
+            for (int l = 0; l < kTeamSizes; ++l)
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(&sh.bar[l])),
+                             "r"(kMaxTeam >> l)
+                             : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
+        cl.sync();
+        int first = 0;
+        for (int l = 0; l < kTeamSizes; first += P.n_team[l++]) {
+            const int size = kMaxTeam >> l;
+            if (P.n_team[l] == 0) continue;
+            Team tm{me % size, size, me / size * size, size == P.cluster, l, 0, 0};
+            for (;;) {
+                if (tm.rank == 0 && threadIdx.x == 0) sh.job = (int)atomicAdd(P.queue + l, 1u);
+                team_barrier(tm, sh);
+                const int job = *cl.map_shared_rank(&sh.job, tm.base);
+                team_barrier(tm, sh);  // every CTA has read the job before rank 0 overwrites it
+                if (job >= P.n_team[l] || *(volatile int *)&sh.lost) break;
+                tm.nred = 0;
+                solve_job<MIXED, NT>(P, P.order[first + job], tm, sh);
+            }
+        }
+    } else if (threadIdx.x == 0) {
+        sh.lost = 0;
     }
     // single-CTA phase
-    const int n_solo = P.n_total - P.n_team;
+    int n_solo = P.n_total, solo0 = 0;
+    for (int l = 0; l < kTeamSizes; ++l) solo0 += P.n_team[l];
+    n_solo -= solo0;
     for (;;) {
-        if (threadIdx.x == 0) sh.job = (int)atomicAdd(P.queue + 1, 1u);
+        if (threadIdx.x == 0) sh.job = (int)atomicAdd(P.queue + kTeamSizes, 1u);
         __syncthreads();
         const int job = sh.job;
         __syncthreads();
         if (job >= n_solo) break;
-        Team tm{0, 1, 0};
-        solve_job<MIXED, NT>(P, P.order[P.n_team + job], tm, sh);
+        Team tm{0, 1, 0, false, 0, 0, 0};
+        solve_job<MIXED, NT>(P, P.order[solo0 + job], tm, sh);
     }
+    // no CTA of a cluster leaves while another may still reach its shared memory
+    if (P.cluster > 1) cg::this_cluster().sync();
 }
 
 }  // namespace
@@ -910,6 +974,7 @@ struct pfg_batch {
     DevBuf<int> order;
     DevBuf<unsigned> queue;
     std::vector<double> work;         // matrix blocks of each system (work per iteration)
+    std::vector<int> team;            // CTAs of each system's team in the current solve
     std::vector<int> last_iters;      // iterations of the previous solve (0: none yet)
     std::vector<int> iters64;         // iterations of the last FP64 solve of each system (0: none)
     std::vector<uint8_t> force64;     // mixed: systems to solve in FP64 (learned)
@@ -933,6 +998,8 @@ struct pfg_batch {
 };
 
 namespace {
+
+constexpr double kLongJob = 0.5, kWiderCluster = 0.9;  // team sizes: see run_batch
 
 void need(bool c, int code, const char *msg)
 {
@@ -987,19 +1054,55 @@ double run_batch(pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c)
         cost[m] = b->work[m] * it;
     }
     std::stable_sort(ord.begin(), ord.end(), [&](int a, int d) { return cost[a] > cost[d]; });
+    PFG_CUDA(cudaMemcpyAsync(b->order.p, ord.data(), count * sizeof(int), cudaMemcpyHostToDevice, b->st));
     int n_team = 0;
     if (c.cluster > 1) n_team = std::min(count, (int)std::lround(c.team_fraction * count));
-    PFG_CUDA(cudaMemcpyAsync(b->order.p, ord.data(), count * sizeof(int), cudaMemcpyHostToDevice, b->st));
-
-    const int grid = persistent_grid(rs.mixed, c.threads, c.cluster);
+    int cluster = c.cluster;
+    int grid = persistent_grid(rs.mixed, c.threads, cluster);
     need(grid > 0, PFG_E_UNSUPPORTED, "batched kernel configuration cannot be resident on this GPU");
+    // Team sizes.  The n_team largest systems get a whole cluster; a system that would
+    // keep its team busy for more than kLongJob of the balanced time (all costs over
+    // all CTAs) gets the next larger team, since one long system bounds the whole solve
+    // otherwise: 256 uneven slabs in pairs and single CTAs are 125 ms of work per SM and
+    // took 220 ms, the longest pair's time; now 178.  A limit of 0.5, 0.7, 0.85, 1.0 and
+    // 1.15 gave 181, 179, 181, 174 and 162 ms there and 179, 198, 203, 203 and 203 in
+    // clusters of four; the low one also does best while the costs are guessed (the
+    // first solve, 291 -> 238 ms).  Clusters of four fill 144 of the 152 SMs, of eight
+    // 120, so pairs grow to fours, only if the longest needs it, and fours don't grow.
+    // A team's CTAs keep at least a slice for each quarter of the SM (FP64) or each of
+    // sixteen warps (mixed, where the barriers weigh more: 37 slices on 1, 2 and 4 CTAs
+    // 19.8, 15.8 and 11.8 us an iteration, in FP64 73.8, 44.5 and 26.0).
+    double total = 0.0;
+    for (int m = 0; m < count; ++m) total += cost[m];
+    if (n_team > 0 && cluster == 2 && cost[ord[0]] > kWiderCluster * 2 * total / grid) {
+        const int wider = persistent_grid(rs.mixed, c.threads, 4);
+        if (wider > 0) {
+            cluster = 4;
+            grid = wider;
+        }
+    }
+    int n_size[kTeamSizes] = {};
+    for (int k = 0; k < count && n_team > 0; ++k) {
+        const int m = ord[k];
+        int size = k < n_team ? c.cluster : 1;
+        while (size < cluster && cost[m] > kLongJob * size * total / grid &&
+               b->ndof[m] >= (int64_t)2 * size * (rs.mixed ? 16 : 4) * 96)
+            size *= 2;
+        // (never a larger team than a costlier system's: the order lists the sizes in turn)
+        if (k > 0) size = std::min(size, b->team[ord[k - 1]]);
+        b->team[m] = size;
+        if (size == 1) break;
+        for (int l = 0; l < kTeamSizes; ++l)
+            if (size == kMaxTeam >> l) ++n_size[l];
+    }
+
     BatchParams P;
     P.mesh = b->meshes.p;
     P.out = b->out.p;
     P.order = b->order.p;
-    P.n_team = n_team;
+    std::copy(n_size, n_size + kTeamSizes, P.n_team);
     P.n_total = count;
-    P.cluster = c.cluster;
+    P.cluster = cluster;
     P.queue = b->queue.p;
     P.precond = rs.precond;
     P.itrmax = rs.itrmax;
@@ -1013,7 +1116,7 @@ double run_batch(pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c)
 
     uint64_t key = 0x51ab;
     for (uint64_t v : {(uint64_t)rs.mixed, (uint64_t)rs.precond, (uint64_t)rs.itrmax, (uint64_t)c.threads,
-                       (uint64_t)c.cluster, (uint64_t)n_team, (uint64_t)count, (uint64_t)grid,
+                       (uint64_t)cluster, (uint64_t)n_size[0], (uint64_t)n_size[1], (uint64_t)n_size[2], (uint64_t)count, (uint64_t)grid,
                        (uint64_t)(uintptr_t)b->meshes.p, (uint64_t)(uintptr_t)b->v64.p,
                        (uint64_t)(uintptr_t)b->abort_d, (uint64_t)(uintptr_t)b->force64_d.p})
         key = mix(key, v);
@@ -1028,10 +1131,10 @@ double run_batch(pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c)
         PFG_CUDA(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
         // x0 = 0 for every system, empty job queues, then the persistent kernel
         cudaMemsetAsync(b->v64.p, 0, b->total * sizeof(double), b->st);
-        cudaMemsetAsync(b->queue.p, 0, 2 * sizeof(unsigned), b->st);
+        cudaMemsetAsync(b->queue.p, 0, (kTeamSizes + 1) * sizeof(unsigned), b->st);
         cudaLaunchConfig_t lc;
         cudaLaunchAttribute attr;
-        fill_launch(lc, attr, grid, c.threads, c.cluster, b->st);
+        fill_launch(lc, attr, grid, c.threads, cluster, b->st);
         void *args[] = {&P};
         const cudaError_t le = cudaLaunchKernelExC(&lc, batch_kernel(rs.mixed, c.threads), args);
         const cudaError_t ce = cudaStreamEndCapture(b->st, &g);
@@ -1082,7 +1185,7 @@ int pfg_batch_create(pfg_batch **out)
             PFG_CUDA(cudaHostAlloc((void **)&b->abort_h, sizeof(int), cudaHostAllocMapped));
             *b->abort_h = 0;
             PFG_CUDA(cudaHostGetDevicePointer((void **)&b->abort_d, b->abort_h, 0));
-            b->queue.alloc(2);
+            b->queue.alloc(kTeamSizes + 1);
         } catch (...) {
             delete b;
             throw;
@@ -1122,6 +1225,7 @@ int pfg_batch_set(pfg_batch *b, int64_t count, pfg_solver *const *handles)
         b->ndof.resize((size_t)count);
         b->off.resize((size_t)count);
         b->work.resize((size_t)count);
+        b->team.assign((size_t)count, 1);
         b->last_iters.assign((size_t)count, 0);
         b->iters64.assign((size_t)count, 0);
         b->force64.assign((size_t)count, 0);

@@ -61,14 +61,16 @@ struct BatchOut {
     double rel_residual;   // true |b - Kx| / |b|
 };
 
+constexpr int kMaxTeam = 8, kTeamSizes = 3;  // teams of 8, 4 and 2 CTAs
+
 struct BatchParams {
     const BatchMesh *mesh;
     BatchOut *out;
-    const int *order;         // job order: team jobs, then single-CTA jobs
-    int n_team;               // first n_team jobs are solved by a whole cluster
+    const int *order;         // job order: the jobs of the largest teams first, single-CTA jobs last
+    int n_team[kTeamSizes];   // jobs of teams of 8, 4 and 2 CTAs
     int n_total;
-    int cluster;              // CTAs per cluster (1: no cluster launch)
-    unsigned *queue;          // [0] team queue, [1] single-CTA queue (zero at launch)
+    int cluster;              // CTAs per cluster (1: no cluster launch), the largest team's size
+    unsigned *queue;          // a queue per team size, then the single-CTA queue (zero at launch)
     int precond;              // PFG_PC_NONE / PFG_PC_JACOBI / PFG_PC_BLOCK_JACOBI
     int itrmax;
     int max_restarts;

@@ -174,3 +174,26 @@ def test_batch_error_returns(cuda):
         b.set([s1])
     assert e.value.code == -9
     del dom
+
+
+# Team sizes: one or two long systems among short ones get teams of four or of both
+# halves of a cluster, down to sizes whose slices are fewer than the team's warps (and
+# than its CTAs, where the whole batch is solved in clusters); the second solve
+# knows the iteration counts.
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("cfg", [(256, 2, 0.1), (512, 2, 0.1), (512, 4, 0.1), (512, 8, 0.1), (1024, 8, 1.0)])
+def test_batch_long_systems_in_larger_teams(cuda, precision, cfg):
+    if "teams" not in _CACHE:
+        dims = [(24, 20, 3), (20, 7, 2), (14, 14, 2), (9, 9, 3), (7, 6, 1), (4, 4, 1)] + [(5, 3, 1), (2, 2, 1)] * 4
+        ps = [problems.slab(*d, 1.0e4 * (1.0 + 0.1 * k)) for k, d in enumerate(dims)]
+        _CACHE["teams"] = (ps, [_oracle(p) for p in ps])
+    ps, refs = _CACHE["teams"]
+    b = FEMSolverBatch([_solver(p) for p in ps])
+    b.config = {"threads": cfg[0], "cluster": cfg[1], "team_fraction": cfg[2]}
+    for _ in range(3):
+        xs = b.solve(precision=precision, relative_er=TOL)
+        assert b.last_info["launches"] == 1
+        for k, (x, ref) in enumerate(zip(xs, refs)):
+            inf = b.last_infos[k]
+            assert inf["status"] == 0 and inf["rel_residual"] <= TOL, (k, inf)
+            assert _rel(x, ref) <= 1e-8, (k, _rel(x, ref))  # conditioning times TOL, as above
