@@ -1065,7 +1065,10 @@ __global__ void __launch_bounds__(kT)
     }
 }
 
-constexpr int kGramRows = 32;  // rows staged in shared memory per step
+// Rows staged in shared memory per step.  16, 32, 48 and 64 rows took 34, 29, 27 and
+// 27 us (FP32) and 90, 94, 85 and 105 us (double-float) at 95k rows and 12 columns, and
+// 356, 256, 228, 210 and 1,302, 1,177, 1,167, 1,160 us at 398k and 24.
+constexpr int kGramRows = 48;
 constexpr int kGramSub = 4;    // each thread owns a 4 x 4 sub-tile of both Gram matrices
 
 // Shared-memory tile of the Gram staging: kGramRows rows of one 8-column
@@ -1276,24 +1279,27 @@ __global__ void __launch_bounds__(320)
         }
 }
 
-// Sum the per-CTA partials (deterministic): a CTA takes 32 values, its 32 warps a
-// share of the partials each, added in warp order.  (A thread per value that ran
-// through the partials alone: 55 us for 304 partials of 1,332 values; this 15.)
-__global__ void __launch_bounds__(1024)
+// Sum the per-CTA partials (deterministic): a CTA takes 8 values, 32 threads a share
+// of the partials of each, added in thread order.  The additions alone hold the FP64
+// pipe (1,520 partials of 1,332 values are 2 M, 4 us over all SMs), so the values go to
+// as many SMs as there are: 15 us with 32 values to a CTA, 8 now (a thread per
+// value that ran through the partials alone: 55).
+constexpr int kReduceValues = 8;
+__global__ void __launch_bounds__(256)
     k_reduce_parts(const double *__restrict__ part, int nparts, int len, double *__restrict__ out)
 {
-    __shared__ double sums[32][33];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + lane;
+    __shared__ double sums[32][kReduceValues + 1];
+    const int v = threadIdx.x % kReduceValues, g = threadIdx.x / kReduceValues;
+    const int i = blockIdx.x * kReduceValues + v;
     double s = 0.0;
     if (i < len)
 #pragma unroll 8
-        for (int b = w; b < nparts; b += 32) s += part[(int64_t)b * len + i];
-    sums[w][lane] = s;
+        for (int b = g; b < nparts; b += 32) s += part[(int64_t)b * len + i];
+    sums[g][v] = s;
     __syncthreads();
-    if (w == 0 && i < len) {
+    if (g == 0 && i < len) {
         double t = 0.0;
-        for (int k = 0; k < 32; ++k) t += sums[k][lane];
+        for (int k = 0; k < 32; ++k) t += sums[k][v];
         out[i] = t;
     }
 }
@@ -1382,7 +1388,7 @@ __global__ void __launch_bounds__(kT)
 // sums are FP64 (no FP32 underflow of squares for badly scaled systems); what bounds
 // a small system is adding them across the CTA on the FP64 pipe, so the 16 sums
 // are halved from lane to lane (16 additions per warp instead of 80) and FP32
-// maxima stay FP32: 56 -> 22 us at 95k rows, k = 12.
+// maxima stay FP32, and a thread takes two rows or more: 56 -> 14 us at 95k rows, k = 12.
 // double-float panels: the difference on the FP32 pipe (lam split once per
 // column), the sums of the leading floats (seven digits are all a norm needs).
 __device__ __forceinline__ float res_lam(float, double l) { return (float)l; }
@@ -1786,7 +1792,7 @@ void gram(Ctx &c, int nblk, const Blocks<T> &B, std::vector<double> &GA, std::ve
     auto kern = k_gram<T>;
     PFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // about 20 warps per SM: two CTAs of ten at k = 24, seven of three at k = 12 (two of
-    // three left the pipes to latency: 58 us at 95k rows, now 29), a staged step each
+    // three left the pipes to latency: 58 us at 95k rows, now 27), a staged step each
     int occ = 0;
     PFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
     const int per_sm = std::max(1, std::min(std::max(2, 20 * 32 / threads), occ));
@@ -1795,7 +1801,7 @@ void gram(Ctx &c, int nblk, const Blocks<T> &B, std::vector<double> &GA, std::ve
     c.gram.ensure((size_t)2 * npairs);
     kern<<<g, threads, smem, c.st>>>(c.n, c.k, nblk, B.X.p, B.W.p, B.P.p, B.KX.p, B.KW.p, B.KP.p, B.MX.p, B.MW.p,
                                      B.MP.p, c.part.p);
-    k_reduce_parts<<<(2 * npairs + 31) / 32, 1024, 0, c.st>>>(c.part.p, g, 2 * npairs, c.gram.p);
+    k_reduce_parts<<<(2 * npairs + kReduceValues - 1) / kReduceValues, 256, 0, c.st>>>(c.part.p, g, 2 * npairs, c.gram.p);
     PFG_CUDA(cudaGetLastError());
     c.launches += 2;
     PFG_CUDA(cudaMemcpyAsync(c.pin, c.gram.p, 2 * npairs * sizeof(double), cudaMemcpyDeviceToHost, c.st));
@@ -1874,7 +1880,7 @@ struct ResInfo {
 template <typename T>
 void residuals(Ctx &c, Blocks<T> &B)
 {
-    const int g = (int)std::min<int64_t>((c.n + kT - 1) / kT, c.ngrid);
+    const int g = (int)std::min<int64_t>((c.n + 2 * kT - 1) / (2 * kT), c.ngrid);
     c.part.ensure((size_t)g * 3 * c.k);
     c.rsum.ensure((size_t)3 * c.k);
     k_residual<T><<<dim3(g, c.np), kT, 0, c.st>>>(c.n, c.k, B.KX.p, B.MX.p, c.lam_d.p, B.R.p, c.part.p);
