@@ -1642,22 +1642,27 @@ struct Ctx {
     DevBuf<float2> df_K, df_M;  // the sliced FP64 matrix values as double-float pairs (mixed second phase)
     const DevMatrix *dfK = nullptr, *dfM = nullptr;
     int launches = 0;
-    DevBuf<double> part, gram, C, lam_d, dinv, rsum;
+    DevBuf<double> part, C, dinv;
+    const double *lam_d = nullptr;  // behind the coefficients in C
     std::vector<double> hC, hlam;
-    double *pin = nullptr;     // page-locked: the small matrices and sums on their way
+    double *pin = nullptr;     // page-locked, read and written by the device: small matrices and sums
     cudaEvent_t sums = nullptr;  // the residuals' sums have arrived
     bool one_pattern = false;  // K and M share their sliced pattern
     int ngrid;
     ~Ctx()
     {
-        if (pin) cudaFreeHost(pin);
+        if (pin) {
+            cudaStreamSynchronize(st);  // (kernels write there)
+            cudaFreeHost(pin);
+        }
         if (sums) cudaEventDestroy(sums);
     }
 };
 
-// doubles of Ctx::pin: both Gram triangles and the coefficients of three blocks of
-// at most 32 columns
-constexpr size_t kPinDoubles = 96 * 97 + 96 * 32 + 3 * 32;
+// Ctx::pin, in doubles: both Gram triangles of three blocks of at most 32 columns and
+// the residuals' sums, which the kernels that form them write straight to the host (a copy of
+// its own costs more than the few KB take), then the coefficients and Ritz values.
+constexpr size_t kPinSums = 96 * 97, kPinCoef = kPinSums + 3 * 32, kPinDoubles = kPinCoef + 96 * 32 + 32;
 
 template <typename T>
 SellView<T> sell_of(const DevMatrix &A)
@@ -1798,13 +1803,11 @@ void gram(Ctx &c, int nblk, const Blocks<T> &B, std::vector<double> &GA, std::ve
     const int per_sm = std::max(1, std::min(std::max(2, 20 * 32 / threads), occ));
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((c.n + kGramRows - 1) / kGramRows, (int64_t)sms() * per_sm));
     c.part.ensure((size_t)g * 2 * npairs);
-    c.gram.ensure((size_t)2 * npairs);
     kern<<<g, threads, smem, c.st>>>(c.n, c.k, nblk, B.X.p, B.W.p, B.P.p, B.KX.p, B.KW.p, B.KP.p, B.MX.p, B.MW.p,
                                      B.MP.p, c.part.p);
-    k_reduce_parts<<<(2 * npairs + kReduceValues - 1) / kReduceValues, 256, 0, c.st>>>(c.part.p, g, 2 * npairs, c.gram.p);
+    k_reduce_parts<<<(2 * npairs + kReduceValues - 1) / kReduceValues, 256, 0, c.st>>>(c.part.p, g, 2 * npairs, c.pin);
     PFG_CUDA(cudaGetLastError());
     c.launches += 2;
-    PFG_CUDA(cudaMemcpyAsync(c.pin, c.gram.p, 2 * npairs * sizeof(double), cudaMemcpyDeviceToHost, c.st));
     PFG_CUDA(cudaStreamSynchronize(c.st));
     GA.assign((size_t)m * m, 0.0);
     GB.assign((size_t)m * m, 0.0);
@@ -1844,14 +1847,13 @@ int rayleigh_ritz(Ctx &c, int nblk, const Blocks<T> &B, double rank_tol)
     c.hlam.assign(c.k, 0.0);
     const int got = small_generalized_eig(m, GA.data(), GB.data(), c.k, rank_tol, c.hlam.data(), c.hC.data());
     if (got < c.k) return got;
-    c.C.ensure((size_t)m * c.k);
-    c.lam_d.ensure((size_t)c.k);
-    // (the copies have left these buffers before the next synchronisation that precedes their reuse)
-    double *pc = c.pin + 96 * 97, *pl = pc + 96 * 32;
-    std::copy(c.hC.begin(), c.hC.end(), pc);
-    std::copy(c.hlam.begin(), c.hlam.end(), pl);
-    PFG_CUDA(cudaMemcpyAsync(c.C.p, pc, (size_t)m * c.k * sizeof(double), cudaMemcpyHostToDevice, c.st));
-    PFG_CUDA(cudaMemcpyAsync(c.lam_d.p, pl, c.k * sizeof(double), cudaMemcpyHostToDevice, c.st));
+    // (the copy has left this buffer before the next synchronisation that precedes its reuse)
+    const size_t len = (size_t)m * c.k;
+    c.C.ensure(len + c.k);
+    c.lam_d = c.C.p + len;
+    std::copy(c.hC.begin(), c.hC.end(), c.pin + kPinCoef);
+    std::copy(c.hlam.begin(), c.hlam.end(), c.pin + kPinCoef + len);
+    PFG_CUDA(cudaMemcpyAsync(c.C.p, c.pin + kPinCoef, (len + c.k) * sizeof(double), cudaMemcpyHostToDevice, c.st));
     return got;
 }
 
@@ -1882,20 +1884,17 @@ void residuals(Ctx &c, Blocks<T> &B)
 {
     const int g = (int)std::min<int64_t>((c.n + 2 * kT - 1) / (2 * kT), c.ngrid);
     c.part.ensure((size_t)g * 3 * c.k);
-    c.rsum.ensure((size_t)3 * c.k);
-    k_residual<T><<<dim3(g, c.np), kT, 0, c.st>>>(c.n, c.k, B.KX.p, B.MX.p, c.lam_d.p, B.R.p, c.part.p);
-    k_reduce_residual<<<(3 * c.k + 7) / 8, 256, 0, c.st>>>(c.part.p, g, 3 * c.k, c.rsum.p);
+    k_residual<T><<<dim3(g, c.np), kT, 0, c.st>>>(c.n, c.k, B.KX.p, B.MX.p, c.lam_d, B.R.p, c.part.p);
+    k_reduce_residual<<<(3 * c.k + 7) / 8, 256, 0, c.st>>>(c.part.p, g, 3 * c.k, c.pin + kPinSums);
     PFG_CUDA(cudaGetLastError());
     c.launches += 2;
-    double *h = c.pin + 96 * 97 + 96 * 32;
-    PFG_CUDA(cudaMemcpyAsync(h, c.rsum.p, (size_t)3 * c.k * sizeof(double), cudaMemcpyDeviceToHost, c.st));
     PFG_CUDA(cudaEventRecord(c.sums, c.st));
 }
 
 static ResInfo read_residuals(Ctx &c)
 {
     PFG_CUDA(cudaEventSynchronize(c.sums));
-    const double *h = c.pin + 96 * 97 + 96 * 32;
+    const double *h = c.pin + kPinSums;
     ResInfo ri;
     ri.rel.assign(c.k, 0.0);
     ri.maxabs.assign(c.k, 0.0);
