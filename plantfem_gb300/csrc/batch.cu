@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <functional>
 #include <mutex>
 #include <numeric>
 #include <vector>
@@ -974,7 +975,6 @@ struct pfg_batch {
     DevBuf<int> order;
     DevBuf<unsigned> queue;
     std::vector<double> work;         // matrix blocks of each system (work per iteration)
-    std::vector<int> team;            // CTAs of each system's team in the current solve
     std::vector<int> last_iters;      // iterations of the previous solve (0: none yet)
     std::vector<int> iters64;         // iterations of the last FP64 solve of each system (0: none)
     std::vector<uint8_t> force64;     // mixed: systems to solve in FP64 (learned)
@@ -999,7 +999,6 @@ struct pfg_batch {
 
 namespace {
 
-constexpr double kLongJob = 0.5, kWiderCluster = 0.9;  // team sizes: see run_batch
 
 void need(bool c, int code, const char *msg)
 {
@@ -1034,6 +1033,106 @@ RunSpec run_spec(const pfg_solve_opts *opts)
     return RunSpec{o.precision == PFG_PREC_MIXED, o.precond, o.itrmax, o.relative_er, o.reliable_delta, o.debug};
 }
 
+struct TeamPlan {
+    int cluster, grid;
+    int n[kTeamSizes];  // systems, in the job order, for teams of 8, 4 and 2 CTAs
+};
+
+// Team sizes.  The n_team largest systems get a whole cluster; a system that would keep
+// its team busy for more than `limit` of the balanced time (all costs over all
+// CTAs) gets the next larger team, since one long system bounds the whole solve
+// otherwise.  A team's CTAs keep at least a slice for each quarter of the SM (FP64)
+// or each of sixteen warps (mixed, where the barriers weigh more).  No system gets a
+// larger team than a costlier one: the job order lists the sizes in turn.
+TeamPlan teams_within(const pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c, const std::vector<int> &ord,
+                      const std::vector<double> &cost, double total, int n_team, int cluster, int grid, double limit)
+{
+    TeamPlan p{cluster, grid, {}};
+    int last = kMaxTeam;
+    for (size_t k = 0; k < ord.size(); ++k) {
+        const int m = ord[k];
+        int size = (int)k < n_team ? c.cluster : 1;
+        while (size < cluster && cost[m] > limit * size * total / grid &&
+               b->ndof[m] >= (int64_t)2 * size * (rs.mixed ? 16 : 4) * 96)
+            size *= 2;
+        last = size = std::min(size, last);
+        if (size == 1) break;
+        for (int l = 0; l < kTeamSizes; ++l)
+            if (size == kMaxTeam >> l) ++p.n[l];
+    }
+    return p;
+}
+
+// Time of a plan when every queue's jobs go to the team that is free first, as on the
+// device.  An iteration in microseconds, fitted to 6, 11, 19, 37, 79 and 211 slices on
+// 1, 2, 4 and 8 CTAs (FP64: the slices of the busiest quarter of an SM, and a
+// cluster's barriers; larger teams up to 9 % more, as the odd slices' warps run alone).
+double plan_time(const pfg_batch *b, const RunSpec &rs, const std::vector<int> &ord, const TeamPlan &p)
+{
+    std::vector<double> free_at((size_t)p.grid / p.cluster, 0.0);
+    size_t k = 0;
+    for (int size = p.cluster; size >= 1; size /= 2) {
+        size_t n = ord.size() - k;
+        for (int l = 0; l < kTeamSizes; ++l)
+            if (size == kMaxTeam >> l) n = (size_t)p.n[l];
+        std::make_heap(free_at.begin(), free_at.end(), std::greater<double>());
+        for (size_t j = 0; j < n; ++j, ++k) {
+            const int m = ord[k];
+            const double ns = std::ceil((double)b->ndof[m] / 96.0);
+            const bool f64 = !rs.mixed || b->force64[m];
+            const double width = 3.0 * b->work[m] / (double)b->ndof[m];  // blocks in a row
+            const double us = f64 ? (0.31 * width + 0.9) * std::ceil(ns / (4.0 * size)) + (size > 1 ? 5.0 : 1.0)
+                                  : 1.65 * ns / (4.0 * size) + (size > 1 ? 8.0 : 4.5);
+            std::pop_heap(free_at.begin(), free_at.end(), std::greater<double>());
+            free_at.back() += (size > 2 ? 1.05 * us : us) * b->last_iters[m];
+            std::push_heap(free_at.begin(), free_at.end(), std::greater<double>());
+        }
+        if (size > 1) {  // each team splits in two
+            const size_t teams = free_at.size();
+            free_at.resize(2 * teams);
+            std::copy(free_at.begin(), free_at.begin() + teams, free_at.begin() + teams);
+        }
+    }
+    return *std::max_element(free_at.begin(), free_at.end());
+}
+
+// The limit.  256 uneven slabs in pairs and single CTAs are 125 ms of FP64 work per SM
+// and took 220 ms, the longest pair's time.  Limits of 0.5, 0.7, 0.85, 1.0 and 1.15 gave
+// 181, 179, 181, 174 and 162 ms, and 179, 198, 203, 203 and 203 in clusters of four, so
+// once a solve has counted the iterations the one of the shortest plan is taken (163-170
+// ms); in a first solve, with costs guessed, 0.5 (291 -> 218 ms; 1.15 is the longest
+// pair's time again).  Clusters of four fill 144 of the 152 SMs, of eight 120: pairs may
+// grow to fours, for a first solve only if the longest clearly needs it, and
+// fours don't grow.  Many systems for each CTA balance by themselves: no plans compared.
+TeamPlan plan_teams(const pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c, const std::vector<int> &ord,
+                    const std::vector<double> &cost, int n_team, int grid)
+{
+    constexpr double kGuessed = 0.5, kWider = 0.9;
+    const double total = std::accumulate(cost.begin(), cost.end(), 0.0);
+    const int wider = c.cluster == 2 ? persistent_grid(rs.mixed, c.threads, 4) : 0;
+    const bool known = std::all_of(b->last_iters.begin(), b->last_iters.end(), [](int it) { return it > 0; });
+    if (!known || ord.size() > (size_t)16 * grid) {
+        const bool wide = wider > 0 && cost[ord[0]] > kWider * 2 * total / grid;
+        return teams_within(b, rs, c, ord, cost, total, n_team, wide ? 4 : c.cluster, wide ? wider : grid, kGuessed);
+    }
+    TeamPlan best{};
+    double best_time = 0.0;
+    for (int cluster : {c.cluster, 4}) {
+        if (cluster != c.cluster && wider <= 0) continue;
+        for (double limit = 0.4; limit < 1.65; limit += 0.1) {
+            const TeamPlan p = teams_within(b, rs, c, ord, cost, total, n_team, cluster,
+                                            cluster == c.cluster ? grid : wider, limit);
+            const double t = plan_time(b, rs, ord, p);
+            if (best.cluster == 0 || t < best_time) {
+                best = p;
+                best_time = t;
+            }
+        }
+        if (c.cluster == 4) break;
+    }
+    return best;
+}
+
 // Launches one batched solve with configuration c (graph replay when the
 // captured one matches); returns the device milliseconds of the launch.
 double run_batch(pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c)
@@ -1060,47 +1159,16 @@ double run_batch(pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c)
     int cluster = c.cluster;
     int grid = persistent_grid(rs.mixed, c.threads, cluster);
     need(grid > 0, PFG_E_UNSUPPORTED, "batched kernel configuration cannot be resident on this GPU");
-    // Team sizes.  The n_team largest systems get a whole cluster; a system that would
-    // keep its team busy for more than kLongJob of the balanced time (all costs over
-    // all CTAs) gets the next larger team, since one long system bounds the whole solve
-    // otherwise: 256 uneven slabs in pairs and single CTAs are 125 ms of work per SM and
-    // took 220 ms, the longest pair's time; now 178.  A limit of 0.5, 0.7, 0.85, 1.0 and
-    // 1.15 gave 181, 179, 181, 174 and 162 ms there and 179, 198, 203, 203 and 203 in
-    // clusters of four; the low one also does best while the costs are guessed (the
-    // first solve, 291 -> 238 ms).  Clusters of four fill 144 of the 152 SMs, of eight
-    // 120, so pairs grow to fours, only if the longest needs it, and fours don't grow.
-    // A team's CTAs keep at least a slice for each quarter of the SM (FP64) or each of
-    // sixteen warps (mixed, where the barriers weigh more: 37 slices on 1, 2 and 4 CTAs
-    // 19.8, 15.8 and 11.8 us an iteration, in FP64 73.8, 44.5 and 26.0).
-    double total = 0.0;
-    for (int m = 0; m < count; ++m) total += cost[m];
-    if (n_team > 0 && cluster == 2 && cost[ord[0]] > kWiderCluster * 2 * total / grid) {
-        const int wider = persistent_grid(rs.mixed, c.threads, 4);
-        if (wider > 0) {
-            cluster = 4;
-            grid = wider;
-        }
-    }
-    int n_size[kTeamSizes] = {};
-    for (int k = 0; k < count && n_team > 0; ++k) {
-        const int m = ord[k];
-        int size = k < n_team ? c.cluster : 1;
-        while (size < cluster && cost[m] > kLongJob * size * total / grid &&
-               b->ndof[m] >= (int64_t)2 * size * (rs.mixed ? 16 : 4) * 96)
-            size *= 2;
-        // (never a larger team than a costlier system's: the order lists the sizes in turn)
-        if (k > 0) size = std::min(size, b->team[ord[k - 1]]);
-        b->team[m] = size;
-        if (size == 1) break;
-        for (int l = 0; l < kTeamSizes; ++l)
-            if (size == kMaxTeam >> l) ++n_size[l];
-    }
+    TeamPlan plan{cluster, grid, {}};
+    if (n_team > 0) plan = plan_teams(b, rs, c, ord, cost, n_team, grid);
+    cluster = plan.cluster;
+    grid = plan.grid;
 
     BatchParams P;
     P.mesh = b->meshes.p;
     P.out = b->out.p;
     P.order = b->order.p;
-    std::copy(n_size, n_size + kTeamSizes, P.n_team);
+    std::copy(plan.n, plan.n + kTeamSizes, P.n_team);
     P.n_total = count;
     P.cluster = cluster;
     P.queue = b->queue.p;
@@ -1116,7 +1184,7 @@ double run_batch(pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c)
 
     uint64_t key = 0x51ab;
     for (uint64_t v : {(uint64_t)rs.mixed, (uint64_t)rs.precond, (uint64_t)rs.itrmax, (uint64_t)c.threads,
-                       (uint64_t)cluster, (uint64_t)n_size[0], (uint64_t)n_size[1], (uint64_t)n_size[2], (uint64_t)count, (uint64_t)grid,
+                       (uint64_t)cluster, (uint64_t)plan.n[0], (uint64_t)plan.n[1], (uint64_t)plan.n[2], (uint64_t)count, (uint64_t)grid,
                        (uint64_t)(uintptr_t)b->meshes.p, (uint64_t)(uintptr_t)b->v64.p,
                        (uint64_t)(uintptr_t)b->abort_d, (uint64_t)(uintptr_t)b->force64_d.p})
         key = mix(key, v);
@@ -1225,7 +1293,6 @@ int pfg_batch_set(pfg_batch *b, int64_t count, pfg_solver *const *handles)
         b->ndof.resize((size_t)count);
         b->off.resize((size_t)count);
         b->work.resize((size_t)count);
-        b->team.assign((size_t)count, 1);
         b->last_iters.assign((size_t)count, 0);
         b->iters64.assign((size_t)count, 0);
         b->force64.assign((size_t)count, 0);
