@@ -2,14 +2,16 @@
 //
 // Restates bicgstab_CRS_2 (FEMSolverClass.f90:2199-2298) and adds CG for the
 // symmetric eliminated system.  Design:
+//   * a solve small enough for the SMs' shared memory runs as one cooperative launch
+//     (resident.cu); what follows is the kernel-by-kernel form of the larger ones;
 //   * every scalar (rho, alpha, beta, c1..c3, norms) lives in device memory
 //     (KState); the last CTA of each fused reduction computes the next scalars,
-//     so one iteration is 2 (CG) or 3 (BiCGSTAB) kernel launches and no host
+//     so one iteration is 3 (CG) or 5 (BiCGSTAB) kernel launches and no host
 //     round trip;
 //   * the direction update p = z + beta p (CG) or p = r + beta (p - c3 y)
-//     (BiCGSTAB) is fused into the SpMV that consumes p: the gathered source
-//     value of every block column is formed on the fly, the owning warp writes
-//     the row's new p to a ping-pong buffer;
+//     (BiCGSTAB) is its own pass, or (update_mode "fused") part of the SpMV that
+//     consumes p: the gathered source value of every block column is formed on the
+//     fly, the owning warp writes the row's new p to a ping-pong buffer;
 //   * a chunk of iterations is captured once into a CUDA graph and replayed;
 //     kernels return at entry once KState says done (or, mixed precision, that
 //     a residual replacement is due), and the host checks KState once per chunk;
