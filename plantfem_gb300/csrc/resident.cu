@@ -79,6 +79,20 @@ __device__ __forceinline__ void ld_entry(const double *p, double &a, double &b)
         asm volatile("ld.volatile.global.f64 %0, [%1];" : "=d"(a) : "l"(p) : "memory");
 }
 
+// Sum over a warp of one or two FP64 values; value k's total ends up in lane 16 k.  For
+// two the halves of the warp trade values first and then carry one each: 5 additions
+// instead of 10, each 64 cycles of the quarter SM's pipe.
+template <int NV>
+__device__ __forceinline__ double lanes_sum(const double (&v)[NV], int lane)
+{
+    if (NV == 1) return warp_sum(v[0]);
+    const bool upper = (lane & 16) != 0;
+    double t = (upper ? v[NV - 1] : v[0]) + __shfl_xor_sync(0xffffffffu, upper ? v[0] : v[NV - 1], 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
 enum Step { kGo, kDone, kReplace, kLost };
 
 // The scalars an iteration changes.
@@ -121,7 +135,8 @@ struct Grid {
     // empties its inbox of the buffer four rounds ahead, which it has read (it was
     // used four rounds ago) and which a published round orders before its next use
     // (no loop here goes four rounds without one).  False: a wait ran out.
-    template <int NV, bool PUBLISH, typename Mid, typename Fin>
+    // SUM false: a barrier only, without the 650 cycles of the additions.
+    template <int NV, bool PUBLISH, bool SUM = true, typename Mid, typename Fin>
     __device__ bool exchange(double (&v)[NV], const Mid &mid, const Fin &fin)
     {
         const unsigned buf = round % kResRounds;
@@ -169,49 +184,51 @@ struct Grid {
             if (PUBLISH) __threadfence();
             static_assert(U == 5, "the sum below takes five values per lane");
             double acc[NV];
+            if (SUM) {
 #pragma unroll
-            for (int k = 0; k < NV; ++k) acc[k] = warp_sum(((t[0][k] + t[1][k]) + (t[2][k] + t[3][k])) + t[4][k]);
+                for (int k = 0; k < NV; ++k) acc[k] = ((t[0][k] + t[1][k]) + (t[2][k] + t[3][k])) + t[4][k];
+                const double all = lanes_sum<NV>(acc, lane);
+#pragma unroll
+                for (int k = 0; k < NV; ++k) acc[k] = __shfl_sync(0xffffffffu, all, 16 * k);
+            }
             if (lane == 0) {
                 if (!ok) {
                     sh->fail = 1;
                     *(volatile int *)err = 1;
                 }
+                if (SUM) {
 #pragma unroll
-                for (int k = 0; k < NV; ++k) sh->tot[round & 1][k] = acc[k];
-                fin(acc);
+                    for (int k = 0; k < NV; ++k) sh->tot[round & 1][k] = acc[k];
+                    fin(acc);
+                }
             }
         }
         __syncthreads();
+        if (SUM)
 #pragma unroll
-        for (int k = 0; k < NV; ++k) v[k] = sh->tot[round & 1][k];
+            for (int k = 0; k < NV; ++k) v[k] = sh->tot[round & 1][k];
         ++round;
         return sh->fail == 0;
     }
 
     __device__ int active() const { return min(kNW, nsl); }  // warps that own rows
 
-    __device__ double lanes_sum(double v, int n) const  // of lanes 0 .. n - 1 (n <= 16), in lane 0
-    {
-        if (lane >= n) v = 0.0;
-        for (int o = 1; o < n; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        return __shfl_sync(0xffffffffu, v, 0);
-    }
-
     template <int NV, bool PUBLISH, typename Mid, typename Fin>
     __device__ bool sum(double (&v)[NV], const Mid &mid, const Fin &fin)
     {
         const int act = active();
         if (wid < act) {
-#pragma unroll
-            for (int k = 0; k < NV; ++k) {
-                v[k] = warp_sum(v[k]);
-                if (lane == 0) sh->red[k][wid] = v[k];
-            }
+            const double t = lanes_sum<NV>(v, lane);
+            if (NV == 1 ? lane == 0 : (lane & 15) == 0) sh->red[lane >> 4][wid] = t;
         }
         __syncthreads();
-        if (wid == 0)
+        if (wid == 0) {
+            // lane 16 k + w: value k of warp w
+            double t = (lane & 15) < act && lane < 16 * NV ? sh->red[NV == 1 ? 0 : lane >> 4][lane & 15] : 0.0;
+            for (int o = 1; o < act; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
 #pragma unroll
-            for (int k = 0; k < NV; ++k) v[k] = lanes_sum(sh->red[k][lane & (kNW - 1)], act);
+            for (int k = 0; k < NV; ++k) v[k] = __shfl_sync(0xffffffffu, t, 16 * k);
+        }
         return exchange<NV, PUBLISH>(v, mid, fin);
     }
 
@@ -254,7 +271,7 @@ struct Grid {
     {
         double v[1] = {0.0};
         __syncthreads();
-        return exchange<1, true>(v, [] {}, [](double(&)[1]) {});
+        return exchange<1, true, false>(v, [] {}, [](double(&)[1]) {});
     }
 };
 
