@@ -591,7 +591,7 @@ struct DFAcc {
 // both.  The pipe does no more of them per clock than of the scalar forms (measured
 // 128 values per clock and SM either way), but in half the issue slots and fewer
 // registers: linear combinations 996 -> 852 us at 398k rows and 24 columns, 78 -> 56
-// at 95k and 12 (where the half panel counts too), the Gram matrices 104 -> 94 there
+// at 70k and 12 (where the half panel counts too), the Gram matrices 104 -> 94 there
 // and 1,195 -> 1,177 at the larger size (pipe-bound at 12 operations a multiply-add).
 using F2 = unsigned long long;
 __device__ __forceinline__ F2 f2_pack(float a, float b)
@@ -841,7 +841,7 @@ __global__ void __launch_bounds__(kT) k_spmm_df(SellView<double> A, const float2
 // The products with kParts<T> warps per (slice, panel), each with a run of the
 // slice's slots, the parts added in order: for systems whose slices and panels alone
 // do not fill the GPU with warps.  A warp's slots are a chain of dependent loads (column,
-// then three panel rows), 27 of them in a hex mesh: 49 us per launch at 31,775 rows
+// then three panel rows), 27 of them in a hex mesh: 49 us per launch at 23,247 block rows
 // and two panels, whatever the bytes.  PAIR (FP32, K and M of one pattern): both
 // products in one pass, so the columns and the panel rows, most of the traffic, are
 // read once.  Measured there: K X and M X 94 -> 30 us (FP32; two parts 35, eight 42), one
@@ -1066,7 +1066,7 @@ __global__ void __launch_bounds__(kT)
 }
 
 // Rows staged in shared memory per step.  16, 32, 48 and 64 rows took 34, 29, 27 and
-// 27 us (FP32) and 90, 94, 85 and 105 us (double-float) at 95k rows and 12 columns, and
+// 27 us (FP32) and 90, 94, 85 and 105 us (double-float) at 70k rows and 12 columns, and
 // 356, 256, 228, 210 and 1,302, 1,177, 1,167, 1,160 us at 398k and 24.
 constexpr int kGramRows = 48;
 constexpr int kGramSub = 4;    // each thread owns a 4 x 4 sub-tile of both Gram matrices
@@ -1388,7 +1388,7 @@ __global__ void __launch_bounds__(kT)
 // sums are FP64 (no FP32 underflow of squares for badly scaled systems); what bounds
 // a small system is adding them across the CTA on the FP64 pipe, so the 16 sums
 // are halved from lane to lane (16 additions per warp instead of 80) and FP32
-// maxima stay FP32, and a thread takes two rows or more: 56 -> 14 us at 95k rows, k = 12.
+// maxima stay FP32, and a thread takes two rows or more: 56 -> 14 us at 70k rows, k = 12.
 // double-float panels: the difference on the FP32 pipe (lam split once per
 // column), the sums of the leading floats (seven digits are all a norm needs).
 __device__ __forceinline__ float res_lam(float, double l) { return (float)l; }
@@ -1797,7 +1797,7 @@ void gram(Ctx &c, int nblk, const Blocks<T> &B, std::vector<double> &GA, std::ve
     auto kern = k_gram<T>;
     PFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // about 20 warps per SM: two CTAs of ten at k = 24, seven of three at k = 12 (two of
-    // three left the pipes to latency: 58 us at 95k rows, now 27), a staged step each
+    // three left the pipes to latency: 58 us at 70k rows, now 27), a staged step each
     int occ = 0;
     PFG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
     const int per_sm = std::max(1, std::min(std::max(2, 20 * 32 / threads), occ));
