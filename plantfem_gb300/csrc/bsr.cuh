@@ -73,6 +73,10 @@ __device__ __forceinline__ void bsr_row_product(const BsrView<T> &A, int64_t row
 // (launch durations): FP64 CG product, 681k unknowns, 760 CTAs, 141 -> 116 us; FP64
 // CG update there 26.7 -> 23.6 us; BiCGSTAB product, 27.8k unknowns, 63.7 -> 48.5 us;
 // FP32 CG update, 3.09M unknowns, 30.6 -> 29.3 us.
+// WIDE false (the sliced products): one warp reads them.  Behind a loop that lives on
+// its loads in flight the wide form makes the compiler give that loop fewer registers:
+// at 1.03M block rows the FP32 CG product took 280 us with it (40 registers) and 186
+// without (48), fused 254 and 200, the FP64 one 475 and 442.
 constexpr int kPartAhead = 4;
 
 struct GridTicket {
@@ -138,7 +142,7 @@ __device__ __forceinline__ void block_sum_comp(Comp32 (&v)[NV], float *smem /* >
 }
 
 // Returns true on thread 0 of the last CTA; totals[] then holds the grid sums.
-template <int NV>
+template <int NV, bool WIDE = true>
 __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, unsigned int *counter,
                                          double (&totals)[NV])
 {
@@ -155,30 +159,44 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, unsi
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    double acc[NV];
+    if constexpr (WIDE) {
+        double acc[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] = 0.0;
-    for (int b0 = threadIdx.x; b0 < (int)gridDim.x; b0 += kPartAhead * blockDim.x) {
-        double t[kPartAhead][NV];
+        for (int k = 0; k < NV; ++k) acc[k] = 0.0;
+        for (int b0 = threadIdx.x; b0 < (int)gridDim.x; b0 += kPartAhead * blockDim.x) {
+            double t[kPartAhead][NV];
 #pragma unroll
-        for (int u = 0; u < kPartAhead; ++u) {
-            const int b = b0 + u * blockDim.x;
+            for (int u = 0; u < kPartAhead; ++u) {
+                const int b = b0 + u * blockDim.x;
 #pragma unroll
-            for (int k = 0; k < NV; ++k) t[u][k] = b < (int)gridDim.x ? __ldcg(&partials[(int64_t)b * NV + k]) : 0.0;
+                for (int k = 0; k < NV; ++k) t[u][k] = b < (int)gridDim.x ? __ldcg(&partials[(int64_t)b * NV + k]) : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < kPartAhead; ++u)
+#pragma unroll
+                for (int k = 0; k < NV; ++k) acc[k] += t[u][k];
         }
+        block_sum<NV>(acc, smem);
 #pragma unroll
-        for (int u = 0; u < kPartAhead; ++u)
+        for (int k = 0; k < NV; ++k) totals[k] = acc[k];
+    } else {
+        if (threadIdx.x < 32) {
+            double acc[NV];
 #pragma unroll
-            for (int k = 0; k < NV; ++k) acc[k] += t[u][k];
+            for (int k = 0; k < NV; ++k) acc[k] = 0.0;
+#pragma unroll 4
+            for (int b = threadIdx.x; b < (int)gridDim.x; b += 32)
+#pragma unroll
+                for (int k = 0; k < NV; ++k) acc[k] += __ldcg(&partials[(int64_t)b * NV + k]);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) totals[k] = warp_sum(acc[k]);
+        }
     }
-    block_sum<NV>(acc, smem);
-#pragma unroll
-    for (int k = 0; k < NV; ++k) totals[k] = acc[k];
     if (threadIdx.x == 0) *counter = 0u;
     return threadIdx.x == 0;
 }
 
-template <int NV>
+template <int NV, bool WIDE = true>
 __device__ __forceinline__ bool grid_sum_comp(Comp32 (&v)[NV], float *partials, unsigned int *counter,
                                               float (&totals)[NV])
 {
@@ -198,27 +216,52 @@ __device__ __forceinline__ bool grid_sum_comp(Comp32 (&v)[NV], float *partials, 
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    Comp32 acc[NV];
+    if constexpr (WIDE) {
+        Comp32 acc[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] = Comp32{0.f, 0.f};
-    const float2 *part2 = reinterpret_cast<const float2 *>(partials);
-    for (int b0 = threadIdx.x; b0 < (int)gridDim.x; b0 += kPartAhead * blockDim.x) {
-        float2 t[kPartAhead][NV];
+        for (int k = 0; k < NV; ++k) acc[k] = Comp32{0.f, 0.f};
+        const float2 *part2 = reinterpret_cast<const float2 *>(partials);
+        for (int b0 = threadIdx.x; b0 < (int)gridDim.x; b0 += kPartAhead * blockDim.x) {
+            float2 t[kPartAhead][NV];
 #pragma unroll
-        for (int u = 0; u < kPartAhead; ++u) {
-            const int b = b0 + u * blockDim.x;
+            for (int u = 0; u < kPartAhead; ++u) {
+                const int b = b0 + u * blockDim.x;
 #pragma unroll
-            for (int k = 0; k < NV; ++k)
-                t[u][k] = b < (int)gridDim.x ? __ldcg(part2 + (int64_t)b * NV + k) : make_float2(0.f, 0.f);
+                for (int k = 0; k < NV; ++k)
+                    t[u][k] = b < (int)gridDim.x ? __ldcg(part2 + (int64_t)b * NV + k) : make_float2(0.f, 0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < kPartAhead; ++u)
+#pragma unroll
+                for (int k = 0; k < NV; ++k) comp_merge(acc[k], t[u][k].x, t[u][k].y);
         }
+        block_sum_comp<NV>(acc, smem);
 #pragma unroll
-        for (int u = 0; u < kPartAhead; ++u)
+        for (int k = 0; k < NV; ++k) totals[k] = acc[k].s + acc[k].c;
+    } else {
+        if (threadIdx.x < 32) {
+            Comp32 acc[NV];
 #pragma unroll
-            for (int k = 0; k < NV; ++k) comp_merge(acc[k], t[u][k].x, t[u][k].y);
+            for (int k = 0; k < NV; ++k) acc[k] = Comp32{0.f, 0.f};
+            for (int b = threadIdx.x; b < (int)gridDim.x; b += 32)
+#pragma unroll
+                for (int k = 0; k < NV; ++k) {
+                    const float2 t = make_float2(*((volatile float *)&partials[((int64_t)b * NV + k) * 2]),
+                                                  *((volatile float *)&partials[((int64_t)b * NV + k) * 2 + 1]));
+                    comp_merge(acc[k], t.x, t.y);
+                }
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    float s2 = __shfl_xor_sync(0xffffffffu, acc[k].s, o);
+                    float c2 = __shfl_xor_sync(0xffffffffu, acc[k].c, o);
+                    comp_merge(acc[k], s2, c2);
+                }
+                totals[k] = acc[k].s + acc[k].c;
+            }
+        }
     }
-    block_sum_comp<NV>(acc, smem);
-#pragma unroll
-    for (int k = 0; k < NV; ++k) totals[k] = acc[k].s + acc[k].c;
     if (threadIdx.x == 0) *counter = 0u;
     return threadIdx.x == 0;
 }

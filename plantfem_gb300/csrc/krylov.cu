@@ -104,17 +104,17 @@ struct Acc<float> {
     __device__ static void add(Comp32 &a, float x, float y) { comp_add_prod(a, x, y); }
 };
 
-template <int NV>
+template <int NV, bool WIDE = true>
 __device__ __forceinline__ bool grid_total(double (&v)[NV], double *pd, float *, unsigned *ticket,
                                            double (&tot)[NV])
 {
-    return grid_sum<NV>(v, pd, ticket, tot);
+    return grid_sum<NV, WIDE>(v, pd, ticket, tot);
 }
-template <int NV>
+template <int NV, bool WIDE = true>
 __device__ __forceinline__ bool grid_total(Comp32 (&v)[NV], double *, float *pf, unsigned *ticket,
                                            float (&tot)[NV])
 {
-    return grid_sum_comp<NV>(v, pf, ticket, tot);
+    return grid_sum_comp<NV, WIDE>(v, pf, ticket, tot);
 }
 
 __device__ __forceinline__ bool finite_d(double x) { return isfinite(x); }
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(kThreads)
         }
     }
     T tot[1];
-    if (grid_total<1>(acc, pd, pf, ticket, tot)) {
+    if (grid_total<1, false>(acc, pd, pf, ticket, tot)) {
         const double pq = (double)tot[0];
         if (!(pq > 0.0) || !finite_d(pq)) {
             S->status = PFG_E_BREAKDOWN;
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(kThreads)
         }
     }
     T tot[1];
-    if (grid_total<1>(acc, pd, pf, ticket, tot)) {
+    if (grid_total<1, false>(acc, pd, pf, ticket, tot)) {
         const double pq = (double)tot[0];
         if (!(pq > 0.0) || !finite_d(pq)) {
             S->status = PFG_E_BREAKDOWN;
@@ -688,7 +688,7 @@ __global__ void __launch_bounds__(kThreads)
         }
     }
     T tot[1];
-    if (grid_total<1>(acc, pd, pf, ticket, tot)) {
+    if (grid_total<1, false>(acc, pd, pf, ticket, tot)) {
         const double c2 = (double)tot[0];
         if (c2 == 0.0 || !finite_d(c2)) {
             bicg_breakdown(S, f64);
@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(kThreads)
         }
     }
     T tot[2];
-    if (grid_total<2>(acc, pd, pf, ticket, tot)) {
+    if (grid_total<2, false>(acc, pd, pf, ticket, tot)) {
         const double vv = (double)tot[1];
         if (vv == 0.0 || !finite_d(vv) || !finite_d((double)tot[0])) {
             bicg_breakdown(S, f64);
@@ -932,7 +932,7 @@ __global__ void __launch_bounds__(kThreads)
         }
     }
     T tot[1];
-    if (grid_total<1>(acc, pd, pf, ticket, tot)) {
+    if (grid_total<1, false>(acc, pd, pf, ticket, tot)) {
         const double c2 = (double)tot[0];
         if (c2 == 0.0 || !finite_d(c2)) {
             bicg_breakdown(S, f64);
@@ -974,7 +974,7 @@ __global__ void __launch_bounds__(kThreads)
         }
     }
     T tot[2];
-    if (grid_total<2>(acc, pd, pf, ticket, tot)) {
+    if (grid_total<2, false>(acc, pd, pf, ticket, tot)) {
         const double vv = (double)tot[1];
         if (vv == 0.0 || !finite_d(vv) || !finite_d((double)tot[0])) {
             bicg_breakdown(S, f64);
