@@ -70,13 +70,14 @@ __device__ __forceinline__ void bsr_row_product(const BsrView<T> &A, int64_t row
 // What bounds it is the chain of L2 round trips after the last CTA's arrival:
 // one warp reading up to 912 partials in turn took 18-29 dependent loads.  Every
 // thread loading its partials (kPartAhead at once) makes it one or two trips
-// (launch durations): FP64 CG product, 681k unknowns, 760 CTAs, 141 -> 116 us; FP64
-// CG update there 26.7 -> 23.6 us; BiCGSTAB product, 27.8k unknowns, 63.7 -> 48.5 us;
-// FP32 CG update, 3.09M unknowns, 30.6 -> 29.3 us.
-// WIDE false (the sliced products): one warp reads them.  Behind a loop that lives on
+// (launch durations): FP64 CG update, 681k unknowns, 760 CTAs, 26.7 -> 23.6 us; FP32 CG
+// update, 3.09M unknowns, 30.6 -> 29.3 us.
+// WIDE false (the sliced products): one warp reads them (FP64: four at once).  Behind a loop that lives on
 // its loads in flight the wide form makes the compiler give that loop fewer registers:
 // at 1.03M block rows the FP32 CG product took 280 us with it (40 registers) and 186
 // without (48), fused 254 and 200, the FP64 one 475 and 442.
+// BiCGSTAB's vector passes use it too (one order for all of its sums, which its
+// iteration count follows; a microsecond of the thousand an iteration takes there).
 constexpr int kPartAhead = 4;
 
 struct GridTicket {

@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(kThreads)
         Acc<T>::add(acc[1], r0[i], ri);
     }
     T tot[2];
-    if (grid_total<2>(acc, pd, pf, ticket, tot)) {
+    if (grid_total<2, false>(acc, pd, pf, ticket, tot)) {
         S->iter += 1;
         S->parity ^= 1;
         const double rr = (double)tot[0], c1n = (double)tot[1];
@@ -1005,7 +1005,7 @@ __global__ void __launch_bounds__(kThreads)
         Acc<T>::add(acc[2], r0i, r0i);
     }
     T tot[3];
-    if (grid_total<3>(acc, pd, pf, ticket, tot)) {
+    if (grid_total<3, false>(acc, pd, pf, ticket, tot)) {
         if (sizeof(T) == 8) {
             S->c1 = (double)tot[0];
             S->rr = (double)tot[1];
@@ -1634,7 +1634,7 @@ __global__ void __launch_bounds__(kThreads)
         }
     }
     float tot[2];
-    if (grid_total<2>(acc, pd, pf, ticket, tot)) {
+    if (grid_total<2, false>(acc, pd, pf, ticket, tot)) {
         S->xmax_bits = 0u;  // every CTA read it at its start
         if (mode == 1) {
             const double c2 = (double)tot[0];
