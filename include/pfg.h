@@ -447,6 +447,12 @@ int pfg_batch_tune(pfg_batch *b, const pfg_solve_opts *opts, pfg_batch_config *b
  * Setting it to 1 from any host thread makes every team retire its system with
  * PFG_E_ABORTED at its next check (every 64 iterations); the caller resets it. */
 int pfg_batch_abort_flag(pfg_batch *b, volatile int32_t **flag);
+/* Longest wait, in clock cycles of the SM, of the CTAs that solve a system together
+ * for one another (default 2^32, about two seconds; a whole cluster's CTAs use the
+ * hardware's barrier, which has none).  A system whose CTAs waited longer ends with
+ * PFG_E_INTERNAL, as does one that they had taken and not begun; the batch stays
+ * usable.  A negative limit has run out before the wait begins. */
+int pfg_batch_set_wait_limit(pfg_batch *b, int64_t cycles);
 
 /* ------------------------------------------------------------ instrumentation */
 /* No counterpart in the reference (it has only wall-clock timers, TimeClass.f90).

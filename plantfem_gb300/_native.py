@@ -149,6 +149,7 @@ SIGNATURES = {
     "pfg_batch_get_config": (C.c_int, [_P, C.POINTER(BatchConfig), C.POINTER(_i32)]),
     "pfg_batch_tune": (C.c_int, [_P, C.POINTER(SolveOpts), C.POINTER(BatchConfig), C.POINTER(_d)]),
     "pfg_batch_abort_flag": (C.c_int, [_P, C.POINTER(C.POINTER(_i32))]),
+    "pfg_batch_set_wait_limit": (C.c_int, [_P, _i64]),
 }
 
 _LIB = None

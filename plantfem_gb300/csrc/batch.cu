@@ -52,7 +52,9 @@ struct TeamShared {
     double wpart[2][32][4];           // per-warp partials (FP64), double-buffered
     float wpart32[2][32][4];          // per-warp compensated partials (s, c pairs), double-buffered
     uint64_t bar[kTeamSizes];         // mbarriers of teams smaller than the cluster, one per size
-    int lost;                         // a wait on one of them ran out
+    long long limit;                  // clock cycles after which a wait on one of them gives up
+    int lost;                         // a wait in one of this CTA's teams ran out (set from any of them, at any time)
+    int gone;                         // the CTA has taken note: written between its own barriers
     double scalar[2][4];              // what thread 0 made of a reduction's totals, for the whole CTA
     int job;
 };
@@ -65,41 +67,58 @@ struct Team {
     int level;         // mbarrier of this size
     unsigned parity;   // of the mbarrier's current phase
     int nred;          // reductions done on this job (alternates the double buffers)
+    // a barrier of this team gave up (the same in every thread of the CTA)
+    __device__ __forceinline__ bool gave_up(const TeamShared &sh) const { return size > 1 && !whole && sh.gone; }
 };
-
-constexpr long long kBarrierClocks = 1ll << 32;  // about two seconds, then a wait gives up
 
 // Barrier of the CTAs of a team, with release and acquire over the cluster: the
 // hardware's cluster barrier for a whole cluster; for a part of one an mbarrier in every
-// CTA's shared memory on which each CTA of the team arrives once.  A wait that runs out
-// marks the CTA lost: its solves end with an internal error.
-__device__ __forceinline__ void team_barrier(Team &tm, TeamShared &sh)
+// CTA's shared memory on which each CTA of the team arrives once and warp 0 waits.
+// False, in every thread of the CTA alike: a wait ran out, here or in another CTA of
+// the team.  The CTA then marks every CTA of the team lost and arrives on none of the
+// team's barriers again, so that no other CTA passes one without it: their waits end too
+// (the mark spares them the limit), and the job's record stays PFG_E_INTERNAL.  Nor does
+// it write into another CTA's slots: one that has passed its last barrier may still be
+// adding them.
+__device__ __forceinline__ bool team_barrier(Team &tm, TeamShared &sh)
 {
     if (tm.whole) {
         cg::this_cluster().sync();
-        return;
+        return true;
     }
-    __syncthreads();
+    if (__syncthreads_or(*(volatile int *)&sh.lost)) {
+        if (threadIdx.x == 0) sh.gone = 1;
+        __syncthreads();
+        return false;
+    }
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&sh.bar[tm.level]);
     if ((int)threadIdx.x < tm.size) {
         uint32_t remote;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(bar), "r"(tm.base + (int)threadIdx.x));
         asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
     }
-    uint32_t done = 0;
-    const long long t0 = clock64();
-    while (!done) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(tm.parity)
-            : "memory");
-        if (!done && (*(volatile int *)&sh.lost || clock64() - t0 > kBarrierClocks)) break;
+    uint32_t done = 1;
+    if (threadIdx.x < 32) {
+        done = 0;
+        const long long t0 = clock64(), limit = sh.limit;
+        while (!done && clock64() - t0 <= limit) {
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(done)
+                : "r"(bar), "r"(tm.parity)
+                : "memory");
+            if (!done && *(volatile int *)&sh.lost) break;
+        }
     }
-    if (!done) *(volatile int *)&sh.lost = 1;
     tm.parity ^= 1;
+    if (__syncthreads_and(done)) return true;
+    if ((int)threadIdx.x < tm.size)
+        *(volatile int *)cg::this_cluster().map_shared_rank(&sh.lost, tm.base + (int)threadIdx.x) = 1;
+    if (threadIdx.x == 0) sh.gone = 1;
+    __syncthreads();
+    return false;
 }
 
 __device__ __forceinline__ void team_sync(Team &tm, TeamShared &sh)
@@ -153,7 +172,7 @@ __device__ __forceinline__ int team_reduce(double (&v)[NV], Team &tm, TeamShared
     }
     if (tm.size > 1) {
         cg::cluster_group cl = cg::this_cluster();
-        if (wid == 0 && lane < tm.size) {
+        if (wid == 0 && lane < tm.size && !tm.gave_up(sh)) {
             double *dst = cl.map_shared_rank(&sh.slot[buf][tm.rank][0], tm.base + lane);
 #pragma unroll
             for (int k = 0; k < NV; ++k) dst[k] = v[k];
@@ -220,7 +239,7 @@ __device__ __forceinline__ void team_sum_comp(Comp32 (&v)[NV], float (&tot)[NV],
     }
     if (tm.size > 1) {
         cg::cluster_group cl = cg::this_cluster();
-        if (wid == 0 && lane < tm.size) {
+        if (wid == 0 && lane < tm.size && !tm.gave_up(sh)) {
             double *dst = cl.map_shared_rank(&sh.slot[buf][tm.rank][0], tm.base + lane);
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
@@ -229,6 +248,11 @@ __device__ __forceinline__ void team_sum_comp(Comp32 (&v)[NV], float (&tot)[NV],
             }
         }
         team_barrier(tm, sh);
+        if (tm.gave_up(sh)) {  // the same in every thread, as what follows from it has to be
+#pragma unroll
+            for (int k = 0; k < NV; ++k) tot[k] = __int_as_float(0x7fc00000);
+            return;
+        }
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             v[k].s = lane < tm.size ? (float)sh.slot[buf][lane][2 * k] : 0.f;
@@ -439,6 +463,7 @@ __device__ int cg64(const BatchParams &P, const BatchMesh &D, Team &tm, TeamShar
     const double tol_b = P.tol * sqrt(bb);
     int status = PFG_OK;
     rel = bb > 0.0 ? sqrt(a01[1] / bb) : 0.0;
+    if (tm.gave_up(sh)) return PFG_E_INTERNAL;
     if (sqrt(a01[1]) <= tol_b) return PFG_OK;
     for (;;) {
         if (it >= P.itrmax) {
@@ -468,7 +493,10 @@ __device__ int cg64(const BatchParams &P, const BatchMesh &D, Team &tm, TeamShar
         if (threadIdx.x == 0) {
             const bool ok = a2[1] == 0.0 && a2[0] > 0.0 && isfinite(a2[0]);
             sh.scalar[b2][0] = ok ? rho / a2[0] : 0.0;
-            sh.scalar[b2][1] = a2[1] != 0.0 ? (double)PFG_E_ABORTED : ok ? (double)PFG_OK : (double)PFG_E_BREAKDOWN;
+            sh.scalar[b2][1] = tm.gave_up(sh)         ? (double)PFG_E_INTERNAL
+                               : a2[1] != 0.0 ? (double)PFG_E_ABORTED
+                               : ok           ? (double)PFG_OK
+                                              : (double)PFG_E_BREAKDOWN;
         }
         __syncthreads();
         status = (int)sh.scalar[b2][1];
@@ -515,6 +543,10 @@ __device__ int cg64(const BatchParams &P, const BatchMesh &D, Team &tm, TeamShar
         double beta = sh.scalar[b4][0];
         const double state = sh.scalar[b4][2];
         rho = sh.scalar[b4][1];
+        if (tm.gave_up(sh)) {
+            status = PFG_E_INTERNAL;
+            break;
+        }
         if (state == 2.0) {
             status = PFG_E_NONFINITE;
             break;
@@ -523,6 +555,7 @@ __device__ int cg64(const BatchParams &P, const BatchMesh &D, Team &tm, TeamShar
             // recursive residual converged: confirm on the true residual
             const double rt = residual64(D, sp, tm, sh);
             rel = bb > 0.0 ? sqrt(rt / bb) : 0.0;
+            if (tm.gave_up(sh)) return PFG_E_INTERNAL;
             if (sqrt(rt) <= tol_b) return PFG_OK;
             if (restarts >= P.max_restarts) {
                 status = PFG_W_NOT_CONVERGED;
@@ -580,7 +613,7 @@ __device__ void finish_job(const BatchParams &P, int m, const BatchMesh &D, Team
     restore_fixed_rows(D, team_span(tm, blockDim.x / 32), D.A64.nb);
     if (tm.rank == 0 && threadIdx.x == 0) {
         BatchOut o;
-        o.status = sh.lost ? PFG_E_INTERNAL : status;
+        o.status = tm.gave_up(sh) ? PFG_E_INTERNAL : status;
         o.iterations = it;
         o.replacements = reps;
         o.team_size = tm.size;
@@ -638,7 +671,7 @@ __device__ void solve_mixed(const BatchParams &P, int m, Team &tm, TeamShared &s
     bool converged = sqrt(a2[0]) <= tol_b;
     bool restart = true;   // the first pass starts from p = z
     float rho = 0.f, rmax = 0.f, rmin = 0.f;
-    while (!converged) {
+    while (!converged && !tm.gave_up(sh)) {
         // (re)start from the FP64 residual: r32 = r64, z = M^-1 r, beta keeps p unless a restart
         {
             Comp32 c2[2] = {Comp32{0.f, 0.f}, Comp32{0.f, 0.f}};
@@ -780,6 +813,7 @@ __device__ void solve_mixed(const BatchParams &P, int m, Team &tm, TeamShared &s
         }
         team_sync(tm, sh);
         ++reps;
+        if (tm.gave_up(sh)) break;
         if (accepted) cur_rt = rt;
         rt = cur_rt;
         rel = bb > 0.0 ? sqrt(rt / bb) : 0.0;
@@ -829,7 +863,8 @@ __global__ void __launch_bounds__(NT, 1) k_batch_cg(const __grid_constant__ Batc
         cg::cluster_group cl = cg::this_cluster();
         const int me = (int)cl.block_rank();
         if (threadIdx.x == 0) {
-            sh.lost = 0;
+            sh.lost = sh.gone = 0;
+            sh.limit = P.wait_limit;
             for (int l = 0; l < kTeamSizes; ++l)
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(
                                  (uint32_t)__cvta_generic_to_shared(&sh.bar[l])),
@@ -843,18 +878,19 @@ __global__ void __launch_bounds__(NT, 1) k_batch_cg(const __grid_constant__ Batc
             const int size = kMaxTeam >> l;
             if (P.n_team[l] == 0) continue;
             Team tm{me % size, size, me / size * size, size == P.cluster, l, 0, 0};
+            // (a job that is taken by a team which then loses a CTA keeps the record
+            // that every job starts with, PFG_E_INTERNAL; a lost CTA takes none)
             for (;;) {
-                if (tm.rank == 0 && threadIdx.x == 0) sh.job = (int)atomicAdd(P.queue + l, 1u);
-                team_barrier(tm, sh);
+                if (tm.rank == 0 && threadIdx.x == 0)
+                    sh.job = *(volatile int *)&sh.lost ? P.n_team[l] : (int)atomicAdd(P.queue + l, 1u);
+                if (!team_barrier(tm, sh)) break;
                 const int job = *cl.map_shared_rank(&sh.job, tm.base);
-                team_barrier(tm, sh);  // every CTA has read the job before rank 0 overwrites it
-                if (job >= P.n_team[l] || *(volatile int *)&sh.lost) break;
+                // every CTA has read the job before rank 0 overwrites it
+                if (!team_barrier(tm, sh) || job >= P.n_team[l]) break;
                 tm.nred = 0;
                 solve_job<MIXED, NT>(P, P.order[first + job], tm, sh);
             }
         }
-    } else if (threadIdx.x == 0) {
-        sh.lost = 0;
     }
     // single-CTA phase
     int n_solo = P.n_total, solo0 = 0;
@@ -972,6 +1008,8 @@ struct pfg_batch {
     int dinv_kind = -1;               // preconditioner the inverses hold
     DevBuf<BatchMesh> meshes;
     DevBuf<BatchOut> out;
+    DevBuf<BatchOut> unsolved;        // what `out` holds until a system has been solved
+    long long wait_limit = 1ll << 32; // clock cycles (about two seconds)
     DevBuf<int> order;
     DevBuf<unsigned> queue;
     std::vector<double> work;         // matrix blocks of each system (work per iteration)
@@ -1178,6 +1216,7 @@ double run_batch(pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c)
     P.tol = rs.tol;
     P.delta = rs.delta;
     P.abort = b->abort_d;
+    P.wait_limit = b->wait_limit;
     P.force64 = rs.mixed ? b->force64_d.p : nullptr;
     if (rs.mixed)
         PFG_CUDA(cudaMemcpyAsync(b->force64_d.p, b->force64.data(), count, cudaMemcpyHostToDevice, b->st));
@@ -1186,7 +1225,8 @@ double run_batch(pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c)
     for (uint64_t v : {(uint64_t)rs.mixed, (uint64_t)rs.precond, (uint64_t)rs.itrmax, (uint64_t)c.threads,
                        (uint64_t)cluster, (uint64_t)plan.n[0], (uint64_t)plan.n[1], (uint64_t)plan.n[2], (uint64_t)count, (uint64_t)grid,
                        (uint64_t)(uintptr_t)b->meshes.p, (uint64_t)(uintptr_t)b->v64.p,
-                       (uint64_t)(uintptr_t)b->abort_d, (uint64_t)(uintptr_t)b->force64_d.p})
+                       (uint64_t)(uintptr_t)b->abort_d, (uint64_t)(uintptr_t)b->force64_d.p,
+                       (uint64_t)b->wait_limit})
         key = mix(key, v);
     uint64_t tb, db;
     memcpy(&tb, &rs.tol, 8);
@@ -1197,8 +1237,10 @@ double run_batch(pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c)
         b->graph = nullptr;
         cudaGraph_t g;
         PFG_CUDA(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
-        // x0 = 0 for every system, empty job queues, then the persistent kernel
+        // x0 = 0 and the record of an unsolved system for every system, empty job
+        // queues, then the persistent kernel
         cudaMemsetAsync(b->v64.p, 0, b->total * sizeof(double), b->st);
+        cudaMemcpyAsync(b->out.p, b->unsolved.p, count * sizeof(BatchOut), cudaMemcpyDeviceToDevice, b->st);
         cudaMemsetAsync(b->queue.p, 0, (kTeamSizes + 1) * sizeof(unsigned), b->st);
         cudaLaunchConfig_t lc;
         cudaLaunchAttribute attr;
@@ -1224,6 +1266,7 @@ double run_batch(pfg_batch *b, const RunSpec &rs, const pfg_batch_config &c)
     PFG_CUDA(cudaEventElapsedTime(&ms, b->e0, b->e1));
     for (int m = 0; m < count; ++m) {
         const BatchOut &o = b->out_h[m];
+        if (o.status == PFG_E_INTERNAL) continue;
         b->last_iters[m] = std::max(o.iterations, 1);
         if (!rs.mixed || o.fallback == 2) {
             if (o.status == PFG_OK) b->iters64[m] = o.iterations;
@@ -1337,9 +1380,14 @@ int pfg_batch_set(pfg_batch *b, int64_t count, pfg_solver *const *handles)
         }
         b->meshes.resize((size_t)count);
         b->out.resize((size_t)count);
+        b->unsolved.resize((size_t)count);
         b->order.resize((size_t)count);
         PFG_CUDA(cudaMemcpyAsync(b->meshes.p, hm.data(), count * sizeof(BatchMesh), cudaMemcpyHostToDevice, b->st));
-        PFG_CUDA(cudaMemsetAsync(b->out.p, 0, count * sizeof(BatchOut), b->st));
+        BatchOut none{};
+        none.status = PFG_E_INTERNAL;
+        none.rel_residual = 1.0;  // of x = 0
+        const std::vector<BatchOut> ho((size_t)count, none);
+        PFG_CUDA(cudaMemcpyAsync(b->unsolved.p, ho.data(), count * sizeof(BatchOut), cudaMemcpyHostToDevice, b->st));
         PFG_CUDA(cudaStreamSynchronize(b->st));
         if (b->graph) cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
@@ -1478,6 +1526,15 @@ int pfg_batch_tune(pfg_batch *b, const pfg_solve_opts *opts, pfg_batch_config *b
         b->tuned = true;
         if (best) *best = top;
         if (best_ms) *best_ms = top_ms;
+    });
+}
+
+int pfg_batch_set_wait_limit(pfg_batch *b, int64_t cycles)
+{
+    return guard([&] {
+        need(b != nullptr, PFG_E_ARG, "NULL batch");
+        std::lock_guard<std::mutex> lk(b->mu);
+        b->wait_limit = cycles;
     });
 }
 

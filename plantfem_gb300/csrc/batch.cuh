@@ -77,6 +77,7 @@ struct BatchParams {
     double tol;
     double delta;             // reliable-update threshold (mixed)
     const volatile int *abort;   // host-mapped abort flag (null: none)
+    long long wait_limit;        // longest wait at a barrier of a part of a cluster, clock cycles
     const uint8_t *force64;      // mixed: per system, 1 = solve in FP64 (learned from earlier solves)
 };
 
