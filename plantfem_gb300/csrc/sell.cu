@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(288)
 // two rows: assembly rounding leaves noise in entries that cancel to zero).
 // One warp per row i, three of its upper blocks at a time: the warp reads row j's
 // block columns (one load per 32) and votes for the slot of (j, i); then 27 lanes
-// compare the three blocks' entries.  Entries with the same bits -- all of an
+// compare the three blocks' entries.  Finite entries with the same bits -- all of an
 // assembled and eliminated matrix's -- need no arithmetic: nine FP64 comparisons
 // for every block kept GB300's FP64 pipe busy for most of the 950 us this took at
 // 274,625 rows (4,032 rows: 297 us); now 425 us and 11 us.
@@ -276,7 +276,9 @@ __global__ void k_sym_check(int64_t nb, const int64_t *__restrict__ rp, const in
                     a = v64[ri * 9 + (int64_t)e3 * ni + k0 + at3];
                     b = v64[st3 * 9 + (int64_t)(3 * c3 + r3) * ln3 + sl3];
                 }
-                const bool differ = have && __double_as_longlong(a) != __double_as_longlong(b);
+                // (equal bits of an infinity or a NaN are no agreement)
+                const bool differ = have && (__double_as_longlong(a) != __double_as_longlong(b) ||
+                                             (__double2hiint(a) & 0x7ff00000) == 0x7ff00000);
                 if (__any_sync(0xffffffffu, differ)) {
                     const double di = diag_scale(i);
                     double dj = 0.0;
