@@ -275,7 +275,7 @@ __device__ __forceinline__ int64_t pc_at(int64_t row)
     return (row >> 5) * (32 * BS * BS) + (row & 31);
 }
 
-// SYM (a matrix found symmetric, whose blocks' inverses are): the entries on and above
+// SYM (symmetric diagonal blocks, whose inverses are): the entries on and above
 // the diagonal stand for both, 24 bytes of a row's 36 and of the 140 that the
 // symmetric CG's update moves: 26.1 -> 23.7 us at 1.03M block rows, 9.8 -> 9.3 at 275k.
 template <int BS, typename T, bool SYM = false>
@@ -553,7 +553,7 @@ __device__ __forceinline__ void cg_update_tail(typename Acc<T>::type (&acc)[2], 
 }
 
 // x += alpha p_new; r -= alpha q; z = M^-1 r; rho' = r.z; rr = r.r.
-template <int BS, typename T, int QS = BS>
+template <int BS, typename T, int QS = BS, bool SYM = false>
 __global__ void __launch_bounds__(kThreads)
     k_cg_update(int64_t nb, T *__restrict__ x, T *__restrict__ r, T *__restrict__ z, const T *pA, const T *pB,
                 T *__restrict__ q, const T *__restrict__ dinv, int pc, KState *S, double *pd, float *pf,
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
             for (int i = 0; i < 4; ++i) q[4 * row + i] = T(0);
         }
-        pc_apply<BS, T, QS == 4>(pc, dinv, row, rv, zv);
+        pc_apply<BS, T, SYM>(pc, dinv, row, rv, zv);
 #pragma unroll
         for (int i = 0; i < BS; ++i) {
             z[(int64_t)BS * row + i] = zv[i];
@@ -1919,7 +1919,7 @@ uint64_t Krylov::graph_key(int kind, const DevMatrix &A, const void *x, const KC
                     u(pA32_.p), u(pB32_.p), u(q32_.p), u(yA32_.p), u(yB32_.p), u(e32_.p), u(v32_.p), u(x32_.p),
                     u(dinv32_.p), u(ph_.p), u(eh_.p), u(ph32_.p), u(eh32_.p), u(partials_.p), u(partials32_.p), u(ticket_.p), u(state_.p),
                     (uint64_t)cfg.precond, (uint64_t)cfg.stop_rule, (uint64_t)cfg.graph_chunk, (uint64_t)cfg.itrmax,
-                    (uint64_t)cfg.fuse, (uint64_t)cfg.storage, u(y4_.p), u(fx_.p), u(A.sptr_u.p), u(A.scol_u.p),
+                    (uint64_t)cfg.fuse, (uint64_t)cfg.storage, (uint64_t)A.skew_diagonal, u(y4_.p), u(fx_.p), u(A.sptr_u.p), u(A.scol_u.p),
                     u(A.s32_u.p), d((double)A.sym_rowsum), d(cfg.relative_er), d(cfg.er0), d(cfg.reliable_delta),
                     ilu_ ? ilu_->generation() : 0, u(ilu_ ? ilu_->lu() : nullptr)});
 }
@@ -2030,23 +2030,23 @@ static int bicg_chunk_ilu(const SellView<double> &A, const Ilu0 &ilu, int chunk,
 
 // One chunk of FP32 CG iterations with the symmetric (upper-half) matrix:
 // dir, product into q4 with <p, Ap> and alpha, update (reads and clears q4).
-static int cg_chunk_sym(const SellView<float> &U, bool fuse, int chunk, int64_t nb, float *x, float *r, float *z,
-                        float *pA, float *pB, float *q4, const float *dinv, int pc, KState *S, double *pd, float *pf,
-                        unsigned *tk, double tol, double delta, int itrmax, cudaStream_t st)
+// skew: a diagonal block is unsymmetric (check_symmetric), so its whole inverse is read.
+static int cg_chunk_sym(const SellView<float> &U, bool skew, bool fuse, int chunk, int64_t nb, float *x, float *r,
+                        float *z, float *pA, float *pB, float *q4, const float *dinv, int pc, KState *S, double *pd,
+                        float *pf, unsigned *tk, double tol, double delta, int itrmax, cudaStream_t st)
 {
     const int64_t n = nb * 3;
     const int gd = resident_grid(k_cg_dir_sym, (n + 127) / 128);
-    const int gu = resident_grid(k_cg_update<3, float, 4>, (nb + 31) / 32);
+    const auto update = skew ? k_cg_update<3, float, 4, false> : k_cg_update<3, float, 4, true>;
+    const int gu = resident_grid(update, (nb + 31) / 32);
     for (int it = 0; it < chunk; ++it) {
         if (fuse) {  // direction update inside the product (ping-pong pA / pB)
             launch_cg_spmv_sym(true, U, z, pA, pB, q4, S, pd, pf, tk, st);
-            k_cg_update<3, float, 4><<<gu, kThreads, 0, st>>>(nb, x, r, z, pA, pB, q4, dinv, pc, S, pd, pf, tk, tol,
-                                                              delta, itrmax);
+            update<<<gu, kThreads, 0, st>>>(nb, x, r, z, pA, pB, q4, dinv, pc, S, pd, pf, tk, tol, delta, itrmax);
         } else {
             k_cg_dir_sym<<<gd, kThreads, 0, st>>>(n, z, pA, S);
             launch_cg_spmv_sym(false, U, nullptr, pA, nullptr, q4, S, pd, pf, tk, st);
-            k_cg_update<3, float, 4><<<gu, kThreads, 0, st>>>(nb, x, r, z, pA, pA, q4, dinv, pc, S, pd, pf, tk, tol,
-                                                              delta, itrmax);
+            update<<<gu, kThreads, 0, st>>>(nb, x, r, z, pA, pA, q4, dinv, pc, S, pd, pf, tk, tol, delta, itrmax);
         }
     }
     PFG_CUDA(cudaGetLastError());
@@ -2464,7 +2464,7 @@ SolveResult Krylov::run_mixed(DevMatrix &A, const double *b, double *x, const KC
             const bool fz = cfg.fuse != 0;
             const int ch = cfg.graph_chunk;
             if (sym && cg)
-                nk = cg_chunk_sym(sell_upper(A), fz, ch, A.nb, x32_.p, r32_.p, z32_.p, pA32_.p, pB32_.p, y4_.p,
+                nk = cg_chunk_sym(sell_upper(A), A.skew_diagonal, fz, ch, A.nb, x32_.p, r32_.p, z32_.p, pA32_.p, pB32_.p, y4_.p,
                                   dinv32_.p,
                                   cfg.precond, state_.p, partials_.p, partials32_.p, ticket_.p, cfg.relative_er,
                                   cfg.reliable_delta, cfg.itrmax, st);

@@ -81,7 +81,8 @@ struct DevMatrix {
     DevBuf<int> scol_u;
     DevBuf<float> s32_u;
     bool sell_u_pattern = false, s32_u_valid = false;
-    bool sym_checked = false;  // the values were found symmetric (check_symmetric)
+    bool sym_checked = false;  // the off-diagonal blocks were found symmetric (check_symmetric)
+    bool skew_diagonal = false;  // a diagonal block was not
     bool sym_rowsum_valid = false;
     float sym_rowsum = 0.f;  // max over scalar rows of sum |a_ij| (FP32; bound_rows)
 
@@ -131,8 +132,9 @@ inline SellView<float> DevMatrix::sell<float>() const { return SellView<float>{n
 // values when stale.  Implemented in sell.cu.
 void build_sell(DevMatrix &A, bool want64, bool want32, cudaStream_t st);
 
-// Checks once per value change that a 3x3-block matrix is symmetric (blockwise,
-// to 1e-9 relative) and throws PFG_E_ARG if it is not.  Implemented in sell.cu.
+// Checks once per value change that a 3x3-block matrix is symmetric (its off-diagonal
+// blocks, to 1e-9 relative), throws PFG_E_ARG if it is not and notes whether a diagonal
+// block is not.  Implemented in sell.cu.
 void check_symmetric(DevMatrix &A, cudaStream_t st);
 
 // A.sym_rowsum, once per value change (the fixed-point product's bound).

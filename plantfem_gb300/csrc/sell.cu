@@ -214,8 +214,11 @@ __global__ void __launch_bounds__(288)
 // assembled and eliminated matrix's -- need no arithmetic: nine FP64 comparisons
 // for every block kept GB300's FP64 pipe busy for most of the 950 us this took at
 // 274,625 rows (4,032 rows: 297 us); now 425 us and 11 us.
+// A diagonal block is no pair and may be anything: *skew is raised where one is not
+// symmetric itself, by the same measure.
 __global__ void k_sym_check(int64_t nb, const int64_t *__restrict__ rp, const int *__restrict__ bcol,
-                            const double *__restrict__ v64, unsigned long long *__restrict__ bad)
+                            const double *__restrict__ v64, unsigned long long *__restrict__ bad,
+                            unsigned long long *__restrict__ skew)
 {
     const int lane = threadIdx.x & 31;
     const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -240,6 +243,18 @@ __global__ void k_sym_check(int64_t nb, const int64_t *__restrict__ rp, const in
         unsigned long long nbad = 0;
         for (int k0 = 0; k0 < ni; k0 += 32) {
             const int mine = k0 + lane < ni ? bcol[ri + k0 + lane] : -1;
+            if (mine == i) {
+                const double *v = v64 + ri * 9 + k0 + lane;
+                const int up[3] = {1, 2, 5}, low[3] = {3, 6, 7};
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                    const double a = v[(int64_t)up[u] * ni], b = v[(int64_t)low[u] * ni];
+                    if (__double_as_longlong(a) == __double_as_longlong(b)) continue;
+                    double d = 0.0;
+                    for (int e = 0; e < 9; e += 4) d = fmax(d, fabs(v[(int64_t)e * ni]));
+                    if (!(fabs(a - b) <= 1e-9 * fmax(fabs(a), fabs(b)) + 1e-12 * d)) *skew = 1ull;
+                }
+            }
             unsigned todo = __ballot_sync(0xffffffffu, mine > i);
             while (todo) {
                 int at[3], to[3], slot[3], len[3];
@@ -327,16 +342,18 @@ void check_symmetric(DevMatrix &A, cudaStream_t st)
     PFG_CHECK(A.bs == 3, PFG_E_UNSUPPORTED, "symmetric storage is built for 3x3-block matrices");
     if (A.sym_checked) return;
     // the values (pattern included) changed: check the symmetry once
-    DevBuf<unsigned long long> bad(1);
-    PFG_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(unsigned long long), st));
-    k_sym_check<<<grid_for(A.nb, 8, sm_count_device() * 16), 256, 0, st>>>(A.nb, A.rp.p, A.col.p, A.v64.p, bad.p);
+    DevBuf<unsigned long long> bad(2);  // pairs that differ; whether a diagonal block does
+    PFG_CUDA(cudaMemsetAsync(bad.p, 0, 2 * sizeof(unsigned long long), st));
+    k_sym_check<<<grid_for(A.nb, 8, sm_count_device() * 16), 256, 0, st>>>(A.nb, A.rp.p, A.col.p, A.v64.p, bad.p,
+                                                                           bad.p + 1);
     PFG_CUDA(cudaGetLastError());
-    unsigned long long nbad = 0;
-    PFG_CUDA(cudaMemcpyAsync(&nbad, bad.p, sizeof nbad, cudaMemcpyDeviceToHost, st));
+    unsigned long long found[2] = {0, 0};
+    PFG_CUDA(cudaMemcpyAsync(found, bad.p, sizeof found, cudaMemcpyDeviceToHost, st));
     PFG_CUDA(cudaStreamSynchronize(st));
-    PFG_CHECK(nbad == 0, PFG_E_ARG,
-              "symmetric storage needs a symmetric matrix: " + std::to_string(nbad) +
+    PFG_CHECK(found[0] == 0, PFG_E_ARG,
+              "symmetric storage needs a symmetric matrix: " + std::to_string(found[0]) +
                   " blocks differ from their transposes");
+    A.skew_diagonal = found[1] != 0;
     A.sym_checked = true;
 }
 
