@@ -2253,12 +2253,15 @@ SolveResult Krylov::run_resident(DevMatrix &A, const double *b, double *x, const
     res.replacements = h.replacements;
     res.rel_residual = h.rel;
     res.fallback = h.fallback;
-    if (cfg.stop_rule == PFG_STOP_REFERENCE && cfg.algorithm == PFG_ALG_BICGSTAB && !mixed)
+    // (only FP64 BiCGSTAB ends by the reference's rule; CG and mixed solves always
+    // mean the true residual)
+    const bool by_reference =
+        cfg.stop_rule == PFG_STOP_REFERENCE && cfg.algorithm == PFG_ALG_BICGSTAB && !mixed;
+    if (by_reference)
         res.iter_residual = h.iter > 0 ? sqrt(h.rr / (h.rr1 > 0 ? h.rr1 : 1.0)) : 0.0;
     else if (mixed || h.iter > 0)
         res.iter_residual = sqrt(h.rr / (h.bb > 0 ? h.bb : 1.0));
-    if (!res.fallback && res.status == PFG_OK && cfg.stop_rule == PFG_STOP_TRUE_RELATIVE &&
-        res.rel_residual > cfg.relative_er)
+    if (!res.fallback && res.status == PFG_OK && !by_reference && res.rel_residual > cfg.relative_er)
         res.status = PFG_W_NOT_CONVERGED;
     return res;
 }

@@ -75,3 +75,17 @@ def test_symmetric_storage_with_unsymmetric_diagonal_blocks(cuda, update_mode):
         got[storage] = (s.last_info["iterations"], s.last_info["fallback"])
     assert got["symmetric"][1] == got["full"][1] == 0, got
     assert abs(got["symmetric"][0] - got["full"][0]) <= 5, got
+
+
+@pytest.mark.parametrize("algorithm,precision", [("CG", "fp64"), ("CG", "mixed"), ("BiCGSTAB", "mixed")])
+def test_unreachable_tolerance_is_reported(cuda, algorithm, precision):
+    """Below FP64's reach (1e-18): CG and the mixed solves end with the warning whatever
+    the stop rule, which is FP64 BiCGSTAB's alone."""
+    s = _solver(problems.cube(4))
+    s.relative_er = 1e-18
+    s.itrmax = 3000
+    for stop_rule in ("reference", "true_relative"):
+        for update_mode in (0, "separate"):
+            s.solve(algorithm=algorithm, precision=precision, stop_rule=stop_rule, preconditioning="BlockJacobi",
+                    update_mode=update_mode)
+            assert s.last_info["status"] == N.PFG_W_NOT_CONVERGED, (stop_rule, update_mode, s.last_info)
