@@ -98,8 +98,10 @@ enum Step { kGo, kDone, kReplace, kLost };
 // The scalars an iteration changes.
 struct Live {
     double beta, rho, inv_rho, alpha, c2, c3, rr;  // rho: <r, z> (CG) or c1 = <r0, r> (BiCGSTAB)
-    double goal, goal1;                            // squared: tol^2 <b, b>, and tol^2 rr1 (reference stop rule)
-    double rr1, er0;
+    double reach;                                  // tol |b|
+    double goal, goal1, near0;                     // squared: reach, and tol sqrt(rr1) and er0 (reference stop rule)
+    double rr1;
+    int exact;                                     // a square is no measure: negative, or lost to underflow
     float beta32, alpha32, c3_32;                  // what the FP32 row passes read
     float rmax, rmin;
     int iter, parity, status, breakdowns, poisoned, next;
@@ -639,6 +641,22 @@ struct Solve {
 // (integer test: an FP64 comparison costs 65 cycles)
 __device__ __forceinline__ bool finite(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 
+// Whether the square of a limit can stand for it: a division or square root takes
+// 660 cycles of an iteration's serial part, a comparison 65.
+__device__ __forceinline__ bool square_holds(double limit, double square)
+{
+    return limit == 0.0 || (limit > 0.0 && square > 1e-280);
+}
+
+// FP64: the stop test on the recursive residual (reference rule: FEMSolverClass.f90:2275-2289)
+template <bool REFERENCE>
+__device__ __forceinline__ bool reached(const Live &v, const ResArgs &a, double rr)
+{
+    if (v.exact)
+        return REFERENCE ? sqrt(rr / v.rr1) < a.tol || sqrt(rr) < a.er0 : sqrt(rr) <= v.reach;
+    return REFERENCE ? rr < v.goal1 || rr < v.near0 : rr <= v.goal;
+}
+
 // FP32: what an iteration's end asks for (replace on progress, at the tolerance,
 // or when the recursion diverged)
 __device__ __forceinline__ bool replace_due(Live &v, const ResArgs &a, double rr)
@@ -646,7 +664,7 @@ __device__ __forceinline__ bool replace_due(Live &v, const ResArgs &a, double rr
     const float rn = sqrtf((float)rr);
     v.rmax = fmaxf(v.rmax, rn);
     v.rmin = fminf(v.rmin, rn);
-    return rn < (float)a.delta * v.rmax || (double)rn * (double)rn <= v.goal || rn > 1000.f * v.rmin;
+    return rn < (float)a.delta * v.rmax || (double)rn <= v.reach || rn > 1000.f * v.rmin;
 }
 
 // One CG iteration.  FP64: p is published, three exchanges.  FP32: z and the
@@ -752,7 +770,7 @@ __device__ Step cg_step(Solve<BS, T> &S, const ResArgs &a, T *xs, T *rs, T *ps, 
             if (f64) {
                 v.beta = rho * v.inv_rho;
                 v.rho = rho;
-                if (rr <= v.goal) v.next = kDone;
+                if (reached<false>(v, a, rr)) v.next = kDone;
             } else if (replace_due(v, a, rr)) {
                 v.next = kReplace;
             } else {
@@ -922,10 +940,10 @@ __device__ Step bicg_step(Solve<BS, T> &S, const ResArgs &a, T *xs, T *rs, T *r0
                 if (v.iter == 1) {
                     v.rr1 = rr;
                     v.goal1 = a.tol * a.tol * rr;
+                    if (a.stop_rule == PFG_STOP_REFERENCE) v.exact |= !square_holds(a.tol, v.goal1);
                 }
-                const bool stop =
-                    a.stop_rule == PFG_STOP_REFERENCE ? (rr < v.goal1 || rr < v.er0) : rr <= v.goal;
-                if (stop) v.next = kDone;
+                if (a.stop_rule == PFG_STOP_REFERENCE ? reached<true>(v, a, rr) : reached<false>(v, a, rr))
+                    v.next = kDone;
             } else if (replace_due(v, a, rr)) {
                 v.next = kReplace;
             }
@@ -1088,7 +1106,7 @@ __device__ void open_solve(Solve<BS, T> &S, Share &h, T *buf, int64_t nb)
 }
 
 // ResState <-> Live, by one thread
-__device__ void set_live(ResShared &sh, const ResArgs &a)
+__device__ void set_live(ResShared &sh, const ResArgs &a, bool by_reference)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1099,10 +1117,13 @@ __device__ void set_live(ResShared &sh, const ResArgs &a)
         v.c2 = s.c2;
         v.c3 = s.c3;
         v.rr = s.rr;
+        v.reach = a.tol * sqrt(s.bb);
         v.goal = a.tol * a.tol * s.bb;
         v.rr1 = s.rr1;
         v.goal1 = a.tol * a.tol * s.rr1;
-        v.er0 = a.er0 * a.er0;
+        v.near0 = a.er0 * a.er0;
+        v.exact = by_reference ? !square_holds(a.er0, v.near0) || (s.iter > 0 && !square_holds(a.tol, v.goal1))
+                               : !square_holds(a.tol, v.goal);
         v.beta32 = (float)s.beta;
         v.c3_32 = (float)s.c3;
         v.rmax = s.rmax32;
@@ -1261,7 +1282,7 @@ __device__ void solve64(Solve<BS, double> &S, ResShared &sh, const ResArgs &a, u
             put_state(sh, s);
         }
         resumed = false;
-        set_live(sh, a);
+        set_live(sh, a, !CG && a.stop_rule == PFG_STOP_REFERENCE);
         Step st = kGo;
         while (st == kGo && left > 0) {
             st = CG ? cg_step(S, a, xs, rs, ps, (double *)nullptr, a.pub64[0], (double *)nullptr, (double *)nullptr,
@@ -1456,7 +1477,7 @@ __device__ void solve_mixed(Solve<BS, float> &S, Solve<BS, double> &D, const Cut
             if (conv || s.fallback) break;
         }
         resumed = false;
-        set_live(sh, a);
+        set_live(sh, a, false);
         Step st = kGo;
         while (st == kGo && left > 0) {
             st = CG ? cg_step(S, a, xs, rs, ps, zs, (float *)nullptr, a.pub32[0], a.pub32[1], a.pub32[2])

@@ -89,3 +89,19 @@ def test_unreachable_tolerance_is_reported(cuda, algorithm, precision):
             s.solve(algorithm=algorithm, precision=precision, stop_rule=stop_rule, preconditioning="BlockJacobi",
                     update_mode=update_mode)
             assert s.last_info["status"] == N.PFG_W_NOT_CONVERGED, (stop_rule, update_mode, s.last_info)
+
+
+@pytest.mark.parametrize("er0,relative_er", [(-1.0, 1e-8), (-1e300, 1e-8), (0.0, 1e-8), (1e-200, 1e-8),
+                                             (1e-9, -1.0), (1e-9, 1e-200), (1e-9, 0.0), (1e200, 1e-8)])
+def test_limits_that_no_square_stands_for(cuda, er0, relative_er):
+    """The reference stop rule compares sqrt(rr / rr1) and sqrt(rr) with its limits: a
+    negative one never holds (er0 = -1 leaves the relative test alone), a tiny one does
+    once the residual is as small."""
+    s = _solver(problems.cube(4))
+    s.er0, s.relative_er = er0, relative_er
+    s.solve()
+    res = dict(s.last_info)
+    s.solve(update_mode="separate")
+    sep = s.last_info
+    assert res["status"] == sep["status"] == 0
+    assert abs(res["iterations"] - sep["iterations"]) <= 3, (res, sep)
