@@ -641,6 +641,14 @@ struct Solve {
 // (integer test: an FP64 comparison costs 65 cycles)
 __device__ __forceinline__ bool finite(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 
+// a / b by way of the reciprocal that was formed meanwhile, unless that is out of range (b of
+// a right-hand side of 1e-153, say)
+__device__ __forceinline__ double quotient(double a, double b, double inv_b)
+{
+    const int e = __double2hiint(inv_b) & 0x7ff00000;
+    return e != 0 && e != 0x7ff00000 ? a * inv_b : a / b;
+}
+
 // Whether the square of a limit can stand for it: a division or square root takes
 // 660 cycles of an iteration's serial part, a comparison 65.
 __device__ __forceinline__ bool square_holds(double limit, double square)
@@ -768,7 +776,7 @@ __device__ Step cg_step(Solve<BS, T> &S, const ResArgs &a, T *xs, T *rs, T *ps, 
             }
             v.rr = rr;
             if (f64) {
-                v.beta = rho * v.inv_rho;
+                v.beta = quotient(rho, v.rho, v.inv_rho);
                 v.rho = rho;
                 if (reached<false>(v, a, rr)) v.next = kDone;
             } else if (replace_due(v, a, rr)) {
@@ -952,7 +960,7 @@ __device__ Step bicg_step(Solve<BS, T> &S, const ResArgs &a, T *xs, T *rs, T *r0
                     if (v.c2 * v.c3 == 0.0) {
                         breakdown();
                     } else {
-                        v.beta = c1 * v.inv_rho;
+                        v.beta = quotient(c1, v.c2 * v.c3, v.inv_rho);
                         v.rho = c1;
                     }
                 } else {

@@ -105,3 +105,23 @@ def test_limits_that_no_square_stands_for(cuda, er0, relative_er):
     sep = s.last_info
     assert res["status"] == sep["status"] == 0
     assert abs(res["iterations"] - sep["iterations"]) <= 3, (res, sep)
+
+
+@pytest.mark.parametrize("scale", [1e-140, 1e-152, 1e-154, 1e-155, 1e150])
+@pytest.mark.parametrize("algorithm", ["CG", "BiCGSTAB"])
+def test_right_hand_sides_of_extreme_scale(cuda, algorithm, scale):
+    """FP64 solves of K x = scale b to 1e-4: <r, z> down to 1e-312, whose reciprocal is
+    out of range, and up to 1e302.  Scaling by a power of two changes no bit until
+    numbers become subnormal; those still hold more digits than the tolerance."""
+    p = problems.cube(4)
+    p["E"] = np.ones_like(p["E"])
+    p["rhs"] = p["rhs"] * scale
+    s = _solver(p)
+    s.relative_er = 1e-4
+    kw = dict(algorithm=algorithm, stop_rule="true_relative", preconditioning="BlockJacobi")
+    s.solve(**kw)
+    res = dict(s.last_info)
+    s.solve(update_mode="separate", **kw)
+    sep = s.last_info
+    assert res["status"] == sep["status"] == 0 and res["rel_residual"] <= 1e-4, (res, sep)
+    assert abs(res["iterations"] - sep["iterations"]) <= 2, (res, sep)
