@@ -98,9 +98,8 @@ enum Step { kGo, kDone, kReplace, kLost };
 // The scalars an iteration changes.
 struct Live {
     double beta, rho, inv_rho, alpha, c2, c3, rr;  // rho: <r, z> (CG) or c1 = <r0, r> (BiCGSTAB)
-    double reach;                                  // tol |b|
-    double goal, goal1, near0;                     // squared: reach, and tol sqrt(rr1) and er0 (reference stop rule)
-    double rr1;
+    double goal, goal1, near0;                     // squared: tol |b|, and tol sqrt(rr1) and er0 (reference stop rule)
+    double bb, rr1;
     int exact;                                     // a square is no measure: negative, or lost to underflow
     float beta32, alpha32, c3_32;                  // what the FP32 row passes read
     float rmax, rmin;
@@ -661,7 +660,7 @@ template <bool REFERENCE>
 __device__ __forceinline__ bool reached(const Live &v, const ResArgs &a, double rr)
 {
     if (v.exact)
-        return REFERENCE ? sqrt(rr / v.rr1) < a.tol || sqrt(rr) < a.er0 : sqrt(rr) <= v.reach;
+        return REFERENCE ? sqrt(rr / v.rr1) < a.tol || sqrt(rr) < a.er0 : sqrt(rr) <= a.tol * sqrt(v.bb);
     return REFERENCE ? rr < v.goal1 || rr < v.near0 : rr <= v.goal;
 }
 
@@ -672,7 +671,7 @@ __device__ __forceinline__ bool replace_due(Live &v, const ResArgs &a, double rr
     const float rn = sqrtf((float)rr);
     v.rmax = fmaxf(v.rmax, rn);
     v.rmin = fminf(v.rmin, rn);
-    return rn < (float)a.delta * v.rmax || (double)rn <= v.reach || rn > 1000.f * v.rmin;
+    return rn < (float)a.delta * v.rmax || (double)rn * (double)rn <= v.goal || rn > 1000.f * v.rmin;
 }
 
 // One CG iteration.  FP64: p is published, three exchanges.  FP32: z and the
@@ -1125,8 +1124,8 @@ __device__ void set_live(ResShared &sh, const ResArgs &a, bool by_reference)
         v.c2 = s.c2;
         v.c3 = s.c3;
         v.rr = s.rr;
-        v.reach = a.tol * sqrt(s.bb);
-        v.goal = a.tol * a.tol * s.bb;
+        v.bb = s.bb;
+        v.goal = a.tol < 0.0 ? -1.0 : a.tol * a.tol * s.bb;
         v.rr1 = s.rr1;
         v.goal1 = a.tol * a.tol * s.rr1;
         v.near0 = a.er0 * a.er0;
