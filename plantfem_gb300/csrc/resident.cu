@@ -1602,6 +1602,37 @@ ResPlan plan_resident(const DevMatrix &A, int algorithm, bool mixed, bool precon
     return pl;
 }
 
+namespace {
+
+// One grid whose CTAs wait for one another at a time on a device (each fills it: two that
+// held half the SMs each would wait until their limits).  The order is made on the device,
+// launch by launch: a launch waits in its stream for the end of the one before, whichever
+// thread's that was, and no thread waits for another solve on the host.  Several threads'
+// solves so alternate after at most one launch each (4,096 iterations), and those on
+// different devices do not meet.
+struct Turn {
+    std::mutex mu;
+    cudaEvent_t last = nullptr;
+};
+
+void launch_in_turn(const void *kern, dim3 grid, void **args, size_t smem, cudaStream_t st)
+{
+    static Turn turns[64];
+    int dev = 0;
+    PFG_CUDA(cudaGetDevice(&dev));
+    PFG_CHECK(dev >= 0 && dev < 64, PFG_E_UNSUPPORTED, "device ordinal above 63");
+    Turn &t = turns[dev];
+    std::lock_guard<std::mutex> lk(t.mu);
+    if (t.last)
+        PFG_CUDA(cudaStreamWaitEvent(st, t.last, 0));
+    else
+        PFG_CUDA(cudaEventCreateWithFlags(&t.last, cudaEventDisableTiming));
+    PFG_CUDA(cudaLaunchCooperativeKernel(kern, grid, dim3(kNT), args, smem, st));
+    PFG_CUDA(cudaEventRecord(t.last, st));
+}
+
+}  // namespace
+
 int run_resident_kernel(const ResPlan &pl, ResArgs a, int bs, int algorithm, bool mixed, ResState *host,
                         cudaStream_t st)
 {
@@ -1610,14 +1641,9 @@ int run_resident_kernel(const ResPlan &pl, ResArgs a, int bs, int algorithm, boo
     a.stages = pl.stages;
     a.near = pl.near;
     void *args[] = {&a};
-    // One grid whose CTAs wait for one another at a time, whatever the thread and
-    // stream (each fills the device): two that held half the SMs each would wait
-    // until their limits.
-    static std::mutex one;
-    std::lock_guard<std::mutex> lk(one);
     PFG_CUDA(cudaMemcpyAsync(a.st, host, sizeof(ResState), cudaMemcpyHostToDevice, st));
     for (int launches = 1;; ++launches) {
-        PFG_CUDA(cudaLaunchCooperativeKernel((const void *)kern, dim3(pl.ctas), dim3(kNT), args, pl.smem, st));
+        launch_in_turn((const void *)kern, dim3(pl.ctas), args, pl.smem, st);
         PFG_CUDA(cudaMemcpyAsync(host, a.st, sizeof(ResState), cudaMemcpyDeviceToHost, st));
         PFG_CUDA(cudaStreamSynchronize(st));
         PFG_CHECK(host->err == 0, PFG_E_INTERNAL, "resident solve: a wait between CTAs ran out");

@@ -1,0 +1,75 @@
+"""Resident solves that share the device: threads, device memory, launches."""
+import threading
+import time
+
+import numpy as np
+import pytest
+
+from plantfem_gb300 import FEMSolver, problems
+
+pytestmark = pytest.mark.gpu
+
+
+def _solver(p):
+    s = FEMSolver()
+    s.setDomain(p["domain"])
+    s.setCRS(3)
+    s.assembleStiffness(p["E"], p["nu"])
+    s.setRHS(p["rhs"])
+    s.fix(1, p["fix_ids"], FixValue=0.0)
+    return s
+
+
+def _poisson(n=6000):
+    """1-D Poisson matrix: CG takes about n iterations."""
+    rows = [[j for j in (i - 1, i, i + 1) if 0 <= j < n] for i in range(n)]
+    rp = np.concatenate([[1], 1 + np.cumsum([len(r) for r in rows])]).astype(np.int64)
+    ci = np.concatenate(rows).astype(np.int32) + 1
+    v = np.concatenate([[2.0 if j == i else -1.0 for j in r] for i, r in enumerate(rows)])
+    s = FEMSolver()
+    s.setCRS(CRS=(rp, ci, v))
+    s.setRHS(np.random.default_rng(8).normal(size=n))
+    return s
+
+
+def test_a_short_solve_does_not_wait_for_a_long_one(cuda):
+    """While one thread runs 100,000 iterations (25 launches, about a second), another's
+    solve of a few milliseconds comes in between two launches; neither's bits change."""
+    kw = dict(algorithm="CG", stop_rule="true_relative")
+    long = _poisson()
+    long.relative_er, long.itrmax = 1e-30, 100000
+    ref = long.solve(**kw)
+    short = _solver(problems.cube(8))
+    alone = short.solve(**kw)
+    got = []
+    t = threading.Thread(target=lambda: got.append(long.solve(**kw)))
+    t.start()
+    time.sleep(0.1)
+    x = short.solve(**kw)
+    between = t.is_alive()
+    t.join()
+    assert between and np.array_equal(x, alone) and np.array_equal(got[0], ref)
+
+
+def test_threads_get_their_own_answers(cuda):
+    """Four threads, each with its own systems and forms, over and over: the bits of
+    the solves made one after another."""
+    forms = [dict(algorithm=a, precision=p, stop_rule="true_relative") for a in ("CG", "BiCGSTAB")
+             for p in ("fp64", "mixed")]
+    meshes = [problems.lognormal(n, seed=n) for n in (3, 6, 9, 12)]
+    ref = [[_solver(m).solve(**kw) for m in meshes] for kw in forms]
+    wrong = []
+
+    def work(k):
+        solvers = [_solver(m) for m in meshes]
+        for rep in range(6):
+            for i, s in enumerate(solvers):
+                kw = forms[(k + rep) % 4]
+                s.setRHS(meshes[i]["rhs"])
+                if not np.array_equal(s.solve(**kw), ref[(k + rep) % 4][i]):
+                    wrong.append((k, rep, i))
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not wrong, wrong
