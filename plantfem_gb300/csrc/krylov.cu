@@ -1753,13 +1753,17 @@ void Krylov::make_v32(DevMatrix &A, cudaStream_t st)
     A.v32_valid = true;
 }
 
-void Krylov::prepare(const DevMatrix &A, const KConfig &cfg, cudaStream_t st)
+void Krylov::prepare(const DevMatrix &A, const KConfig &cfg, bool resident, cudaStream_t st)
 {
     const int64_t n = A.ndof();
     const bool mixed = cfg.precision == PFG_PREC_MIXED;
     n_ = n;
     bs_ = A.bs;
     const size_t nn = (size_t)std::max<int64_t>(n, 1);
+    if (resident) {  // (its own vectors: run_resident)
+        if (mixed) xb_.ensure(nn);
+        return;
+    }
     r_.ensure(nn);
     z_.ensure(nn);
     pA_.ensure(nn);
@@ -2115,7 +2119,6 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
     const bool free_mode = cfg.fuse != 0 && cfg.fuse != 1;
     if (free_mode) cfg.fuse = 0;
     if (cfg.algorithm == PFG_ALG_BICGSTAB && cfg.precond != PFG_PC_NONE) cfg.fuse = 0;
-    prepare(A, cfg, st);
     launches_ = 0;
     // A solve that fits the SMs runs resident (run_resident); update_mode 1 and
     // 2 name one of the kernel-by-kernel forms, debug prints their progress.
@@ -2134,6 +2137,7 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
         return pl;
     };
     const ResPlan plan = plan_for(cfg);
+    prepare(A, cfg, plan.ctas > 0, st);
     // the Krylov kernels read the sliced copy: FP64 always (residuals), FP32
     // for the mixed inner iterations
     // the symmetric-storage inner iterations read only the upper-half FP32 copy
@@ -2158,8 +2162,8 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
                 c64.precision = PFG_PREC_FP64;
                 c64.stop_rule = PFG_STOP_TRUE_RELATIVE;
                 c64.itrmax = std::max(1, cfg.itrmax - res.iterations);
-                prepare(A, c64, st);
                 const ResPlan p64 = plan_for(c64);
+                prepare(A, c64, p64.ctas > 0, st);
                 SolveResult r2 = p64.ctas > 0                     ? run_resident(A, b, x, c64, p64, st)
                                  : cfg.algorithm == PFG_ALG_CG    ? run_cg64(A, b, x, c64, st)
                                                                   : run_bicgstab64(A, b, x, c64, st);
@@ -2198,20 +2202,9 @@ SolveResult Krylov::run_resident(DevMatrix &A, const double *b, double *x, const
 {
     const bool mixed = cfg.precision == PFG_PREC_MIXED;
     build_precond(A, cfg.precond, mixed, st);
-    if (!host_res_) {
-        PFG_CUDA(cudaMallocHost((void **)&host_res_, sizeof(ResState)));
-        memset(host_res_, 0, sizeof(ResState));
-        res_state_.alloc(sizeof(ResState));
-        res_slots_.alloc(kResSlots);
-    }
-    // the inboxes start empty; the rounds run on from solve to solve of one grid
-    // size, whose buffers each leaves in the order the next expects
-    unsigned round = host_res_->round;
-    if (res_ctas_ != plan.ctas || host_res_->err) {
-        PFG_CUDA(cudaMemsetAsync(res_slots_.p, 0xff, res_slots_.bytes(), st));
-        round = 0;
-    }
-    res_ctas_ = 0;  // until this solve has ended well
+    if (!host_res_) PFG_CUDA(cudaMallocHost((void **)&host_res_, sizeof(ResState)));
+    if (!res_state_.p) res_state_.alloc(sizeof(ResState));
+    if (!res_dev_) res_dev_ = ResDevice::current();
     ResArgs a;
     memset(&a, 0, sizeof a);
     a.A64 = A.sell<double>();
@@ -2233,7 +2226,6 @@ SolveResult Krylov::run_resident(DevMatrix &A, const double *b, double *x, const
     a.dinv64 = dinv_.p;
     a.dinv32 = dinv32_.p;
     a.st = reinterpret_cast<ResState *>(res_state_.p);
-    a.slots = res_slots_.p;
     a.pc = cfg.precond;
     a.stop_rule = cfg.stop_rule;
     a.itrmax = cfg.itrmax;
@@ -2243,9 +2235,7 @@ SolveResult Krylov::run_resident(DevMatrix &A, const double *b, double *x, const
     a.delta = cfg.reliable_delta;
     memset(host_res_, 0, sizeof(ResState));
     host_res_->first = 1;
-    host_res_->round = round;
-    launches_ += run_resident_kernel(plan, a, A.bs, cfg.algorithm, mixed, host_res_, st);
-    res_ctas_ = plan.ctas;
+    launches_ += run_resident_kernel(*res_dev_, plan, a, A.bs, cfg.algorithm, mixed, host_res_, st);
     const ResState &h = *host_res_;
     SolveResult res;
     res.status = h.status;

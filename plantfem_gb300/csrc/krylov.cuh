@@ -156,6 +156,7 @@ void block_jacobi(const DevMatrix &A, int precond, double *d64, float *d32, cuda
 class Ilu0;
 struct ResPlan;
 struct ResState;
+struct ResDevice;
 
 inline bool is_ilu(int precond) { return precond == PFG_PC_ILU0 || precond == PFG_PC_ILU0_SORTED; }
 
@@ -187,7 +188,8 @@ class Krylov {
     void ilu_reset();
 
   private:
-    void prepare(const DevMatrix &A, const KConfig &cfg, cudaStream_t st);
+    // Work vectors of a solve in either form.
+    void prepare(const DevMatrix &A, const KConfig &cfg, bool resident, cudaStream_t st);
     void build_precond(const DevMatrix &A, int precond, bool fp32, cudaStream_t st);
     SolveResult run_cg64(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st);
     SolveResult run_bicgstab64(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st);
@@ -218,14 +220,14 @@ class Krylov {
     DevBuf<unsigned int> ticket_;
     DevBuf<KState> state_;
     KState *host_state_ = nullptr;  // pinned mirror
-    // resident solves: state, its pinned mirror, exchange slots, published
-    // vectors, own vectors
+    // resident solves: state, its pinned mirror, published vectors, own vectors, and
+    // what all handles of the device share
     DevBuf<unsigned char> res_state_;
-    DevBuf<double> res_slots_, res_pub64_;
+    DevBuf<double> res_pub64_;
     DevBuf<float> res_pub32_;
     DevBuf<unsigned char> res_home_;
     ResState *host_res_ = nullptr;
-    int res_ctas_ = 0;       // CTAs that share the slots now
+    std::shared_ptr<ResDevice> res_dev_;
     // cached CUDA graphs of one chunk of iterations
     cudaGraphExec_t graph_ = nullptr;
     uint64_t graph_key_ = 0;

@@ -126,7 +126,7 @@ struct Grid {
     // the entry of CTA `from` in CTA `to`'s inbox
     __device__ double *entry(unsigned buf, int to, int from) const
     {
-        return slots + (((size_t)buf * kResMaxCtas + to) * kResMaxCtas + from) * kResValues;
+        return slots + (((size_t)buf * gridDim.x + to) * gridDim.x + from) * kResValues;
     }
 
     // v (valid in warp 0) -> the grid's totals in every thread; `fin(totals)` runs
@@ -1076,7 +1076,7 @@ __device__ void open_share(Share &h, ResShared &sh, const ResArgs &a, const int6
     g.err = &a.st->err;
     g.lane = threadIdx.x & 31;
     g.wid = threadIdx.x >> 5;
-    g.round = a.st->round;
+    g.round = 0;
     g.s0 = a.bounds[blockIdx.x];
     g.nsl = a.bounds[blockIdx.x + 1] - g.s0;
     int64_t *sp = take<int64_t>(mem, (size_t)g.nsl + 1 + ((g.nsl + 1) & 1));
@@ -1177,7 +1177,6 @@ __device__ void close_state(ResShared &sh, const Grid &g, const ResArgs &a, int 
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sh.state.phase = phase;
-        sh.state.round = g.round;
         sh.state.err = *(volatile int *)&a.st->err;
         *a.st = sh.state;
     }
@@ -1602,48 +1601,52 @@ ResPlan plan_resident(const DevMatrix &A, int algorithm, bool mixed, bool precon
     return pl;
 }
 
-namespace {
-
-// One grid whose CTAs wait for one another at a time on a device (each fills it: two that
-// held half the SMs each would wait until their limits).  The order is made on the device,
-// launch by launch: a launch waits in its stream for the end of the one before, whichever
-// thread's that was, and no thread waits for another solve on the host.  Several threads'
-// solves so alternate after at most one launch each (4,096 iterations), and those on
-// different devices do not meet.
-struct Turn {
-    std::mutex mu;
-    cudaEvent_t last = nullptr;
-};
-
-void launch_in_turn(const void *kern, dim3 grid, void **args, size_t smem, cudaStream_t st)
+std::shared_ptr<ResDevice> ResDevice::current()
 {
-    static Turn turns[64];
+    static std::mutex mu;
+    static std::weak_ptr<ResDevice> known[64];
     int dev = 0;
     PFG_CUDA(cudaGetDevice(&dev));
     PFG_CHECK(dev >= 0 && dev < 64, PFG_E_UNSUPPORTED, "device ordinal above 63");
-    Turn &t = turns[dev];
-    std::lock_guard<std::mutex> lk(t.mu);
-    if (t.last)
-        PFG_CUDA(cudaStreamWaitEvent(st, t.last, 0));
-    else
-        PFG_CUDA(cudaEventCreateWithFlags(&t.last, cudaEventDisableTiming));
-    PFG_CUDA(cudaLaunchCooperativeKernel(kern, grid, dim3(kNT), args, smem, st));
-    PFG_CUDA(cudaEventRecord(t.last, st));
+    std::lock_guard<std::mutex> lk(mu);
+    std::shared_ptr<ResDevice> d = known[dev].lock();
+    if (!d) {
+        d = std::make_shared<ResDevice>();
+        d->slots.alloc(kResSlots);
+        PFG_CUDA(cudaEventCreateWithFlags(&d->last, cudaEventDisableTiming));
+        known[dev] = d;
+    }
+    return d;
+}
+
+namespace {
+
+// The launch, after the one before on this device and with empty inboxes (a memset of at
+// most 3 MB, 2 us in the stream).
+void launch_in_turn(ResDevice &dev, const void *kern, int ctas, void **args, size_t smem, cudaStream_t st)
+{
+    std::lock_guard<std::mutex> lk(dev.mu);
+    PFG_CUDA(cudaStreamWaitEvent(st, dev.last, 0));
+    const size_t used = (size_t)kResRounds * kResValues * ctas * ctas;
+    PFG_CUDA(cudaMemsetAsync(dev.slots.p, 0xff, used * sizeof(double), st));
+    PFG_CUDA(cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(kNT), args, smem, st));
+    PFG_CUDA(cudaEventRecord(dev.last, st));
 }
 
 }  // namespace
 
-int run_resident_kernel(const ResPlan &pl, ResArgs a, int bs, int algorithm, bool mixed, ResState *host,
-                        cudaStream_t st)
+int run_resident_kernel(ResDevice &dev, const ResPlan &pl, ResArgs a, int bs, int algorithm, bool mixed,
+                        ResState *host, cudaStream_t st)
 {
     const ResKernel kern = pick_kernel(bs, algorithm, mixed);
     PFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
     a.stages = pl.stages;
     a.near = pl.near;
+    a.slots = dev.slots.p;
     void *args[] = {&a};
     PFG_CUDA(cudaMemcpyAsync(a.st, host, sizeof(ResState), cudaMemcpyHostToDevice, st));
     for (int launches = 1;; ++launches) {
-        launch_in_turn((const void *)kern, dim3(pl.ctas), args, pl.smem, st);
+        launch_in_turn(dev, (const void *)kern, pl.ctas, args, pl.smem, st);
         PFG_CUDA(cudaMemcpyAsync(host, a.st, sizeof(ResState), cudaMemcpyDeviceToHost, st));
         PFG_CUDA(cudaStreamSynchronize(st));
         PFG_CHECK(host->err == 0, PFG_E_INTERNAL, "resident solve: a wait between CTAs ran out");

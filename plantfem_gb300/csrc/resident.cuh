@@ -3,6 +3,8 @@
 // Implemented in resident.cu.
 #pragma once
 
+#include <mutex>
+
 #include "krylov.cuh"
 
 namespace pfg {
@@ -18,7 +20,6 @@ struct ResState {
     double rel, prev_rel, best_rel;
     float rmax32, rmin32;
     int err;         // raised when a wait runs out
-    unsigned round;  // exchanges made so far by the CTAs that share the slots
 };
 
 // What every resident kernel reads: matrices, the published (gathered) vectors
@@ -37,7 +38,7 @@ struct ResArgs {
     const double *dinv64;
     const float *dinv32;
     ResState *st;
-    double *slots;
+    double *slots;  // set by run_resident_kernel
     int pc, stop_rule, itrmax, budget, stages, near;
     double er0, tol, delta;
 };
@@ -54,6 +55,25 @@ constexpr int kResValues = 2;    // most values of one exchange
 constexpr int kResMaxCtas = 160;
 constexpr size_t kResSlots = (size_t)kResRounds * kResValues * kResMaxCtas * kResMaxCtas;
 
+// What the resident solves of a device share: the exchange slots, 3.3 MB, and their order.
+// One grid whose CTAs wait for one another at a time (each fills the device: two that
+// held half the SMs each would wait until their limits).  The order is made on the
+// device, launch by launch: a launch waits in its stream for the end of the one before,
+// whichever thread's that was, and no thread waits for another solve on the host.  Several
+// threads' solves so alternate after at most one launch each (4,096 iterations), and
+// those on different devices do not meet.  Held by the handles that have solved resident;
+// the last one gives it back.
+struct ResDevice {
+    std::mutex mu;
+    cudaEvent_t last = nullptr;  // end of the last launch
+    DevBuf<double> slots;
+    ~ResDevice()
+    {
+        if (last) cudaEventDestroy(last);
+    }
+    static std::shared_ptr<ResDevice> current();
+};
+
 // Cuts the sliced matrix into one run of slices per CTA with about equal work
 // (once per pattern: A.share, A.ctas, A.share_max).
 void share_slices(DevMatrix &A, cudaStream_t st);
@@ -63,7 +83,7 @@ ResPlan plan_resident(const DevMatrix &A, int algorithm, bool mixed, bool precon
 // Runs the solve from the state *host (page-locked; copied to a.st) until it is
 // finished, several launches if need be; *host then holds the final state.
 // Returns the launches made.
-int run_resident_kernel(const ResPlan &pl, ResArgs a, int bs, int algorithm, bool mixed, ResState *host,
-                        cudaStream_t st);
+int run_resident_kernel(ResDevice &dev, const ResPlan &pl, ResArgs a, int bs, int algorithm, bool mixed,
+                        ResState *host, cudaStream_t st);
 
 }  // namespace pfg
