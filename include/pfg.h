@@ -202,6 +202,14 @@ int pfg_element_stress(pfg_solver *h, const double *displacement, int64_t n_prop
  * x_out receives n values; info may be NULL. */
 int pfg_solve(pfg_solver *h, const pfg_solve_opts *opts, const double *x0, double *x_out, pfg_info *info);
 
+/* Limits of the handle's resident solves (a system that fits the SMs is solved by one
+ * cooperative launch; resident.cu).  launch_iterations: most iterations of one launch, a
+ * solve of more is continued by further launches with the same result (0: 4096).  ctas:
+ * CTAs of a launch, one to an SM (0: one for every SM); the order of the sums, and so the
+ * last digits, follow it.  Where the device does not hold them at once, the solve runs
+ * kernel by kernel. */
+int pfg_set_resident(pfg_solver *h, int32_t launch_iterations, int32_t ctas);
+
 /* Drop the ILU(0) factor the handle keeps for PFG_PC_ILU0* solves (the
  * reference keeps FEMSolver_%ILU_MATRIX for good, FEMSolverClass.f90:67,
  * LinearSolverClass.f90:4126-4135): the next ILU solve factors again. */

@@ -128,6 +128,7 @@ SIGNATURES = {
     "pfg_linear_solver_crs_noalloc": (C.c_int, [_P, _P, _P, _P, _P, _i64, C.POINTER(SolveOpts), C.POINTER(Info),
                                                 _P]),
     "pfg_eliminate": (C.c_int, [_P]),
+    "pfg_set_resident": (C.c_int, [_P, _i32, _i32]),
     "pfg_ilu_reset": (C.c_int, [_P]),
     "pfg_ilu_factor": (C.c_int, [_P, C.c_int32, _P]),
     "pfg_ilu_apply": (C.c_int, [_P, _P, _P]),

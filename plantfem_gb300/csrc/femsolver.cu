@@ -497,6 +497,16 @@ int pfg_solve(pfg_solver *h, const pfg_solve_opts *opts, const double *x0, doubl
     return solve_status(res);
 }
 
+int pfg_set_resident(pfg_solver *h, int32_t launch_iterations, int32_t ctas)
+{
+    return guard([&] {
+        need(h != nullptr, PFG_E_ARG, "NULL handle");
+        need(launch_iterations >= 0 && ctas >= 0, PFG_E_ARG, "negative limit of resident solves");
+        std::lock_guard<std::mutex> lk(h->mu);
+        h->kry.resident_limits(launch_iterations, ctas);
+    });
+}
+
 int pfg_dev_spmv(pfg_solver *h, const double *d_x, double *d_y, void *stream)
 {
     return guard([&] {

@@ -2131,7 +2131,7 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
                                                          : kResidentRowsBiCG64;
         if (may_reside && A.nb <= most) {
             build_sell(A, true, false, st);  // the pattern
-            share_slices(A, st);
+            share_slices(A, res_want_ctas_, st);
             pl = plan_resident(A, c.algorithm, mixed, c.precond != PFG_PC_NONE);
         }
         return pl;
@@ -2151,33 +2151,36 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
     PFG_CUDA(cudaEventRecord(e0, st));
     SolveResult res;
     try {
-        if (cfg.precision == PFG_PREC_MIXED) {
-            res = plan.ctas > 0 ? run_resident(A, b, x, cfg, plan, st) : run_mixed(A, b, x, cfg, st);
-            if (res.fallback) {
-                // The FP32 copy of the operator failed (repeated breakdowns or
-                // overflow, or FP64 residuals that stopped falling: a system
-                // whose conditioning is beyond FP32).  Finish in FP64 from the
-                // current x, within what is left of itrmax.
-                KConfig c64 = cfg;
-                c64.precision = PFG_PREC_FP64;
-                c64.stop_rule = PFG_STOP_TRUE_RELATIVE;
-                c64.itrmax = std::max(1, cfg.itrmax - res.iterations);
-                const ResPlan p64 = plan_for(c64);
-                prepare(A, c64, p64.ctas > 0, st);
-                SolveResult r2 = p64.ctas > 0                     ? run_resident(A, b, x, c64, p64, st)
-                                 : cfg.algorithm == PFG_ALG_CG    ? run_cg64(A, b, x, c64, st)
-                                                                  : run_bicgstab64(A, b, x, c64, st);
-                r2.iterations += res.iterations;
-                r2.replacements = res.replacements;
-                r2.fallback = 1;
-                res = r2;
+        // resident where planned and launched, else kernel by kernel
+        auto run = [&](const KConfig &c, const ResPlan &p) {
+            SolveResult r;
+            if (p.ctas > 0) {
+                if (run_resident(A, b, x, c, p, r, st)) return r;
+                prepare(A, c, false, st);
+                build_sell(A, true, c.precision == PFG_PREC_MIXED && c.storage != PFG_STORAGE_SYMMETRIC, st);
             }
-        } else if (plan.ctas > 0)
-            res = run_resident(A, b, x, cfg, plan, st);
-        else if (cfg.algorithm == PFG_ALG_CG)
-            res = run_cg64(A, b, x, cfg, st);
-        else
-            res = run_bicgstab64(A, b, x, cfg, st);
+            return c.precision == PFG_PREC_MIXED ? run_mixed(A, b, x, c, st)
+                   : c.algorithm == PFG_ALG_CG   ? run_cg64(A, b, x, c, st)
+                                                 : run_bicgstab64(A, b, x, c, st);
+        };
+        res = run(cfg, plan);
+        if (res.fallback) {
+            // The FP32 copy of the operator failed (repeated breakdowns or
+            // overflow, or FP64 residuals that stopped falling: a system
+            // whose conditioning is beyond FP32).  Finish in FP64 from the
+            // current x, within what is left of itrmax.
+            KConfig c64 = cfg;
+            c64.precision = PFG_PREC_FP64;
+            c64.stop_rule = PFG_STOP_TRUE_RELATIVE;
+            c64.itrmax = std::max(1, cfg.itrmax - res.iterations);
+            const ResPlan p64 = plan_for(c64);
+            prepare(A, c64, p64.ctas > 0, st);
+            SolveResult r2 = run(c64, p64);
+            r2.iterations += res.iterations;
+            r2.replacements = res.replacements;
+            r2.fallback = 1;
+            res = r2;
+        }
     } catch (...) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
@@ -2197,8 +2200,8 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
 // Most iterations of one resident launch.
 constexpr int kResidentBudget = 4096;
 
-SolveResult Krylov::run_resident(DevMatrix &A, const double *b, double *x, const KConfig &cfg, const ResPlan &plan,
-                                 cudaStream_t st)
+bool Krylov::run_resident(DevMatrix &A, const double *b, double *x, const KConfig &cfg, const ResPlan &plan,
+                          SolveResult &res, cudaStream_t st)
 {
     const bool mixed = cfg.precision == PFG_PREC_MIXED;
     build_precond(A, cfg.precond, mixed, st);
@@ -2229,15 +2232,16 @@ SolveResult Krylov::run_resident(DevMatrix &A, const double *b, double *x, const
     a.pc = cfg.precond;
     a.stop_rule = cfg.stop_rule;
     a.itrmax = cfg.itrmax;
-    a.budget = kResidentBudget;
+    a.budget = res_iterations_ > 0 ? res_iterations_ : kResidentBudget;
     a.er0 = cfg.er0;
     a.tol = cfg.relative_er;
     a.delta = cfg.reliable_delta;
     memset(host_res_, 0, sizeof(ResState));
     host_res_->first = 1;
-    launches_ += run_resident_kernel(*res_dev_, plan, a, A.bs, cfg.algorithm, mixed, host_res_, st);
+    const int made = run_resident_kernel(*res_dev_, plan, a, A.bs, cfg.algorithm, mixed, host_res_, st);
+    if (made == 0) return false;
+    launches_ += made;
     const ResState &h = *host_res_;
-    SolveResult res;
     res.status = h.status;
     res.iterations = h.iter;
     res.replacements = h.replacements;
@@ -2253,7 +2257,7 @@ SolveResult Krylov::run_resident(DevMatrix &A, const double *b, double *x, const
         res.iter_residual = sqrt(h.rr / (h.bb > 0 ? h.bb : 1.0));
     if (!res.fallback && res.status == PFG_OK && !by_reference && res.rel_residual > cfg.relative_er)
         res.status = PFG_W_NOT_CONVERGED;
-    return res;
+    return true;
 }
 
 SolveResult Krylov::run_cg64(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st)

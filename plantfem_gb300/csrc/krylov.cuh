@@ -183,6 +183,12 @@ class Krylov {
     // The ILU(0) factor kept for PFG_PC_ILU0* solves (ilu.cuh); factored from
     // A (if not held for A's pattern and this column order) by ilu_factor.
     const Ilu0 &ilu_factor(const DevMatrix &A, bool sorted, cudaStream_t st);
+    // Resident solves: iterations of one launch, CTAs (0: the defaults).
+    void resident_limits(int iterations, int ctas)
+    {
+        res_iterations_ = iterations;
+        res_want_ctas_ = ctas;
+    }
     // The factor held now (null if none).
     const Ilu0 *ilu_held() const;
     void ilu_reset();
@@ -194,9 +200,9 @@ class Krylov {
     SolveResult run_cg64(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st);
     SolveResult run_bicgstab64(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st);
     SolveResult run_mixed(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st);
-    // The whole solve in one cooperative launch (resident.cuh).
-    SolveResult run_resident(DevMatrix &A, const double *b, double *x, const KConfig &cfg, const ResPlan &plan,
-                             cudaStream_t st);
+    // The whole solve in one cooperative launch (resident.cuh).  False: not launched.
+    bool run_resident(DevMatrix &A, const double *b, double *x, const KConfig &cfg, const ResPlan &plan,
+                      SolveResult &res, cudaStream_t st);
     void read_state(KState &h, cudaStream_t st);
     // Hash of everything a captured chunk graph bakes in: every device pointer
     // its kernels receive and the configuration scalars.
@@ -228,6 +234,7 @@ class Krylov {
     DevBuf<unsigned char> res_home_;
     ResState *host_res_ = nullptr;
     std::shared_ptr<ResDevice> res_dev_;
+    int res_iterations_ = 0, res_want_ctas_ = 0;
     // cached CUDA graphs of one chunk of iterations
     cudaGraphExec_t graph_ = nullptr;
     uint64_t graph_key_ = 0;

@@ -1546,13 +1546,15 @@ ResKernel pick_kernel(int bs, int algorithm, bool mixed)
 // Work of a slice: its slots, and about four slots' worth of row updates.
 constexpr int64_t kRowWork = 4;
 
-void share_slices(DevMatrix &A, cudaStream_t st)
+void share_slices(DevMatrix &A, int ctas, cudaStream_t st)
 {
-    if (A.share_ctas > 0 || A.ns <= 0) return;
+    if (A.ns <= 0) return;
+    const int64_t G = std::min<int64_t>(A.ns, std::min(ctas > 0 ? ctas : sm_count_device(), kResMaxCtas));
+    if (A.share_ctas == G) return;
+    A.share_ctas = 0;
     std::vector<int64_t> sp((size_t)A.ns + 1);
     PFG_CUDA(cudaMemcpyAsync(sp.data(), A.sptr.p, sp.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     PFG_CUDA(cudaStreamSynchronize(st));
-    const int64_t G = std::min<int64_t>(A.ns, std::min(sm_count_device(), kResMaxCtas));
     const double total = (double)(sp[(size_t)A.ns] + kRowWork * A.ns);
     std::vector<int> b((size_t)G + 1, 0);
     int64_t s = 0, most = 0;
@@ -1622,15 +1624,21 @@ std::shared_ptr<ResDevice> ResDevice::current()
 namespace {
 
 // The launch, after the one before on this device and with empty inboxes (a memset of at
-// most 3 MB, 2 us in the stream).
-void launch_in_turn(ResDevice &dev, const void *kern, int ctas, void **args, size_t smem, cudaStream_t st)
+// most 3 MB, 2 us in the stream).  False: the device does not hold the grid at once.
+bool launch_in_turn(ResDevice &dev, const void *kern, int ctas, void **args, size_t smem, cudaStream_t st)
 {
     std::lock_guard<std::mutex> lk(dev.mu);
     PFG_CUDA(cudaStreamWaitEvent(st, dev.last, 0));
     const size_t used = (size_t)kResRounds * kResValues * ctas * ctas;
     PFG_CUDA(cudaMemsetAsync(dev.slots.p, 0xff, used * sizeof(double), st));
-    PFG_CUDA(cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(kNT), args, smem, st));
+    const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(kNT), args, smem, st);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    PFG_CUDA(e);
     PFG_CUDA(cudaEventRecord(dev.last, st));
+    return true;
 }
 
 }  // namespace
@@ -1646,7 +1654,10 @@ int run_resident_kernel(ResDevice &dev, const ResPlan &pl, ResArgs a, int bs, in
     void *args[] = {&a};
     PFG_CUDA(cudaMemcpyAsync(a.st, host, sizeof(ResState), cudaMemcpyHostToDevice, st));
     for (int launches = 1;; ++launches) {
-        launch_in_turn(dev, (const void *)kern, pl.ctas, args, pl.smem, st);
+        if (!launch_in_turn(dev, (const void *)kern, pl.ctas, args, pl.smem, st)) {
+            PFG_CHECK(launches == 1, PFG_E_CUDA, "resident solve: the device took no further launch");
+            return 0;
+        }
         PFG_CUDA(cudaMemcpyAsync(host, a.st, sizeof(ResState), cudaMemcpyDeviceToHost, st));
         PFG_CUDA(cudaStreamSynchronize(st));
         PFG_CHECK(host->err == 0, PFG_E_INTERNAL, "resident solve: a wait between CTAs ran out");

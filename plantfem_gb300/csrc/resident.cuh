@@ -75,14 +75,16 @@ struct ResDevice {
 };
 
 // Cuts the sliced matrix into one run of slices per CTA with about equal work
-// (once per pattern: A.share, A.ctas, A.share_max).
-void share_slices(DevMatrix &A, cudaStream_t st);
+// (once per pattern and number of CTAs: A.share, A.share_ctas, A.share_max).  ctas 0: one
+// for every SM.
+void share_slices(DevMatrix &A, int ctas, cudaStream_t st);
 
 ResPlan plan_resident(const DevMatrix &A, int algorithm, bool mixed, bool precond);
 
 // Runs the solve from the state *host (page-locked; copied to a.st) until it is
 // finished, several launches if need be; *host then holds the final state.
-// Returns the launches made.
+// Returns the launches made; 0 where the device does not hold the grid at once (it may
+// give a process fewer SMs than it has): x is as it was.
 int run_resident_kernel(ResDevice &dev, const ResPlan &pl, ResArgs a, int bs, int algorithm, bool mixed,
                         ResState *host, cudaStream_t st);
 

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from plantfem_gb300 import FEMSolver, problems
+from plantfem_gb300 import _native as N
 
 pytestmark = pytest.mark.gpu
 
@@ -93,3 +94,38 @@ def test_small_handles_stay_small(cuda, kw):
 
     before = more(4)
     assert (before - more(64)) / 64 < 1.0e6
+
+
+def _resident(s, launch_iterations=0, ctas=0):
+    N.check(N.load().pfg_set_resident(s.handle, launch_iterations, ctas))
+
+
+@pytest.mark.parametrize("algorithm", ["CG", "BiCGSTAB"])
+@pytest.mark.parametrize("precision,storage", [("fp64", "full"), ("mixed", "full"), ("mixed", "symmetric")])
+def test_a_grid_the_device_does_not_hold(cuda, algorithm, precision, storage):
+    """More CTAs than the device has SMs: the launch is refused and the solve runs kernel
+    by kernel, to the same bits as when that form is asked for (all but the symmetric
+    CG's, whose sums go by atomics).  Fewer CTAs: resident, with its own order of sums
+    (tolerance as in the resident tests)."""
+    s = _solver(problems.lognormal(17, seed=4))  # 183 slices
+    s.relative_er = 1e-12
+    kw = dict(algorithm=algorithm, precision=precision, storage=storage, stop_rule="true_relative",
+              preconditioning="BlockJacobi")
+    sep = s.solve(update_mode="separate", **kw)
+    _resident(s, ctas=160)
+    x = s.solve(**kw)
+    info = dict(s.last_info)
+    assert info["status"] == 0 and info["kernel_launches"] > 10, info
+    if (algorithm, storage) == ("CG", "symmetric"):
+        assert np.linalg.norm(x - sep) <= 1e-8 * np.linalg.norm(sep)
+    else:
+        assert np.array_equal(x, sep)
+    _resident(s, ctas=40)
+    y = s.solve(**kw)
+    assert s.last_info["status"] == 0 and s.last_info["kernel_launches"] < 10, s.last_info
+    assert np.linalg.norm(y - sep) <= 1e-8 * np.linalg.norm(sep)
+    _resident(s)
+    z = s.solve(**kw)
+    t = _solver(problems.lognormal(17, seed=4))
+    t.relative_er = 1e-12
+    assert np.array_equal(z, t.solve(**kw))
