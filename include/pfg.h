@@ -84,7 +84,7 @@ typedef struct pfg_solve_opts {
     double relative_er;      /* FEMSolver_%relative_er, default 1e-10 (FEMSolverClass.f90:71) */
     double reliable_delta;   /* mixed: replace the FP32 residual by the FP64 one whenever it fell
                                 by this factor since the last replacement; default 0.1 */
-    int32_t debug;           /* FEMSolver_%debug: print the residual per graph chunk */
+    int32_t debug;           /* FEMSolver_%debug: print the residual every graph_chunk iterations */
     int32_t update_mode;     /* 0 auto, 1 vector updates fused into the SpMV gathers,
                                 2 separate streaming passes (see krylov.cu) */
     int32_t storage;         /* mixed: PFG_STORAGE_FULL (default) or PFG_STORAGE_SYMMETRIC */

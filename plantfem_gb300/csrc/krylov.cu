@@ -2121,8 +2121,8 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
     if (cfg.algorithm == PFG_ALG_BICGSTAB && cfg.precond != PFG_PC_NONE) cfg.fuse = 0;
     launches_ = 0;
     // A solve that fits the SMs runs resident (run_resident); update_mode 1 and
-    // 2 name one of the kernel-by-kernel forms, debug prints their progress.
-    const bool may_reside = free_mode && cfg.debug == 0 && !is_ilu(cfg.precond);
+    // 2 name one of the kernel-by-kernel forms.
+    const bool may_reside = free_mode && !is_ilu(cfg.precond);
     auto plan_for = [&](const KConfig &c) {
         ResPlan pl;
         const bool mixed = c.precision == PFG_PREC_MIXED;
@@ -2232,13 +2232,17 @@ bool Krylov::run_resident(DevMatrix &A, const double *b, double *x, const KConfi
     a.pc = cfg.precond;
     a.stop_rule = cfg.stop_rule;
     a.itrmax = cfg.itrmax;
-    a.budget = res_iterations_ > 0 ? res_iterations_ : kResidentBudget;
+    // (debug: progress as often as kernel by kernel; a continued solve has the same bits)
+    a.budget = cfg.debug != 0         ? std::max(1, cfg.graph_chunk)
+               : res_iterations_ > 0 ? res_iterations_
+                                     : kResidentBudget;
     a.er0 = cfg.er0;
     a.tol = cfg.relative_er;
     a.delta = cfg.reliable_delta;
     memset(host_res_, 0, sizeof(ResState));
     host_res_->first = 1;
-    const int made = run_resident_kernel(*res_dev_, plan, a, A.bs, cfg.algorithm, mixed, host_res_, st);
+    const int made =
+        run_resident_kernel(*res_dev_, plan, a, A.bs, cfg.algorithm, mixed, host_res_, cfg.debug != 0, st);
     if (made == 0) return false;
     launches_ += made;
     const ResState &h = *host_res_;

@@ -1644,7 +1644,7 @@ bool launch_in_turn(ResDevice &dev, const void *kern, int ctas, void **args, siz
 }  // namespace
 
 int run_resident_kernel(ResDevice &dev, const ResPlan &pl, ResArgs a, int bs, int algorithm, bool mixed,
-                        ResState *host, cudaStream_t st)
+                        ResState *host, bool debug, cudaStream_t st)
 {
     const ResKernel kern = pick_kernel(bs, algorithm, mixed);
     PFG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax));
@@ -1661,6 +1661,12 @@ int run_resident_kernel(ResDevice &dev, const ResPlan &pl, ResArgs a, int bs, in
         PFG_CUDA(cudaMemcpyAsync(host, a.st, sizeof(ResState), cudaMemcpyDeviceToHost, st));
         PFG_CUDA(cudaStreamSynchronize(st));
         PFG_CHECK(host->err == 0, PFG_E_INTERNAL, "resident solve: a wait between CTAs ran out");
+        if (debug && mixed)
+            fprintf(stderr, "[pfg] mixed iter %d replacement %d |b-Ax|/|b| %.3e%s\n", host->iter, host->replacements,
+                    host->rel, host->fallback ? ", hand-over to FP64" : "");
+        else if (debug)
+            fprintf(stderr, "[pfg] %s iter %d |r| %.3e\n", algorithm == PFG_ALG_CG ? "CG64" : "BiCGSTAB64", host->iter,
+                    sqrt(host->rr));
         if (host->phase == 2) return launches;
     }
 }

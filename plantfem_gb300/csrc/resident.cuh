@@ -84,8 +84,9 @@ ResPlan plan_resident(const DevMatrix &A, int algorithm, bool mixed, bool precon
 // Runs the solve from the state *host (page-locked; copied to a.st) until it is
 // finished, several launches if need be; *host then holds the final state.
 // Returns the launches made; 0 where the device does not hold the grid at once (it may
-// give a process fewer SMs than it has): x is as it was.
+// give a process fewer SMs than it has): x is as it was.  debug: the state after each
+// launch on stderr.
 int run_resident_kernel(ResDevice &dev, const ResPlan &pl, ResArgs a, int bs, int algorithm, bool mixed,
-                        ResState *host, cudaStream_t st);
+                        ResState *host, bool debug, cudaStream_t st);
 
 }  // namespace pfg

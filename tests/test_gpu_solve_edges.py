@@ -125,3 +125,20 @@ def test_right_hand_sides_of_extreme_scale(cuda, algorithm, scale):
     sep = s.last_info
     assert res["status"] == sep["status"] == 0 and res["rel_residual"] <= 1e-4, (res, sep)
     assert abs(res["iterations"] - sep["iterations"]) <= 2, (res, sep)
+
+
+@pytest.mark.parametrize("algorithm", ["CG", "BiCGSTAB"])
+@pytest.mark.parametrize("precision,storage", [("fp64", "full"), ("mixed", "full"), ("mixed", "symmetric")])
+def test_debug_prints_and_changes_nothing(cuda, capfd, algorithm, precision, storage):
+    """debug shows the solve that runs without it: same bits, same count, a line every 32
+    iterations (graph_chunk)."""
+    s = _solver(problems.lognormal(12, seed=2))
+    kw = dict(algorithm=algorithm, precision=precision, storage=storage, stop_rule="true_relative")
+    x = s.solve(**kw)
+    it = s.last_info["iterations"]
+    assert "[pfg]" not in capfd.readouterr().err
+    s.debug = True
+    y = s.solve(**kw)
+    lines = [t for t in capfd.readouterr().err.splitlines() if t.startswith("[pfg]")]
+    assert np.array_equal(x, y) and s.last_info["iterations"] == it
+    assert len(lines) >= it // 32 >= 2, lines
