@@ -2087,12 +2087,48 @@ static int bicg_chunk_sym(const SellView<float> &U, float rowsum, int chunk, int
     return 7 * chunk;
 }
 
-// Largest systems (block rows) that run resident: FP64 CG, FP64 BiCGSTAB, mixed.
-// Where the two forms meet (us per iteration, kernel by kernel / resident): FP64
-// CG 389,017 rows 217.8 / 215.3; FP64 BiCGSTAB 148,877 rows 179.8 / 180.9; mixed
-// 91,125 rows 30.9 / 24.6 (CG) and 66.9 / 52.6 (BiCGSTAB), 148,877 rows 32.7 / 45.8
-// and 75.3 / 94.4 (the full FP32 copy no longer fits L2).
+// Which systems run resident: up to so many block rows (FP64 CG, FP64 BiCGSTAB, mixed),
+// with two exceptions.  All figures are us per iteration, kernel by kernel / resident, of
+// 48 iterations with block Jacobi (a 1x1 block's is Jacobi; without it both are some per
+// cent less).  3x3 blocks, 27 to a row (hexes):
+//   FP64 CG        91,125 rows 86.7 / 62.0   226,981 rows 171.5 / 136.0   389,017 rows 219.9 / 222.0
+//   FP64 BiCGSTAB  91,125 rows 156.5 / 121.2 148,877 rows 190.5 / 181.6
+//   mixed CG       91,125 rows 31.7 / 26.6 (half stored), 41.9 / 26.7 (full); 148,877 rows 37.4 / 48.2
+//                  and 49.5 / 48.1
+//   mixed BiCGSTAB 91,125 rows 69.9 / 56.6 (half), 97.2 / 56.3 (full); 148,877 rows 79.1 / 95.6 (half)
+// Other 3x3 rows inside the limits: 7 blocks, 140,608 rows, FP64 CG 49.7 / 38.4, mixed 28.3
+// / 18.4; 118 blocks, 97,336 rows, FP64 CG 298 / 214, full mixed CG 132 / 109, half-stored
+// mixed BiCGSTAB 211 / 203.
+// * Mixed CG asked to read the half copy reads the whole one when resident, which pays
+//   while that lies in L2 (here 135.5 MB): 110 to 115 blocks a row, 119 MB 54.2 / 40.6, 176 MB
+//   52.7 / 51.3, 292 MB 67.6 / 76.9, 450 MB 90.9 / 108.6.
+// * FP64 with 1x1 blocks: a chunk of the ring is one slot, so 32 entries (384 bytes) cost
+//   a copy and a barrier wait.  CG, 27 entries a row: 46,656 rows
+//   25.1 / 20.1, 85,184 rows 28.0 / 29.2, 389,017 rows 56.5 / 99.2; 7 a row: 314,432 rows 34.4 /
+//   31.6; 112 a row, where a warp's chain of slots is long: 64,000 rows 70.3 / 67.1, 79,507
+//   rows 71.1 / 84.1.  BiCGSTAB 27 a row: 85,184 rows 58.0 / 53.5, 132,651 rows 64.0 / 70.7.
 constexpr int64_t kResidentRowsCG64 = 400000, kResidentRowsBiCG64 = 140000, kResidentRowsMixed = 110000;
+constexpr int64_t kResidentScalarRows = 64000, kResidentScalarEntries = 2000000;
+
+static int64_t l2_bytes()
+{
+    int dev = 0, v = 0;
+    PFG_CUDA(cudaGetDevice(&dev));
+    PFG_CUDA(cudaDeviceGetAttribute(&v, cudaDevAttrL2CacheSize, dev));
+    return v;
+}
+
+// (A's sliced pattern is built)
+static bool resident_pays(const DevMatrix &A, const KConfig &c)
+{
+    const int64_t entries = (int64_t)A.scol.n;  // blocks, padding included
+    if (c.precision == PFG_PREC_MIXED)
+        return A.nb <= kResidentRowsMixed &&
+               (c.algorithm != PFG_ALG_CG || c.storage != PFG_STORAGE_SYMMETRIC ||
+                entries * (4 + 4 * A.bs * A.bs) <= l2_bytes());
+    if (A.nb > (c.algorithm == PFG_ALG_CG ? kResidentRowsCG64 : kResidentRowsBiCG64)) return false;
+    return A.bs > 1 || A.nb <= kResidentScalarRows || entries <= kResidentScalarEntries;
+}
 
 SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfig &cfg_in, cudaStream_t st)
 {
@@ -2125,16 +2161,11 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
     const bool may_reside = free_mode && !is_ilu(cfg.precond);
     auto plan_for = [&](const KConfig &c) {
         ResPlan pl;
-        const bool mixed = c.precision == PFG_PREC_MIXED;
-        const int64_t most = mixed                          ? kResidentRowsMixed
-                             : c.algorithm == PFG_ALG_CG ? kResidentRowsCG64
-                                                         : kResidentRowsBiCG64;
-        if (may_reside && A.nb <= most) {
-            build_sell(A, true, false, st);  // the pattern
-            share_slices(A, res_want_ctas_, st);
-            pl = plan_resident(A, c.algorithm, mixed, c.precond != PFG_PC_NONE);
-        }
-        return pl;
+        if (!may_reside || A.nb > kResidentRowsCG64) return pl;
+        build_sell(A, true, false, st);  // the pattern
+        if (!resident_pays(A, c)) return pl;
+        share_slices(A, res_want_ctas_, st);
+        return plan_resident(A, c.algorithm, c.precision == PFG_PREC_MIXED, c.precond != PFG_PC_NONE);
     };
     const ResPlan plan = plan_for(cfg);
     prepare(A, cfg, plan.ctas > 0, st);

@@ -65,3 +65,55 @@ def test_vectors_outside_shared_memory(cuda, algorithm, precision, pc):
     y = s.solve(update_mode="separate", **kw)
     assert s.last_info["status"] == 0
     assert np.linalg.norm(x - y) <= 2.4e-6 * np.linalg.norm(y)
+
+
+def _band(rows, half, bs, spread=1):
+    """Diagonally dominant band matrix of 2 half + 1 blocks a row as 1-based CRS (fewer at
+    the ends), each block off the diagonal -1 on its diagonal."""
+    off = spread * np.arange(-half, half + 1)
+    j = np.arange(rows)[:, None] + off[None, :]
+    keep = (j >= 0) & (j < rows)
+    cnt = keep.sum(axis=1)
+    cols = j[keep].astype(np.int32)
+    row = np.repeat(np.arange(rows, dtype=np.int32), cnt)
+    val = np.where(cols == row, 2.0 * half + 1.0, -1.0)
+    if bs == 1:
+        return np.concatenate([[1], 1 + np.cumsum(cnt)]).astype(np.int64), cols + 1, val
+    first = np.concatenate([[0], np.cumsum(cnt)])[:-1]
+    pos = np.arange(cols.size) - first[row]
+    rp = np.concatenate([[1], 1 + np.cumsum(np.repeat(bs * cnt, bs))]).astype(np.int64)
+    ci, v = np.empty(bs * bs * cols.size, np.int32), np.zeros(bs * bs * cols.size)
+    for r in range(bs):
+        for c in range(bs):
+            at = bs * bs * first[row] + r * bs * cnt[row] + bs * pos + c
+            ci[at] = bs * cols + c + 1
+            if r == c:
+                v[at] = val
+    return rp, ci, v
+
+
+# (rows, blocks on each side, block size, form, runs resident): both sides of the rules that
+# count entries and bytes.  The 3x3 copy of 30,000 rows with 121 blocks is 145 MB, of 20,000
+# rows 97 MB; 70,000 rows with 31 entries are 2.2 million.
+@pytest.mark.parametrize("rows,half,bs,kw,resident", [
+    (70000, 15, 1, dict(precision="fp64"), False),
+    (60000, 20, 1, dict(precision="fp64"), True),
+    (70000, 10, 1, dict(precision="fp64"), True),
+    (70000, 15, 1, dict(precision="fp64", algorithm="BiCGSTAB"), False),
+    (70000, 15, 1, dict(precision="mixed"), True),
+    (30000, 60, 3, dict(precision="mixed", storage="symmetric"), False),
+    (30000, 60, 3, dict(precision="mixed"), True),
+    (20000, 60, 3, dict(precision="mixed", storage="symmetric"), True)])
+def test_which_solves_run_resident(cuda, rows, half, bs, kw, resident):
+    rp, ci, v = _band(rows, half, bs, spread=3)
+    s = FEMSolver()
+    s.setCRS(CRS=(rp, ci, v))
+    b = np.random.default_rng(1).normal(size=bs * rows)
+    s.setRHS(b)
+    s.relative_er = 1e-8
+    x = s.solve(**{"algorithm": "CG", "stop_rule": "true_relative", "preconditioning": "BlockJacobi", **kw})
+    assert s.last_info["status"] == 0
+    assert (s.last_info["kernel_launches"] < 10) == resident, s.last_info
+    row = np.repeat(np.arange(bs * rows), np.diff(rp))
+    r = b - np.bincount(row, weights=v * x[ci - 1], minlength=bs * rows)
+    assert np.linalg.norm(r) <= 1.01e-8 * np.linalg.norm(b)
