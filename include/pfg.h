@@ -466,9 +466,9 @@ int pfg_batch_set_wait_limit(pfg_batch *b, int64_t cycles);
 /* No counterpart in the reference (it has only wall-clock timers, TimeClass.f90).
  * Times `reps` back-to-back launches of one kernel on the handle's matrix with
  * CUDA events on the handle's stream and returns the mean milliseconds per
- * launch and the algorithmic bytes one launch moves.  kernel: 0 = FP64 block
- * SpMV, 1 = FP32 block SpMV, 2 = the FP32 CG SpMV with the fused direction
- * update, 3 / 4 = FP64 / FP32 warp-per-row BCRS SpMV, 5 / 6 = the FP32 / FP64
+ * launch and the algorithmic bytes one launch moves.  kernel: 0 / 1 = the FP64 /
+ * FP32 product from the sliced copy (0: pfg_dev_spmv's), 2 = the FP32 CG SpMV with the
+ * fused direction update, 3 / 4 = FP64 / FP32 warp-per-row BCRS SpMV, 5 / 6 = the FP32 / FP64
  * CG SpMV with the p.q reduction (the dominant kernels of the mixed and FP64
  * solves with streaming update passes, the default), 7 = the FP32 product from
  * the upper half of a symmetric matrix (PFG_STORAGE_SYMMETRIC), 8 = its CG form

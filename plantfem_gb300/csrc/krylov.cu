@@ -164,25 +164,6 @@ __global__ void __launch_bounds__(kThreads) k_spmv(BsrView<T> A, const T *__rest
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;                     \
     for (int64_t s = w0; s < (A).ns; s += nw)
 
-// y = A x on the sliced copy (plain SpMV, profiling and the FP32 entry point).
-template <int BS, typename T>
-__global__ void __launch_bounds__(kThreads) k_spmv_sell(SellView<T> A, const T *__restrict__ x, T *__restrict__ y)
-{
-    PFG_SLICE_LOOP(A)
-    {
-        T acc[BS];
-        auto src = [&](int c, T(&xv)[BS]) {
-#pragma unroll
-            for (int i = 0; i < BS; ++i) xv[i] = __ldg(x + (int64_t)BS * c + i);
-        };
-        sell_row_product<BS>(A, s, lane, src, acc);
-        const int64_t row = s * 32 + lane;
-        if (row < A.nb)
-#pragma unroll
-            for (int i = 0; i < BS; ++i) y[BS * row + i] = acc[i];
-    }
-}
-
 // y = A x with a CTA of kWarps warps per slice: each takes an eighth of the slots,
 // the sums are added in warp order.  Both ends gain from the fine split: a warp per
 // slice puts a 1,430-row matrix on 6 SMs, each bound by its FP64 pipe (a slice of 27
@@ -1721,15 +1702,23 @@ void Krylov::spmv64(const DevMatrix &A, const double *x, double *y, cudaStream_t
         launch_spmv<1, double>(A, A.view<double>(), x, y, st);
 }
 
+// The product of a caller's pfg_dev_spmv and of a time step (FP64), and what the profile
+// times as the plain product.
+template <typename T>
+static void launch_split(const DevMatrix &A, const T *x, T *y, cudaStream_t st)
+{
+    const int g = (int)std::min<int64_t>(A.ns, 1 << 20);
+    if (A.bs == 3)
+        k_spmv_split<3, T><<<g, kThreads, 0, st>>>(A.sell<T>(), x, y);
+    else
+        k_spmv_split<1, T><<<g, kThreads, 0, st>>>(A.sell<T>(), x, y);
+}
+
 void Krylov::spmv64_sliced(DevMatrix &A, const double *x, double *y, cudaStream_t st)
 {
     if (A.nb == 0) return;
     build_sell(A, true, false, st);
-    const int g = (int)std::min<int64_t>(A.ns, 1 << 20);
-    if (A.bs == 3)
-        k_spmv_split<3, double><<<g, kThreads, 0, st>>>(A.sell<double>(), x, y);
-    else
-        k_spmv_split<1, double><<<g, kThreads, 0, st>>>(A.sell<double>(), x, y);
+    launch_split(A, x, y, st);
     PFG_CUDA(cudaGetLastError());
 }
 
@@ -2763,8 +2752,6 @@ void Krylov::profile(DevMatrix &A, int kernel, int reps, cudaStream_t st, double
         ticket_.alloc(1);
         PFG_CUDA(cudaMemsetAsync(ticket_.p, 0, sizeof(unsigned), st));
     }
-    const int g0 = A.bs == 3 ? resident_grid(k_spmv_sell<3, double>, A.ns) : resident_grid(k_spmv_sell<1, double>, A.ns);
-    const int g1 = A.bs == 3 ? resident_grid(k_spmv_sell<3, float>, A.ns) : resident_grid(k_spmv_sell<1, float>, A.ns);
     const int g2 = A.bs == 3 ? resident_grid(k_cg_spmv<3, float>, A.ns) : resident_grid(k_cg_spmv<1, float>, A.ns);
     const int g5 = A.bs == 3 ? resident_grid(k_cg_spmv_u<3, float>, A.ns) : resident_grid(k_cg_spmv_u<1, float>, A.ns);
     const int g6 = A.bs == 3 ? resident_grid(k_cg_spmv_u<3, double>, A.ns) : resident_grid(k_cg_spmv_u<1, double>, A.ns);
@@ -2774,12 +2761,10 @@ void Krylov::profile(DevMatrix &A, int kernel, int reps, cudaStream_t st, double
     auto launch = [&]() {
         switch (kernel) {
         case 0:
-            if (A.bs == 3) k_spmv_sell<3, double><<<g0, kThreads, 0, st>>>(A.sell<double>(), x64.p, y64.p);
-            else k_spmv_sell<1, double><<<g0, kThreads, 0, st>>>(A.sell<double>(), x64.p, y64.p);
+            launch_split(A, x64.p, y64.p, st);
             break;
         case 1:
-            if (A.bs == 3) k_spmv_sell<3, float><<<g1, kThreads, 0, st>>>(A.sell<float>(), x32.p, y32.p);
-            else k_spmv_sell<1, float><<<g1, kThreads, 0, st>>>(A.sell<float>(), x32.p, y32.p);
+            launch_split(A, x32.p, y32.p, st);
             break;
         case 2:
             if (A.bs == 3)
