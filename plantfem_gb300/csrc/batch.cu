@@ -129,20 +129,6 @@ __device__ __forceinline__ void team_sync(Team &tm, TeamShared &sh)
         __syncthreads();
 }
 
-// Sum over the 32 lanes of NV = 1 or 2 FP64 values: for two, the halves of the warp
-// first trade values and then carry one each, 5 additions instead of 10.  The total of
-// value k ends up in lane 16 k (of one value: in every lane).
-template <int NV>
-__device__ __forceinline__ double lanes_sum(const double (&v)[NV], int lane)
-{
-    if (NV == 1) return warp_sum(v[0]);
-    const bool upper = (lane & 16) != 0;
-    double t = (upper ? v[NV - 1] : v[0]) + __shfl_xor_sync(0xffffffffu, upper ? v[0] : v[NV - 1], 16);
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    return t;
-}
-
 // Team-wide sums of NV = 1 or 2 FP64 values, left in v of thread 0 of every CTA (the
 // same bits in each).  An FP64 instruction holds its quarter of the SM's pipe for 64
 // cycles whichever warp issues it, so what follows the warps' own sums is done by

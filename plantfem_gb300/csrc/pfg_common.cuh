@@ -142,6 +142,20 @@ __device__ __forceinline__ T warp_sum(T v)
     return v;
 }
 
+// Sum over a warp of one or two FP64 values; value k's total ends up in lane 16 k (of one
+// value: in every lane).  For two the halves of the warp trade values first and then carry
+// one each: 5 additions instead of 10, each 64 cycles of the quarter SM's pipe.
+template <int NV>
+__device__ __forceinline__ double lanes_sum(const double (&v)[NV], int lane)
+{
+    if (NV == 1) return warp_sum(v[0]);
+    const bool upper = (lane & 16) != 0;
+    double t = (upper ? v[NV - 1] : v[0]) + __shfl_xor_sync(0xffffffffu, upper ? v[0] : v[NV - 1], 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
 // Streaming load of matrix data that is read once per sweep: read-only path,
 // not allocated in L1, so L1 keeps the gathered source vector.
 __device__ __forceinline__ float ld_stream(const float *p)

@@ -79,20 +79,6 @@ __device__ __forceinline__ void ld_entry(const double *p, double &a, double &b)
         asm volatile("ld.volatile.global.f64 %0, [%1];" : "=d"(a) : "l"(p) : "memory");
 }
 
-// Sum over a warp of one or two FP64 values; value k's total ends up in lane 16 k.  For
-// two the halves of the warp trade values first and then carry one each: 5 additions
-// instead of 10, each 64 cycles of the quarter SM's pipe.
-template <int NV>
-__device__ __forceinline__ double lanes_sum(const double (&v)[NV], int lane)
-{
-    if (NV == 1) return warp_sum(v[0]);
-    const bool upper = (lane & 16) != 0;
-    double t = (upper ? v[NV - 1] : v[0]) + __shfl_xor_sync(0xffffffffu, upper ? v[0] : v[NV - 1], 16);
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    return t;
-}
-
 enum Step { kGo, kDone, kReplace, kLost };
 
 // The scalars an iteration changes.
