@@ -1332,7 +1332,7 @@ __global__ void k_reduce_residual(const double *__restrict__ part, int nparts, i
 // move with 16-byte accesses.
 template <typename T>
 __global__ void __launch_bounds__(kT)
-    k_lincomb(int64_t n, int k, int nblk, const CombSet<T> set, const double *__restrict__ C)
+    k_lincomb(int64_t n, int k, int nblk, const __grid_constant__ CombSet<T> set, const double *__restrict__ C)
 {
     const T *__restrict__ X = set.X[blockIdx.y];
     const T *__restrict__ W = set.W[blockIdx.y];
