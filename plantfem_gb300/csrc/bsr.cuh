@@ -72,13 +72,19 @@ __device__ __forceinline__ void bsr_row_product(const BsrView<T> &A, int64_t row
 // thread loading its partials (kPartAhead at once) makes it one or two trips
 // (launch durations): FP64 CG update, 681k unknowns, 760 CTAs, 26.7 -> 23.6 us; FP32 CG
 // update, 3.09M unknowns, 30.6 -> 29.3 us.
-// WIDE false (the sliced products): one warp reads them (FP64: four at once).  Behind a loop that lives on
-// its loads in flight the wide form makes the compiler give that loop fewer registers:
-// at 1.03M block rows the FP32 CG product took 280 us with it (40 registers) and 186
-// without (48), fused 254 and 200, the FP64 one 475 and 442.
-// BiCGSTAB's vector passes use it too (one order for all of its sums, which its
-// iteration count follows; a microsecond of the thousand an iteration takes there).
+// Up to kFewParts FP64 partials go to one warp all the same: they are one or two trips
+// for it too, and the second tree is 40 warp instructions of the slow pipe (FP64 CG kernel
+// by kernel, 125 and 2,197 block rows, 35.8 and 37.1 us an iteration wide, 35.0 and 36.4 so;
+// the same above 9,261 rows.  FP32: wide is the faster at all sizes, 50,653 rows 21.7
+// and 23.1).
+// WIDE false (the sliced products): one warp reads them (FP64: four at once).  Behind a
+// loop that lives on its loads in flight the wide form makes the compiler give that loop
+// fewer registers: at 1.03M block rows the FP32 CG product took 280 us with it (40
+// registers) and 186 without (48), fused 254 and 200, the FP64 one 475 and 442.
+// BiCGSTAB's vector passes are narrow too: all of its sums then have one order, and it costs
+// a microsecond of the thousand an iteration takes at that size.
 constexpr int kPartAhead = 4;
+constexpr unsigned kFewParts = 256;
 
 struct GridTicket {
     unsigned int *counter;
@@ -160,7 +166,7 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *partials, unsi
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    if constexpr (WIDE) {
+    if (WIDE && gridDim.x > kFewParts) {
         double acc[NV];
 #pragma unroll
         for (int k = 0; k < NV; ++k) acc[k] = 0.0;
