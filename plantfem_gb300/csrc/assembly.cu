@@ -382,17 +382,23 @@ __global__ void __launch_bounds__(kElemThreads, MINB)
     b4 += a4;
     for (int64_t base = (int64_t)blockIdx.x * kEPC; base < n_el; base += (int64_t)gridDim.x * kEPC) {
         const int here = (int)min((int64_t)kEPC, n_el - base);
-        if (tid < 8 * here) {
+        bool twice = false;
+        if (tid < 8 * kEPC) {
             const int q = tid >> 3, v = tid & 7;
-            const int64_t li = base + q;
-            const int e = elems ? elems[li] : (int)li;
-            const int node = conn[(int64_t)v * ne + e];
-            sNode[q][v] = node;
-            sX[q][v][0] = xyz[node];
-            sX[q][v][1] = xyz[nn + node];
-            sX[q][v][2] = xyz[2 * nn + node];
+            int node = -1 - v;
+            if (q < here) {
+                const int64_t li = base + q;
+                const int e = elems ? elems[li] : (int)li;
+                node = conn[(int64_t)v * ne + e];
+                sNode[q][v] = node;
+                sX[q][v][0] = xyz[node];
+                sX[q][v][1] = xyz[nn + node];
+                sX[q][v][2] = xyz[2 * nn + node];
+            }
+#pragma unroll
+            for (int o = 1; o < 8; ++o) twice |= __shfl_xor_sync(0xffffffffu, node, o) == node;
         }
-        __syncthreads();
+        twice = __syncthreads_or(twice && mode == 0);
         for (int t = tid; t < 72 * here; t += kElemThreads) {
             const int q = t / 72, r = t - 72 * q, gp = r / 9, ij = r - 9 * gp, i = ij / 3, j = ij - 3 * i;
             double s = 0.0;
@@ -441,98 +447,104 @@ __global__ void __launch_bounds__(kElemThreads, MINB)
             __syncthreads();
         }
         const int q = q4, a = a4, b = b4;
-        if (q < here && !(kind == 2 && a != b && mode == 0)) {  // lumped: diagonal blocks only
-            const int64_t li = base + q;
-            const int e = elems ? elems[li] : (int)li;
-            double *va = nullptr, *vb = nullptr;
-            int na = 0, nb = 0;
-            if (mode == 0) {
-                const uint16_t *sl = slots + (int64_t)e * 64;
-                const int ra = sNode[q][a], rb = sNode[q][b];
-                const int64_t r0 = rp[ra], r1 = rp[rb];
-                na = (int)(rp[ra + 1] - r0);
-                nb = (int)(rp[rb + 1] - r1);
-                va = val + r0 * 9 + sl[a * 8 + b];
-                vb = val + r1 * 9 + sl[b * 8 + a];
-            }
-            double K[3][3];
-            if (kind == 0) {
-                double P[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-                if (sPos[q]) {
+        // A colour's elements share no node, so every entry has one writer -- unless an
+        // element names a node twice (a hexahedron collapsed to a wedge or a pyramid):
+        // then its blocks are added one after another.
+        for (int turn = twice ? 0 : 35; turn < 36; ++turn) {
+            if (q < here && !(kind == 2 && a != b && mode == 0) &&  // (lumped: diagonal blocks only)
+                (!twice || tid - 36 * q == turn)) {
+                const int64_t li = base + q;
+                const int e = elems ? elems[li] : (int)li;
+                double *va = nullptr, *vb = nullptr;
+                int na = 0, nb = 0;
+                if (mode == 0) {
+                    const uint16_t *sl = slots + (int64_t)e * 64;
+                    const int ra = sNode[q][a], rb = sNode[q][b];
+                    const int64_t r0 = rp[ra], r1 = rp[rb];
+                    na = (int)(rp[ra + 1] - r0);
+                    nb = (int)(rp[rb + 1] - r1);
+                    va = val + r0 * 9 + sl[a * 8 + b];
+                    vb = val + r1 * 9 + sl[b * 8 + a];
+                }
+                double K[3][3];
+                if (kind == 0) {
+                    double P[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+                    if (sPos[q]) {
 #pragma unroll 4
-                    for (int gp = 0; gp < 8; ++gp) {
-                        const double ha[3] = {sH[q][gp][a][0], sH[q][gp][a][1], sH[q][gp][a][2]};
-                        const double hb[3] = {sH[q][gp][b][0], sH[q][gp][b][1], sH[q][gp][b][2]};
+                        for (int gp = 0; gp < 8; ++gp) {
+                            const double ha[3] = {sH[q][gp][a][0], sH[q][gp][a][1], sH[q][gp][a][2]};
+                            const double hb[3] = {sH[q][gp][b][0], sH[q][gp][b][1], sH[q][gp][b][2]};
 #pragma unroll
-                        for (int i = 0; i < 3; ++i)
+                            for (int i = 0; i < 3; ++i)
 #pragma unroll
-                            for (int j = 0; j < 3; ++j) P[i][j] = fma(ha[i], hb[j], P[i][j]);
+                                for (int j = 0; j < 3; ++j) P[i][j] = fma(ha[i], hb[j], P[i][j]);
+                        }
+                    } else {
+                        for (int gp = 0; gp < 8; ++gp) {
+                            const double w = sW[q][gp];
+                            const double wa[3] = {w * sH[q][gp][a][0], w * sH[q][gp][a][1], w * sH[q][gp][a][2]};
+                            const double gb[3] = {sH[q][gp][b][0], sH[q][gp][b][1], sH[q][gp][b][2]};
+#pragma unroll
+                            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                                for (int j = 0; j < 3; ++j) P[i][j] = fma(wa[i], gb[j], P[i][j]);
+                        }
                     }
-                } else {
-                    for (int gp = 0; gp < 8; ++gp) {
-                        const double w = sW[q][gp];
-                        const double wa[3] = {w * sH[q][gp][a][0], w * sH[q][gp][a][1], w * sH[q][gp][a][2]};
-                        const double gb[3] = {sH[q][gp][b][0], sH[q][gp][b][1], sH[q][gp][b][2]};
-#pragma unroll
-                        for (int i = 0; i < 3; ++i)
-#pragma unroll
-                            for (int j = 0; j < 3; ++j) P[i][j] = fma(wa[i], gb[j], P[i][j]);
-                    }
-                }
-                double lam, mu;
-                lame(bcast ? p0[0] : p0[e], bcast ? p1[0] : p1[e], lam, mu);
-                const double mt = mu * (P[0][0] + P[1][1] + P[2][2]);
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) K[i][j] = fma(lam, P[i][j], mu * P[j][i]) + (i == j ? mt : 0.0);
-            } else {
-                const double rho = bcast ? p0[0] : p0[e];
-                double m = 0.0;
-                if (kind == 1) {
-#pragma unroll
-                    for (int gp = 0; gp < 8; ++gp) m += sN[gp][a] * sN[gp][b] * sW[q][gp];
-                    m *= rho;
-                } else if (a == b) {
-                    for (int bb = 0; bb < 8; ++bb) {
-                        double mb = 0.0;
-#pragma unroll
-                        for (int gp = 0; gp < 8; ++gp) mb += sN[gp][a] * sN[gp][bb] * sW[q][gp];
-                        m += rho * mb;
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) K[i][j] = (i == j) ? m : 0.0;
-            }
-            if (mode == 1) {
-                double *o = out + (int64_t)e * 576;
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {
-                        o[(3 * b + j) * 24 + 3 * a + i] = K[i][j];
-                        if (a != b) o[(3 * a + i) * 24 + 3 * b + j] = K[i][j];
-                    }
-            } else {
-                // a colour's elements share no node: every entry has one writer
-                double old[9];
-#pragma unroll
-                for (int k = 0; k < 9; ++k) old[k] = va[(int64_t)k * na];
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) va[(int64_t)(3 * i + j) * na] = old[3 * i + j] + K[i][j];
-                if (a != b) {
-#pragma unroll
-                    for (int k = 0; k < 9; ++k) old[k] = vb[(int64_t)k * nb];
+                    double lam, mu;
+                    lame(bcast ? p0[0] : p0[e], bcast ? p1[0] : p1[e], lam, mu);
+                    const double mt = mu * (P[0][0] + P[1][1] + P[2][2]);
 #pragma unroll
                     for (int i = 0; i < 3; ++i)
 #pragma unroll
-                        for (int j = 0; j < 3; ++j) vb[(int64_t)(3 * j + i) * nb] = old[3 * j + i] + K[i][j];
+                        for (int j = 0; j < 3; ++j) K[i][j] = fma(lam, P[i][j], mu * P[j][i]) + (i == j ? mt : 0.0);
+                } else {
+                    const double rho = bcast ? p0[0] : p0[e];
+                    double m = 0.0;
+                    if (kind == 1) {
+#pragma unroll
+                        for (int gp = 0; gp < 8; ++gp) m += sN[gp][a] * sN[gp][b] * sW[q][gp];
+                        m *= rho;
+                    } else if (a == b) {
+                        for (int bb = 0; bb < 8; ++bb) {
+                            double mb = 0.0;
+#pragma unroll
+                            for (int gp = 0; gp < 8; ++gp) mb += sN[gp][a] * sN[gp][bb] * sW[q][gp];
+                            m += rho * mb;
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) K[i][j] = (i == j) ? m : 0.0;
+                }
+                if (mode == 1) {
+                    double *o = out + (int64_t)e * 576;
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) {
+                            o[(3 * b + j) * 24 + 3 * a + i] = K[i][j];
+                            if (a != b) o[(3 * a + i) * 24 + 3 * b + j] = K[i][j];
+                        }
+                } else {
+                    double old[9];
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) old[k] = va[(int64_t)k * na];
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) va[(int64_t)(3 * i + j) * na] = old[3 * i + j] + K[i][j];
+                    if (a != b) {
+#pragma unroll
+                        for (int k = 0; k < 9; ++k) old[k] = vb[(int64_t)k * nb];
+#pragma unroll
+                        for (int i = 0; i < 3; ++i)
+#pragma unroll
+                            for (int j = 0; j < 3; ++j) vb[(int64_t)(3 * j + i) * nb] = old[3 * j + i] + K[i][j];
+                    }
                 }
             }
+            if (twice) __syncthreads();
         }
         __syncthreads();
     }
