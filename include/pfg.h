@@ -86,7 +86,13 @@ typedef struct pfg_solve_opts {
                                 by this factor since the last replacement; default 0.1 */
     int32_t debug;           /* FEMSolver_%debug: print the residual every graph_chunk iterations */
     int32_t update_mode;     /* 0 auto, 1 vector updates fused into the SpMV gathers,
-                                2 separate streaming passes (see krylov.cu) */
+                                2 separate streaming passes (see krylov.cu).  Auto runs most
+                                systems below some 100,000 block rows in one cooperative
+                                launch that fills the device (resident.cu): several threads'
+                                such solves take turns, launch by launch, where modes 1 and 2
+                                share the device.  One thread solves 17,576 hexes (mixed CG)
+                                in 4.7 ms against 9.6; four threads get a solve every 4.6 ms
+                                against 3.2.  Many systems at once: pfg_batch_*. */
     int32_t storage;         /* mixed: PFG_STORAGE_FULL (default) or PFG_STORAGE_SYMMETRIC */
 } pfg_solve_opts;
 
@@ -396,7 +402,9 @@ int pfg_newmark_step(pfg_solver *h, const pfg_solve_opts *opts, int64_t n, const
  * up exactly as for pfg_solve: setCRS, assembly, fix -- and solves all of them
  * in ONE persistent kernel launch (replayed from a CUDA graph): each system is
  * solved by one CTA, or by a thread-block cluster for the largest ones, taking
- * jobs from an atomic queue in order of decreasing estimated cost.  Handles
+ * jobs from an atomic queue in order of decreasing estimated cost.  The costs follow
+ * the iteration counts of the solve before, and with them the teams: a system's last
+ * digits can differ between a first and a second solve of the same data.  Handles
  * must hold 3-DOF (3x3-block) systems on the batch's device, must outlive the
  * batch's use of them and must not be used while a batched solve runs; re-bind
  * (pfg_batch_set) after changing any of them. */
@@ -407,7 +415,9 @@ typedef struct pfg_batch_config {
     int32_t cluster;       /* CTAs that solve one large system together (1, 2, 4 or 8) */
     double team_fraction;  /* share of the systems, largest estimated cost first, solved by a
                               whole cluster; the rest are solved by single CTAs, or by
-                              larger teams where one would outlast the others */
+                              larger teams where one would outlast the others (pairs may
+                              grow to fours).  A share that rounds to no system: single CTAs
+                              only */
 } pfg_batch_config;
 
 typedef struct pfg_batch_info {

@@ -2,8 +2,8 @@
 //
 // Restates bicgstab_CRS_2 (FEMSolverClass.f90:2199-2298) and adds CG for the
 // symmetric eliminated system.  Design:
-//   * a solve small enough for the SMs' shared memory runs as one cooperative launch
-//     (resident.cu); what follows is the kernel-by-kernel form of the larger ones;
+//   * smaller solves run as one cooperative launch (resident.cu; resident_pays below says
+//     which); what follows is the kernel-by-kernel form of the larger ones;
 //   * every scalar (rho, alpha, beta, c1..c3, norms) lives in device memory
 //     (KState); the last CTA of each fused reduction computes the next scalars,
 //     so one iteration is 3 (CG) or 5 (BiCGSTAB) kernel launches and no host

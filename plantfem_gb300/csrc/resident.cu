@@ -5,8 +5,12 @@
 // cold, drains, and ends in a chain of L2 round trips (partial sums, ticket, the
 // last CTA's total).  Here one cooperative launch holds a CTA on every SM for the
 // whole solve:
-//   * a CTA owns a run of slices (32 block rows each); x, r, p, ... of its rows
-//     stay in its shared memory from the first iteration to the last;
+//   * a CTA owns a run of slices (32 block rows each); x, r, p, ... of its rows lie in
+//     its shared memory, as many of them as fit beside the ring (`near`; in the order of
+//     their use, the inverse diagonal blocks last), the others in global scratch that
+//     only it reads.  With block Jacobi, 3x3 blocks and 152 SMs all fit up to 53,500 block
+//     rows (FP64 CG), 34,000 (FP64 BiCGSTAB), 68,000 (mixed CG), 53,500 (mixed BiCGSTAB); at
+//     119,000 rows two of FP64 CG's six, above 185,000 none;
 //   * only the vector that the next product gathers is written to global memory;
 //   * the CTA's slots are cut into 16 equal runs, one per warp, whatever the
 //     slices' boundaries: a warp stores the sums of each slice it touches and a
@@ -34,13 +38,13 @@
 //   BiCG FP64  61.4 -> 25.1 72.6 -> 31.3 91.7 -> 45.2  107 -> 75.0  138 ->  121  180 ->  181
 //   BiCG mixed 48.2 -> 18.7 46.2 -> 20.2 44.5 -> 24.4 48.0 -> 31.0 66.9 -> 52.6 75.3 -> 94.4
 // (mixed, kernel by kernel, reads the upper half of the matrix from HBM; resident
-// reads the whole FP32 copy, which pays while that fits L2: 98 MB at 91,125 rows).
+// reads the whole FP32 copy, which pays while that fits L2: 98 MB at 91,125 rows).  Other
+// kinds of rows and the limits: krylov.cu, resident_pays.
 //
 // Every wait is bounded: a CTA whose inbox does not fill within the limit raises
 // `err` and leaves, and so do the others; copies in flight are waited for first.
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 
 #include "bulk.cuh"
 #include "resident.cuh"
