@@ -116,7 +116,7 @@ struct Grid {
     // the entry of CTA `from` in CTA `to`'s inbox
     __device__ double *entry(unsigned buf, int to, int from) const
     {
-        return slots + (((size_t)buf * gridDim.x + to) * gridDim.x + from) * kResValues;
+        return slots + (((size_t)buf * kResMaxCtas + to) * kResMaxCtas + from) * kResValues;
     }
 
     // v (valid in warp 0) -> the grid's totals in every thread; `fin(totals)` runs
@@ -1066,7 +1066,7 @@ __device__ void open_share(Share &h, ResShared &sh, const ResArgs &a, const int6
     g.err = &a.st->err;
     g.lane = threadIdx.x & 31;
     g.wid = threadIdx.x >> 5;
-    g.round = 0;
+    g.round = a.round;
     g.s0 = a.bounds[blockIdx.x];
     g.nsl = a.bounds[blockIdx.x + 1] - g.s0;
     int64_t *sp = take<int64_t>(mem, (size_t)g.nsl + 1 + ((g.nsl + 1) & 1));
@@ -1167,6 +1167,7 @@ __device__ void close_state(ResShared &sh, const Grid &g, const ResArgs &a, int 
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sh.state.phase = phase;
+        sh.state.round = g.round;
         sh.state.err = *(volatile int *)&a.st->err;
         *a.st = sh.state;
     }
@@ -1613,22 +1614,47 @@ std::shared_ptr<ResDevice> ResDevice::current()
 
 namespace {
 
-// The launch, after the one before on this device and with empty inboxes (a memset of at
-// most 3 MB, 2 us in the stream).  False: the device does not hold the grid at once.
-bool launch_in_turn(ResDevice &dev, const void *kern, int ctas, void **args, size_t smem, cudaStream_t st)
+// The launch, after the one before on this device.  Its inboxes are those that a launch
+// of as many CTAs left, each buffer in the state that the next round expects, or empty
+// ones (a memset of at most 3 MB) where another grid was there last or may still be.
+// Its number; 0: the device does not hold the grid at once.
+uint64_t launch_in_turn(ResDevice &dev, ResKernel kern, int ctas, ResArgs &a, size_t smem, cudaStream_t st)
 {
     std::lock_guard<std::mutex> lk(dev.mu);
-    PFG_CUDA(cudaStreamWaitEvent(st, dev.last, 0));
-    const size_t used = (size_t)kResRounds * kResValues * ctas * ctas;
-    PFG_CUDA(cudaMemsetAsync(dev.slots.p, 0xff, used * sizeof(double), st));
-    const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(ctas), dim3(kNT), args, smem, st);
+    const bool ready = dev.in_flight == 0 && dev.ready_ctas == ctas;
+    dev.ready_ctas = 0;
+    if (ready) {
+        a.round = dev.ready_round;
+    } else {
+        if (dev.in_flight > 0) PFG_CUDA(cudaStreamWaitEvent(st, dev.last, 0));
+        constexpr size_t inbox = (size_t)kResValues * kResMaxCtas * sizeof(double);
+        PFG_CUDA(cudaMemset2DAsync(dev.slots.p, kResMaxCtas * inbox, 0xff, ctas * inbox, kResRounds, st));
+        a.round = 0;
+    }
+    void *args[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)kern, dim3(ctas), dim3(kNT), args, smem, st);
     if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
         (void)cudaGetLastError();
-        return false;
+        return 0;
     }
     PFG_CUDA(e);
+    ++dev.in_flight;
+    ++dev.launches;
     PFG_CUDA(cudaEventRecord(dev.last, st));
-    return true;
+    return dev.launches;
+}
+
+// Waits for launch `number`; its state in *host.
+void end_turn(ResDevice &dev, uint64_t number, int ctas, const ResState *host, cudaStream_t st)
+{
+    const cudaError_t e = cudaStreamSynchronize(st);
+    std::lock_guard<std::mutex> lk(dev.mu);
+    --dev.in_flight;
+    if (number == dev.launches && e == cudaSuccess && host->err == 0) {
+        dev.ready_ctas = ctas;
+        dev.ready_round = host->round;
+    }
+    PFG_CUDA(e);
 }
 
 }  // namespace
@@ -1641,15 +1667,17 @@ int run_resident_kernel(ResDevice &dev, const ResPlan &pl, ResArgs a, int bs, in
     a.stages = pl.stages;
     a.near = pl.near;
     a.slots = dev.slots.p;
-    void *args[] = {&a};
     PFG_CUDA(cudaMemcpyAsync(a.st, host, sizeof(ResState), cudaMemcpyHostToDevice, st));
     for (int launches = 1;; ++launches) {
-        if (!launch_in_turn(dev, (const void *)kern, pl.ctas, args, pl.smem, st)) {
+        const uint64_t number = launch_in_turn(dev, kern, pl.ctas, a, pl.smem, st);
+        if (number == 0) {
             PFG_CHECK(launches == 1, PFG_E_CUDA, "resident solve: the device took no further launch");
             return 0;
         }
-        PFG_CUDA(cudaMemcpyAsync(host, a.st, sizeof(ResState), cudaMemcpyDeviceToHost, st));
-        PFG_CUDA(cudaStreamSynchronize(st));
+        const cudaError_t e = cudaMemcpyAsync(host, a.st, sizeof(ResState), cudaMemcpyDeviceToHost, st);
+        if (e != cudaSuccess) host->err = 1;
+        end_turn(dev, number, pl.ctas, host, st);
+        PFG_CUDA(e);
         PFG_CHECK(host->err == 0, PFG_E_INTERNAL, "resident solve: a wait between CTAs ran out");
         if (debug && mixed)
             fprintf(stderr, "[pfg] mixed iter %d replacement %d |b-Ax|/|b| %.3e%s\n", host->iter, host->replacements,

@@ -20,6 +20,7 @@ struct ResState {
     double rel, prev_rel, best_rel;
     float rmax32, rmin32;
     int err;         // raised when a wait runs out
+    unsigned round;  // exchanges made by the last launch and those whose slots it took over
 };
 
 // What every resident kernel reads: matrices, the published (gathered) vectors
@@ -38,7 +39,8 @@ struct ResArgs {
     const double *dinv64;
     const float *dinv32;
     ResState *st;
-    double *slots;  // set by run_resident_kernel
+    double *slots;   // set by run_resident_kernel, as is:
+    unsigned round;  // the first round of the launch
     int pc, stop_rule, itrmax, budget, stages, near;
     double er0, tol, delta;
 };
@@ -66,7 +68,13 @@ constexpr size_t kResSlots = (size_t)kResRounds * kResValues * kResMaxCtas * kRe
 struct ResDevice {
     std::mutex mu;
     cudaEvent_t last = nullptr;  // end of the last launch
+    int in_flight = 0;           // launches whose threads have not seen their end
+    uint64_t launches = 0;
     DevBuf<double> slots;
+    // what the last launch left: inboxes ready for this round of a grid of as many CTAs
+    // (0: not known, or not well)
+    int ready_ctas = 0;
+    unsigned ready_round = 0;
     ~ResDevice()
     {
         if (last) cudaEventDestroy(last);
