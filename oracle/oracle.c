@@ -770,14 +770,18 @@ void orc_crs_spmm(int64_t n, const int64_t *row_ptr, const int32_t *col_idx, con
  * one at a time (nai = v_j . viold, viold = viold - nai v_j) and normalised.
  * The projection off v_j and the dot with v_{j+1} share one pass over viold;
  * the dots are OpenMP reductions (summation order differs from a sequential
- * loop in the last bits only). */
+ * loop in the last bits only), whose partial sums meet in the order the threads
+ * finish.  Short columns are taken by one thread: the threads' start costs more than
+ * the loop, and LOBPCG's path, which follows those bits into degenerate bases now
+ * and then, is the same in every run. */
+enum { kGsParallel = 32768 };
 void orc_gram_schmidt(int64_t n, int64_t m, double *V)
 {
     double *viold = malloc((size_t)n * sizeof(double));
     for (int64_t i = 0; i < m; ++i) {
         double *vi = V + i * n;
         double s = 0.0;
-#pragma omp parallel for reduction(+ : s) schedule(static)
+#pragma omp parallel for reduction(+ : s) schedule(static) if (n >= kGsParallel)
         for (int64_t k = 0; k < n; ++k) {
             viold[k] = vi[k];
             s += vi[k] * vi[k];
@@ -786,7 +790,7 @@ void orc_gram_schmidt(int64_t n, int64_t m, double *V)
         double nai = 0.0;
         if (i > 0) {
             const double *v0 = V;
-#pragma omp parallel for reduction(+ : nai) schedule(static)
+#pragma omp parallel for reduction(+ : nai) schedule(static) if (n >= kGsParallel)
             for (int64_t k = 0; k < n; ++k) nai += v0[k] * viold[k];
         }
         for (int64_t j = 0; j < i; ++j) {
@@ -794,7 +798,7 @@ void orc_gram_schmidt(int64_t n, int64_t m, double *V)
             const double *vn = j + 1 < i ? V + (j + 1) * n : viold;  /* next dot, or |viold|^2 */
             const double a = nai;
             double t = 0.0;
-#pragma omp parallel for reduction(+ : t) schedule(static)
+#pragma omp parallel for reduction(+ : t) schedule(static) if (n >= kGsParallel)
             for (int64_t k = 0; k < n; ++k) {
                 const double v = viold[k] - a * vj[k];
                 viold[k] = v;
@@ -804,7 +808,7 @@ void orc_gram_schmidt(int64_t n, int64_t m, double *V)
         }
         /* here nai = |viold|^2 (for i > 0: the last pass dotted viold with itself) */
         const double nrm = i > 0 ? sqrt(nai) : sqrt(s);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (n >= kGsParallel)
         for (int64_t k = 0; k < n; ++k) vi[k] = viold[k] / nrm;
     }
     free(viold);
@@ -818,14 +822,14 @@ void orc_gram_schmidt(int64_t n, int64_t m, double *V)
 void orc_gram_schmidt_rm(int64_t n, int64_t m, double *V, double *scratch)
 {
     double *T = scratch ? scratch : malloc((size_t)n * (size_t)m * sizeof(double));
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (n >= kGsParallel)
     for (int64_t r0 = 0; r0 < n; r0 += 64) {
         const int64_t r1 = r0 + 64 < n ? r0 + 64 : n;
         for (int64_t c = 0; c < m; ++c)
             for (int64_t r = r0; r < r1; ++r) T[c * n + r] = V[r * m + c];
     }
     orc_gram_schmidt(n, m, T);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (n >= kGsParallel)
     for (int64_t r0 = 0; r0 < n; r0 += 64) {
         const int64_t r1 = r0 + 64 < n ? r0 + 64 : n;
         for (int64_t r = r0; r < r1; ++r)
