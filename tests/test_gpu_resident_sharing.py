@@ -5,7 +5,7 @@ import time
 import numpy as np
 import pytest
 
-from plantfem_gb300 import FEMSolver, problems
+from plantfem_gb300 import FEMSolver, FEMSolverBatch, problems
 from plantfem_gb300 import _native as N
 
 pytestmark = pytest.mark.gpu
@@ -129,3 +129,32 @@ def test_a_grid_the_device_does_not_hold(cuda, algorithm, precision, storage):
     t = _solver(problems.lognormal(17, seed=4))
     t.relative_er = 1e-12
     assert np.array_equal(z, t.solve(**kw))
+
+
+def test_beside_a_batch_and_kernel_by_kernel_solves(cuda):
+    """A batch's persistent kernel, resident solves and kernel-by-kernel ones from three
+    threads: each waits for its SMs and ends with the bits it has alone (the batch: its
+    teams follow the solve before, so the answers to 1e-8 relative residuals)."""
+    ps = [problems.lognormal(n, seed=n) for n in (4, 5, 6, 7, 8)]
+    batch = FEMSolverBatch([_solver(p) for p in ps])
+    batch.config = {"threads": 512, "cluster": 2, "team_fraction": 0.4}
+    ref_b = batch.solve(precision="fp64", relative_er=1e-8)
+    p = problems.lognormal(14, seed=3)
+    kw = dict(algorithm="BiCGSTAB", stop_rule="true_relative", preconditioning="BlockJacobi")
+    res, sep = _solver(p), _solver(p)
+    ref_r, ref_s = res.solve(**kw), sep.solve(update_mode="separate", **kw)
+    wrong = []
+
+    def again(what, f, good):
+        for k in range(12):
+            if not good(f()):
+                wrong.append((what, k))
+
+    ts = [threading.Thread(target=again, args=a) for a in (
+        ("batch", lambda: batch.solve(precision="fp64", relative_er=1e-8),
+         lambda xs: all(np.linalg.norm(x - r) <= 1e-4 * np.linalg.norm(r) for x, r in zip(xs, ref_b))),
+        ("resident", lambda: res.solve(**kw), lambda x: np.array_equal(x, ref_r)),
+        ("separate", lambda: sep.solve(update_mode="separate", **kw), lambda x: np.array_equal(x, ref_s)))]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not wrong, wrong
