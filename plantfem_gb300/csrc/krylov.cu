@@ -1742,15 +1742,22 @@ void Krylov::make_v32(DevMatrix &A, cudaStream_t st)
     A.v32_valid = true;
 }
 
-void Krylov::prepare(const DevMatrix &A, const KConfig &cfg, bool resident, cudaStream_t st)
+void Krylov::prepare(const DevMatrix &A, const KConfig &cfg, const ResPlan &plan, cudaStream_t st)
 {
     const int64_t n = A.ndof();
     const bool mixed = cfg.precision == PFG_PREC_MIXED;
     n_ = n;
     bs_ = A.bs;
     const size_t nn = (size_t)std::max<int64_t>(n, 1);
-    if (resident) {  // (its own vectors: run_resident)
-        if (mixed) xb_.ensure(nn);
+    if (plan.ctas > 0) {
+        const size_t np = (size_t)A.nb * (A.bs == 3 ? 4 : 1);
+        if (mixed) {
+            xb_.ensure(nn);
+            res_pub32_.ensure(3 * np);
+        } else {
+            res_pub64_.ensure(2 * np);
+        }
+        res_home_.ensure(plan.home_bytes);
         return;
     }
     r_.ensure(nn);
@@ -2151,13 +2158,13 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
     auto plan_for = [&](const KConfig &c) {
         ResPlan pl;
         if (!may_reside || A.nb > kResidentRowsCG64) return pl;
-        build_sell(A, true, false, st);  // the pattern
+        build_sell(A, false, false, st);  // the pattern
         if (!resident_pays(A, c)) return pl;
         share_slices(A, res_want_ctas_, st);
         return plan_resident(A, c.algorithm, c.precision == PFG_PREC_MIXED, c.precond != PFG_PC_NONE);
     };
     const ResPlan plan = plan_for(cfg);
-    prepare(A, cfg, plan.ctas > 0, st);
+    prepare(A, cfg, plan, st);
     // the Krylov kernels read the sliced copy: FP64 always (residuals), FP32
     // for the mixed inner iterations
     // the symmetric-storage inner iterations read only the upper-half FP32 copy
@@ -2176,7 +2183,7 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
             SolveResult r;
             if (p.ctas > 0) {
                 if (run_resident(A, b, x, c, p, r, st)) return r;
-                prepare(A, c, false, st);
+                prepare(A, c, ResPlan(), st);
                 build_sell(A, true, c.precision == PFG_PREC_MIXED && c.storage != PFG_STORAGE_SYMMETRIC, st);
             }
             return c.precision == PFG_PREC_MIXED ? run_mixed(A, b, x, c, st)
@@ -2194,7 +2201,7 @@ SolveResult Krylov::solve(DevMatrix &A, const double *b, double *x, const KConfi
             c64.stop_rule = PFG_STOP_TRUE_RELATIVE;
             c64.itrmax = std::max(1, cfg.itrmax - res.iterations);
             const ResPlan p64 = plan_for(c64);
-            prepare(A, c64, p64.ctas > 0, st);
+            prepare(A, c64, p64, st);
             SolveResult r2 = run(c64, p64);
             r2.iterations += res.iterations;
             r2.replacements = res.replacements;
@@ -2237,13 +2244,10 @@ bool Krylov::run_resident(DevMatrix &A, const double *b, double *x, const KConfi
     a.x = x;
     a.xb = xb_.p;
     const size_t np = (size_t)A.nb * (A.bs == 3 ? 4 : 1);
-    res_home_.ensure(plan.home_bytes);
     a.home = res_home_.p;
     if (mixed) {
-        res_pub32_.ensure(3 * np);
         for (int k = 0; k < 3; ++k) a.pub32[k] = res_pub32_.p + (size_t)k * np;
     } else {
-        res_pub64_.ensure(2 * np);
         for (int k = 0; k < 2; ++k) a.pub64[k] = res_pub64_.p + (size_t)k * np;
     }
     a.dinv64 = dinv_.p;

@@ -194,8 +194,8 @@ class Krylov {
     void ilu_reset();
 
   private:
-    // Work vectors of a solve in either form.
-    void prepare(const DevMatrix &A, const KConfig &cfg, bool resident, cudaStream_t st);
+    // Work vectors of a solve: resident if plan is one, else kernel by kernel.
+    void prepare(const DevMatrix &A, const KConfig &cfg, const ResPlan &plan, cudaStream_t st);
     void build_precond(const DevMatrix &A, int precond, bool fp32, cudaStream_t st);
     SolveResult run_cg64(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st);
     SolveResult run_bicgstab64(DevMatrix &A, const double *b, double *x, const KConfig &cfg, cudaStream_t st);
